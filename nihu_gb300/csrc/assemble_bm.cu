@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(BM_SING_THREADS) k_singular_bm(BmArgs a, NearL
                 self_tria4_ck(e, fam, kc, x0, ops, acc);
             } else {
                 near_dynamic4_ck(e, kc, x0, nx, ops, acc, a.trial.dyn42 + 42 * (int64_t)j);
-                near_static4(e, x0, nx, ops, acc);
+                near_static4_out<Out>(e, a.trial.frame + 16 * (int64_t)j, a.precision, x0, nx, ops, acc);
             }
         } else if (self) {
             self_tria4(e, fam, k, x0, ops, acc);
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(BM_SING_THREADS) k_singular_bm(BmArgs a, NearL
                 if (a.precision == 0) near_dynamic4_f32(e, k, x0, nx, ops, acc);
                 else near_dynamic4(e, k, x0, nx, ops, acc, a.trial.dyn42 + 42 * (int64_t)j, short_series);
             }
-            near_static4(e, x0, nx, ops, acc);
+            near_static4_out<Out>(e, a.trial.frame + 16 * (int64_t)j, a.precision, x0, nx, ops, acc);
         }
         const int64_t off = (int64_t)(j - a.j0) * a.ld + i;
         if (ops.d || ops.h)

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(PAIR_SING_THREADS) k_pairs_singular(PairArgs a
                     self_tria4_ck(e, fam, kc, x0, ops, acc);
                 } else {
                     near_dynamic4_ck(e, kc, x0, nx, ops, acc, a.trial.dyn42 + 42 * (int64_t)j);
-                    near_static4(e, x0, nx, ops, acc);
+                    near_static4_out<Out>(e, a.trial.frame + 16 * (int64_t)j, a.precision, x0, nx, ops, acc);
                 }
             } else if (self) {
                 self_tria4(e, fam, k, x0, ops, acc);
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(PAIR_SING_THREADS) k_pairs_singular(PairArgs a
                     if (bm_ops && a.precision == 0) near_dynamic4_f32(e, k, x0, nx, ops, acc);
                     else near_dynamic4(e, k, x0, nx, ops, acc, a.trial.dyn42 + 42 * (int64_t)j, short_series);
                 }
-                near_static4(e, x0, nx, ops, acc);
+                near_static4_out<Out>(e, a.trial.frame + 16 * (int64_t)j, a.precision, x0, nx, ops, acc);
             }
         } else {
             // quads (SLP and DLP only): Duffy self term, inverse mapping with
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(PAIR_SING_THREADS) k_pairs_singular(PairArgs a
                         linearized(e, r5[0], r5[1], lin);
                         near_polar_sum(e, lin, fam, kc, x0, r5[0], r5[1], S, polar_d, q);
                         if (fam == FAM_HELMHOLTZ) near_dynamic_ck(lin, kc, x0, S, polar_d, q, nullptr);
-                        near_static(lin, x0, S, polar_d, q);
+                        near_static(lin, nullptr, x0, S, polar_d, q);
                     }
                     if (telles) near_telles_sum(e, fam, kc, x0, r6, q);
                 }
@@ -268,10 +268,10 @@ __global__ void __launch_bounds__(PAIR_SING_THREADS) k_pairs_singular(PairArgs a
                         // FP32 regular quadrature: the schemes' sums in FP32 as well
                         near_polar_sum_f32(e, fam, k, x0, r5[0], r5[1], S, polar_d, q);
                         if (fam == FAM_HELMHOLTZ) near_dynamic_quad_f32(lin, k, x0, S, polar_d, q);
-                        near_static(lin, x0, S, polar_d, q);
+                        near_static(lin, nullptr, x0, S, polar_d, q);
                     } else {
                         near_polar_sum(e, lin, fam, k, x0, r5[0], r5[1], S, polar_d, q);
-                        near_plane(lin, fam, k, x0, S, polar_d, q);
+                        near_plane(lin, nullptr, fam, k, x0, S, polar_d, q);
                     }
                 }
                 if (telles) {
@@ -330,7 +330,10 @@ cudaError_t launch_assemble_pairs(const PairArgs &a, cudaStream_t s)
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // the singular list's length stays on the device: the kernel reads it
     const int64_t swant = (a.n + PAIR_SING_THREADS - 1) / PAIR_SING_THREADS;
-    const int sblocks = (int)std::max<int64_t>(1, std::min<int64_t>(swant, 2 * (int64_t)sms));
+    // three 4-warp blocks per SM, what the registers hold (the float-float sums
+    // are bound by FP32 issue): 5.1 M pairs, 310 k of them nearly singular, in
+    // 0.78 ms (two blocks 0.86 ms)
+    const int sblocks = (int)std::max<int64_t>(1, std::min<int64_t>(swant, 3 * (int64_t)sms));
     const bool ck = a.family == FAM_HELMHOLTZ && a.k_im != 0.0;
     if (ck) {
         if (a.dtype == 0) k_pairs_singular<float2, true><<<sblocks, PAIR_SING_THREADS, 0, s>>>(a);

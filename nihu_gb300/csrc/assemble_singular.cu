@@ -285,7 +285,7 @@ __device__ bool pair_ck(const RegularArgs &a, const Elem64 &e, const double x0[3
     }
     if (e.nc == 3) {
         if (fam == FAM_HELMHOLTZ) near_dynamic_ck(e, kc, x0, do_s, do_d, acc, a.trial.dyn42 + 42 * (int64_t)j);
-        near_static(e, x0, do_s, do_d, acc);
+        near_static(e, a.trial.frame + 16 * (int64_t)j, x0, do_s, do_d, acc);
         return true;
     }
     const bool telles = fam == FAM_HELMHOLTZ && do_d;
@@ -297,7 +297,7 @@ __device__ bool pair_ck(const RegularArgs &a, const Elem64 &e, const double x0[3
         linearized(e, r5[0], r5[1], lin);
         near_polar_sum(e, lin, fam, kc, x0, r5[0], r5[1], do_s, polar_d, acc);
         if (fam == FAM_HELMHOLTZ) near_dynamic_ck(lin, kc, x0, do_s, polar_d, acc, nullptr);
-        near_static(lin, x0, do_s, polar_d, acc);
+        near_static(lin, nullptr, x0, do_s, polar_d, acc);
     }
     if (telles) near_telles_sum(e, fam, kc, x0, r6, acc);
     return true;
@@ -379,7 +379,7 @@ __device__ __forceinline__ void singular_pairs(const RegularArgs &a, const NearL
             double *mS = s_mom + threadIdx.x, *mT = s_mom + MOM_J * SING_THREADS + threadIdx.x;
             const Pt4 *pts = a.trial.dyn42 + 42 * (int64_t)j;
             if (!self) {
-                near_static(e, x0, do_s, do_d, st);
+                near_static(e, a.trial.frame + 16 * (int64_t)j, x0, do_s, do_d, st);
                 if (fam == FAM_HELMHOLTZ) near_moments(e, pts, x0, a.k_absmax, mS, mT, &rmax);
             } else if (do_s) {
                 st.sr = self_static(e, x0) * INV_FOUR_PI;
@@ -428,7 +428,7 @@ __device__ __forceinline__ void singular_pairs(const RegularArgs &a, const NearL
                     if (fam == FAM_HELMHOLTZ) near_dynamic_f32(e, kf, x0, do_s, do_d, acc);
                     near_static_f32(e, a.trial.frame + 16 * (int64_t)j, x0, do_s, do_d, acc);
                 } else {
-                    near_plane(e, fam, kf, x0, do_s, do_d, acc, a.trial.dyn42 + 42 * (int64_t)j, short_f);
+                    near_plane(e, a.trial.frame + 16 * (int64_t)j, fam, kf, x0, do_s, do_d, acc, a.trial.dyn42 + 42 * (int64_t)j, short_f);
                 }
             } else {
                 const bool telles = fam == FAM_HELMHOLTZ && do_d;
@@ -443,10 +443,10 @@ __device__ __forceinline__ void singular_pairs(const RegularArgs &a, const NearL
                             // FP32 regular quadrature: the schemes' sums in FP32 as well
                             near_polar_sum_f32(e, fam, kf, x0, r5[0], r5[1], do_s, polar_d, acc);
                             if (fam == FAM_HELMHOLTZ) near_dynamic_quad_f32(lin, kf, x0, do_s, polar_d, acc);
-                            near_static(lin, x0, do_s, polar_d, acc);
+                            near_static(lin, nullptr, x0, do_s, polar_d, acc);
                         } else {
                             near_polar_sum(e, lin, fam, kf, x0, r5[0], r5[1], do_s, polar_d, acc);
-                            near_plane(lin, fam, kf, x0, do_s, polar_d, acc);
+                            near_plane(lin, nullptr, fam, kf, x0, do_s, polar_d, acc);
                         }
                     }
                     if (telles) {

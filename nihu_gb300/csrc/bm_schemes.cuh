@@ -4,6 +4,7 @@
 // References are paths inside the NiHu project.
 #pragma once
 
+#include "ffloat.cuh"
 #include "planar.cuh"
 
 namespace nihu {
@@ -180,78 +181,51 @@ struct OpSet {
 //   DLPt, 6 Gauss points: -nx.r_vec/r + (nx_0 cos + nx_1 sin) ln(R + r) - nx_2 sgn(z)
 //   HSP, 21 Gauss points: -R^2/(r^2 z) (-r_vec.nx/r), or -nx_2/R when |z| <= 1e-12
 // all over 4 pi (nihu/library/laplace_nearly_singular_integrals.hpp:62-209, :212-298, :301-380).
-// With phi = theta - t0 (|phi| < pi/2 on the side), cos(theta) and sin(theta)
-// follow from the foot direction (cos t0, sin t0) and one short-argument sincos
-// of phi, which also gives R.
-__device__ inline void near_static4(const Elem64 &e, const double x0[3], const double nxg[3], OpSet ops, Acc4 &a)
+// With phi = theta - t0 (PlaneSide), t = R^2 + z^2 times cos^2 phi and
+//   A = dref (n.f) - nx_2 z, B = dref (n.l) (f the foot direction, l the side's)
+// r_vec.nx = (A cos + B sin) / cos, and HSP's integrand is
+// -dref^2 / z (A cos + B sin) t^{-3/2}: no division per point.
+__device__ inline void near_static4(const Elem64 &e, const double *__restrict__ frame, const double x0[3],
+                                    const double nxg[3], OpSet ops, Acc4 &a)
 {
-    double loc[4][2], z, T[3][3];
-    plane_local_frame(e, x0, loc, z, T);
-    const double n0 = dot3(T[0], nxg), n1 = dot3(T[1], nxg), n2 = dot3(T[2], nxg);
+    double loc[4][2], z;
+    frame_local(frame, e.c[0], x0, loc, z);
+    const double n0 = dot3(frame, nxg), n1 = dot3(frame + 3, nxg), n2 = dot3(frame + 6, nxg);
     const double sg = (0.0 < z) - (z < 0.0);
     const double az = fabs(z), z2 = z * z;
     const bool in_plane = !(az > 1e-12);
-    const double iz = in_plane ? 0.0 : 1.0 / z;
     const bool six = ops.s || ops.d || ops.t;
     double s_sum = 0.0, d_sum = 0.0, t_sum = 0.0, h_sum = 0.0;
-    double tl[3], t0[3], dref[3], fc[3], fs[3];
+#pragma unroll 1
     for (int s = 0; s < 3; ++s) {
-        side_geometry(loc[s], loc[(s + 1) % 3], tl[s], t0[s], dref[s], false);
-        // foot direction; atan2(0, 0) = 0 when x0 lies on the side's line
-        double f0 = loc[s][0], f1 = loc[s][1];
-        {
-            const double d0 = loc[(s + 1) % 3][0] - loc[s][0], d1 = loc[(s + 1) % 3][1] - loc[s][1];
-            const double il = 1.0 / sqrt(d0 * d0 + d1 * d1);
-            const double l0 = d0 * il, l1 = d1 * il;
-            const double pr = f0 * l0 + f1 * l1;
-            f0 -= l0 * pr;
-            f1 -= l1 * pr;
+        const PlaneSide sd(loc[s], loc[s == 2 ? 0 : s + 1]);
+        const double s2 = sd.s * sd.s;
+        const double pa = n0 * sd.f0 + n1 * sd.f1, pb = n0 * sd.l0 + n1 * sd.l1;
+        const double A = sd.s * pa - n2 * z, B = sd.s * pb;
+        if (six) {
+            double ss = 0.0, dd = 0.0, tt = 0.0;
+            sd.points<6>([&](double c, double sn, double w) {
+                const double t = fma(z2 * c, c, s2);
+                const double rinv = rsqrt(t), rt = t * rinv, ic = 1.0 / c;
+                if (ops.s) ss += (rt - az * c) * ic * w;
+                if (ops.d) dd += (1.0 - az * c * rinv) * w;
+                if (ops.t) tt += ((pa * c + pb * sn) * log((sd.s + rt) * ic) - (A * c + B * sn) * rinv - n2 * sg) * w;
+            });
+            s_sum += ss * sd.wj;
+            d_sum += dd * sd.wj;
+            t_sum += tt * sd.wj;
         }
-        if (dref[s] > 0.0) {
-            fc[s] = f0 / dref[s];
-            fs[s] = f1 / dref[s];
-        } else {
-            fc[s] = 1.0;
-            fs[s] = 0.0;
-        }
-    }
-    for (int s = 0; s < 3; ++s) {
-        double t1 = tl[s], t2 = tl[(s + 1) % 3];
-        wrap_limits(t1, t2);
-        const double jac = (t2 - t1) / 2.0;
-        // nx_0 cos(theta) + nx_1 sin(theta) = pa cos(phi) + pb sin(phi)
-        const double pa = n0 * fc[s] + n1 * fs[s], pb = n1 * fc[s] - n0 * fs[s];
-        const double dr = dref[s];
-        for (int pass = 0; pass < 2; ++pass) {
-            // pass 0: the 6-point rule of SLP, DLP and DLPt; pass 1: HSP's 21 points
-            const int ng = pass == 0 ? 6 : 21;
-            if (pass == 0 ? !six : !ops.h) continue;
-            for (int q = 0; q < ng; ++q) {
-                double xi, w;
-                gauss_pt(ng, q, xi, w);
-                const double th = t1 * (1.0 - xi) / 2.0 + t2 * (1.0 + xi) / 2.0;
-                double phi = th - t0[s];
-                phi -= (2.0 * PI) * rint(phi * (0.5 / PI));
-                double sp, cp;
-                sincos_bounded(phi, &sp, &cp, false);
-                const double R = dr / cp;
-                const double rnx = R * (pa * cp + pb * sp) - n2 * z;  // r_vec.nx
-                const double jw = jac * w;
-                if (pass == 0) {
-                    const double r2 = R * R + z2;
-                    const double rinv = rsqrt(r2);
-                    const double r = r2 * rinv;
-                    if (ops.s) s_sum += (r - az) * jw;
-                    if (ops.d) d_sum += (1.0 - az * rinv) * jw;
-                    if (ops.t) t_sum += (-rnx * rinv + (pa * cp + pb * sp) * log(R + r) - n2 * sg) * jw;
-                } else if (in_plane) {
-                    h_sum += -n2 / R * jw;
-                } else {
-                    const double r2 = R * R + z2;
-                    const double rinv = rsqrt(r2);
-                    // -R^2/(r^2 z) (-r_vec.nx/r)
-                    h_sum += R * R * rinv * rinv * rinv * rnx * iz * jw;
-                }
+        if (ops.h) {
+            double hh = 0.0;
+            if (in_plane) {
+                sd.points<21>([&](double c, double, double w) { hh += c * w; });
+                h_sum -= n2 / sd.s * sd.wj * hh;
+            } else {
+                sd.points<21>([&](double c, double sn, double w) {
+                    const double rinv = rsqrt(fma(z2 * c, c, s2));
+                    hh += (A * c + B * sn) * (rinv * rinv) * (rinv * w);
+                });
+                h_sum += s2 / z * sd.wj * hh;
             }
         }
     }
@@ -259,6 +233,152 @@ __device__ inline void near_static4(const Elem64 &e, const double x0[3], const d
     a.dr += sg * d_sum * INV_FOUR_PI;
     a.tr += t_sum * INV_FOUR_PI;
     a.hr += h_sum * INV_FOUR_PI;
+}
+
+// near_static4 in float-float arithmetic, for results that are stored in FP32
+// (ffloat.cuh): the same points and formulas, with the plane coordinates, the
+// side lines and the products of the normals in FP64 (about 120 FP64
+// instructions per pair), everything per angular point in float-float.
+//
+// Per side, with the foot point's distance s = |c1 x l| from the side's line
+// and the corners at u1, u2 along it, psi = theta - t0 runs over
+// [atan2(u1, s), atan2(u2, s)] (measured from the foot towards c2), and with
+// t = s^2 + z^2 cos^2 psi, r = sqrt(t) / cos psi the integrands need neither a
+// division nor an angle per point:
+//   HSP   s^2/z (A cos psi + B sin psi) t^{-3/2},  A = s (n.f) - n_2 z, B = s (n.l)
+//   DLPt  -(A cos psi + B sin psi) / sqrt(t) + (n.f cos psi + n.l sin psi)
+//         log((s + sqrt t) / cos psi) - n_2 sgn(z)
+// (f the foot direction, l the side's).  The rule is symmetric about the
+// side's middle angle, so one sin / cos of h x serves the two points +-x.
+// cos psi never falls below s / max(rho_1, rho_2), which the clamp keeps
+// against rounding when x0 lies on a side's line.  Lengths are scaled by a
+// power of two near the element's size, so that no product leaves FP32 range.
+//
+// Bound by FP32 issue: about 18 000 FP32 instructions per pair in place of
+// 8 500 FP64 ones (GB300: 128 against 2 per SM and cycle).  On the sphere of
+// 20480 triangles the singular kernel of the Burton-Miller system, beside the
+// regular one, went from 4.04 to 0.84 ms and the near field list of 5.1 M
+// pairs from 3.53 to 0.78 ms; the complex64 entries' error against 64 bits
+// stays 2.6e-8 and 2.4e-8.  Returns false (nothing added) where the HSP's 1/z
+// cancels between the sides by more than three digits: |z| small against the
+// in-plane part of nx times the side, a folded pair whose collocation point
+// nearly lies in the element's plane; those take FP64.
+__device__ inline bool near_static4_ff(const double *__restrict__ frame, const double c0[3], const double x0[3],
+                                       const double nxg[3], OpSet ops, Acc4 &a)
+{
+    const double dv0 = c0[0] - x0[0], dv1 = c0[1] - x0[1], dv2 = c0[2] - x0[2];
+    const double u0 = frame[0] * dv0 + frame[1] * dv1 + frame[2] * dv2;
+    const double v0 = frame[3] * dv0 + frame[4] * dv1 + frame[5] * dv2;
+    const double z = -(frame[6] * dv0 + frame[7] * dv1 + frame[8] * dv2);
+    const double n0 = dot3(frame, nxg), n1 = dot3(frame + 3, nxg), n2 = dot3(frame + 6, nxg);
+    const bool in_plane = !(fabs(z) > 1e-12);
+    const float len0 = (float)frame[11];  // first side: along the first axis
+    if (ops.h && !in_plane && 1e3f * (float)fabs(z) < (float)(fabs(n0) + fabs(n1)) * len0) return false;
+    const int ex2 = ((__float_as_int(len0) >> 23) & 255) - 127;
+    const float sc = __int_as_float((127 - ex2) << 23), isc = __int_as_float((127 + ex2) << 23);  // 2^-+ex2
+    const ff zf = ff_scale(ff_from(fabs(z)), sc), z2 = ff_mul(zf, zf), n2f = ff_from(n2);
+    const ff n2sg = z > 0.0 ? n2f : (z < 0.0 ? ff_neg(n2f) : ff{0.0f, 0.0f});
+    const bool six = ops.s || ops.d || ops.t;
+    double s_sum = 0.0, d_sum = 0.0, t_sum = 0.0, h_sum = 0.0;
+#pragma unroll 1
+    for (int sd = 0; sd < 3; ++sd) {
+        const int e1 = sd, e2 = sd == 2 ? 0 : sd + 1;
+        const double a0 = frame[9 + 2 * e1], a1 = frame[10 + 2 * e1], b0 = frame[9 + 2 * e2], b1 = frame[10 + 2 * e2];
+        const double d0 = b0 - a0, d1 = b1 - a1, il = rsqrt(d0 * d0 + d1 * d1);
+        const double l0 = d0 * il, l1 = d1 * il;
+        const double p0 = a0 + u0, p1 = a1 + v0;
+        const double sv = p0 * l1 - p1 * l0;  // signed distance of the line
+        const double u1 = p0 * l0 + p1 * l1, u2 = (b0 + u0) * l0 + (b1 + v0) * l1;
+        const double sgn = sv < 0.0 ? -1.0 : 1.0, sa = fabs(sv);
+        const double na = sgn * (n0 * l1 - n1 * l0), nb = n0 * l0 + n1 * l1;  // n.f and n.l
+        const ff u1f = ff_scale(ff_from(u1), sc), u2f = ff_scale(ff_from(u2), sc);
+        ff s = ff_scale(ff_from(sa), sc);
+        s.h = fmaxf(s.h, 1e-14f);
+        const ff A = ff_scale(ff_from(sa * na - n2 * z), sc), B = ff_scale(ff_from(sa * nb), sc);
+        const ff s2 = ff_mul(s, s);
+        const float cmin = s.h * rsqrtf(fmaxf(u1f.h * u1f.h, u2f.h * u2f.h) + s2.h);
+        const ff q1 = ff_angle(u1f, s), q2 = ff_angle(u2f, s);
+        const ff mid = ff_scale(ff_add(q1, q2), 0.5f), hw = ff_scale(ff_sub(q2, q1), 0.5f);
+        ff sm, cm;
+        ff_sincos(mid, sm, cm);
+        // f(cos psi, sin psi) at the points +-x, weights w
+        auto pair_points = [&](ff x, auto &&f) {
+            ff sh, ch;
+            ff_sincos(ff_mul(hw, x), sh, ch);
+            const ff cc = ff_mul(cm, ch), ss = ff_mul(sm, sh), scp = ff_mul(sm, ch), csp = ff_mul(cm, sh);
+            f(ff_sub(cc, ss), ff_add(scp, csp));
+            f(ff_add(cc, ss), ff_sub(scp, csp));
+        };
+        auto clamp_cos = [&](ff c) { return c.h < cmin ? ff{cmin, 0.0f} : c; };
+        const double wj = sgn * ff_double(hw);  // half the side's angle in theta
+        if (six) {
+            const ff naf = ff_from(na), nbf = ff_from(nb);
+            ff sl{0.0f, 0.0f}, sdl{0.0f, 0.0f}, st{0.0f, 0.0f};
+#pragma unroll 1
+            for (int q = 0; q < 3; ++q) {
+                const ff w{GAUSS6_FF.wh[q], GAUSS6_FF.wl[q]};
+                pair_points(ff{GAUSS6_FF.xh[q], GAUSS6_FF.xl[q]}, [&](ff c, ff sn) {
+                    c = clamp_cos(c);
+                    const ff t = ff_add(s2, ff_mul(z2, ff_mul(c, c)));
+                    const ff rs = ff_rsqrt(t), rt = ff_mul(t, rs);
+                    const ff ic = ff_recip(c);
+                    const ff zc = ff_mul(zf, c);
+                    if (ops.s) sl = ff_add(sl, ff_mul(w, ff_mul(ff_sub(rt, zc), ic)));
+                    if (ops.d) sdl = ff_add(sdl, ff_mul(w, ff_sub(ff{1.0f, 0.0f}, ff_mul(zc, rs))));
+                    if (ops.t) {
+                        const ff g = ff_add(ff_mul(naf, c), ff_mul(nbf, sn));
+                        const ff v = ff_mul(ff_add(ff_mul(A, c), ff_mul(B, sn)), rs);
+                        const ff lg = ff_log(ff_mul(ff_add(s, rt), ic), ex2);
+                        st = ff_add(st, ff_mul(w, ff_sub(ff_sub(ff_mul(g, lg), v), n2sg)));
+                    }
+                });
+            }
+            s_sum += wj * ff_double(sl);
+            d_sum += wj * ff_double(sdl);
+            t_sum += wj * ff_double(st);
+        }
+        if (ops.h) {
+            ff sum{0.0f, 0.0f};
+            auto point = [&](ff w, ff c, ff sn) {
+                c = clamp_cos(c);
+                if (in_plane) {
+                    sum = ff_add(sum, ff_mul(w, c));
+                } else {
+                    const ff t = ff_add(s2, ff_mul(z2, ff_mul(c, c)));
+                    const ff rs = ff_rsqrt(t);
+                    // (r_vec.nx / r) (s / sqrt t)^2: both factors stay within 1
+                    const ff v = ff_mul(ff_add(ff_mul(A, c), ff_mul(B, sn)), rs), sr = ff_mul(s, rs);
+                    sum = ff_add(sum, ff_mul(ff_mul(w, v), ff_mul(sr, sr)));
+                }
+            };
+#pragma unroll 1
+            for (int q = 0; q < 10; ++q) {
+                const ff w{GAUSS21_FF.wh[q], GAUSS21_FF.wl[q]};
+                pair_points(ff{GAUSS21_FF.xh[q], GAUSS21_FF.xl[q]}, [&](ff c, ff sn) { point(w, c, sn); });
+            }
+            point(ff{GAUSS21_FF.wh[10], GAUSS21_FF.wl[10]}, cm, sm);
+            // in the plane: -n_2 cos psi / s
+            if (in_plane) h_sum -= wj * n2 * ff_double(sum) / ff_double(s);
+            else h_sum += wj * ff_double(sum);
+        }
+    }
+    const double sg = (0.0 < z) - (z < 0.0);
+    a.sr += s_sum * (INV_FOUR_PI * isc);
+    a.dr += sg * d_sum * INV_FOUR_PI;
+    a.tr += t_sum * INV_FOUR_PI;
+    if (ops.h) a.hr += (in_plane ? h_sum : h_sum / (z * (double)sc)) * (INV_FOUR_PI * sc);
+    return true;
+}
+
+// the static parts for an output type: float-float where the result is stored
+// as complex64 under FP32 regular quadrature, FP64 otherwise
+template <typename Out>
+__device__ __forceinline__ void near_static4_out(const Elem64 &e, const double *__restrict__ frame, int precision,
+                                                 const double x0[3], const double nx[3], OpSet ops, Acc4 &a)
+{
+    if constexpr (sizeof(Out) == 8)
+        if (precision == 0 && near_static4_ff(frame, e.c[0], x0, nx, ops, a)) return;
+    near_static4(e, frame, x0, nx, ops, a);
 }
 
 // dynamic parts K_k - K_0 of the four operators with the 42-point rule
@@ -343,11 +463,10 @@ __device__ inline void near_dynamic4_f32(const Elem64 &e, double k, const double
         const float r2 = rv0 * rv0 + rv1 * rv1 + rv2 * rv2;
         const float rinv = rsqrtf(r2);
         const float kr = kf * (r2 * rinv);
-        float sn, cs;
-        sincosf(kr, &sn, &cs);
-        // cos(kr) - 1 without cancellation
-        const float hs = sinf(0.5f * kr);
-        const float cm1 = -2.0f * hs * hs;
+        // one sincos of the half angle: cos(kr) - 1 without cancellation
+        float hs, hc;
+        sincosf(0.5f * kr, &hs, &hc);
+        const float cm1 = -2.0f * hs * hs, sn = 2.0f * hs * hc, cs = 1.0f + cm1;
         const float t = w * wj * rinv;
         const float rdnx = -(rv0 * xn[0] + rv1 * xn[1] + rv2 * xn[2]) * rinv;
         const float rdny = (rv0 * en[0] + rv1 * en[1] + rv2 * en[2]) * rinv;

@@ -73,16 +73,18 @@ __device__ __forceinline__ void sincos_bounded(double x, double *s, double *c, b
     *s = ps * x;
 }
 
-// cos of an angle difference known to lie within pi/2 of 0 modulo 2 pi
-__device__ __forceinline__ double cos_angle(double x)
+// the series alone: |x| <= pi/2 is the caller's promise
+__device__ __forceinline__ void sincos_series(double x, double &s, double &c)
 {
-    x -= (2.0 * PI) * rint(x * (0.5 / PI));
-    if (fabs(x) > HALF_PI) return cos(x);
     const double u = x * x;
-    double pc = TAYLOR.c[11];
+    double pc = TAYLOR.c[11], ps = TAYLOR.s[11];
 #pragma unroll
-    for (int n = 10; n >= 0; --n) pc = fma(pc, u, TAYLOR.c[n]);
-    return pc;
+    for (int n = 10; n >= 0; --n) {
+        pc = fma(pc, u, TAYLOR.c[n]);
+        ps = fma(ps, u, TAYLOR.s[n]);
+    }
+    c = pc;
+    s = ps * x;
 }
 
 // rotate the element parallel to the x-y plane (nihu/library/plane_element_helper.hpp:112-126):
@@ -114,6 +116,83 @@ __device__ __forceinline__ void plane_local(const Elem64 &e, const double x0in[3
 {
     double T[3][3];
     plane_local_frame(e, x0in, loc, z, T);
+}
+
+// cos of an angle difference known to lie within pi/2 of 0 modulo 2 pi
+__device__ __forceinline__ double cos_angle(double x)
+{
+    x -= (2.0 * PI) * rint(x * (0.5 / PI));
+    if (fabs(x) > HALF_PI) return cos(x);
+    const double u = x * x;
+    double pc = TAYLOR.c[11];
+#pragma unroll
+    for (int n = 10; n >= 0; --n) pc = fma(pc, u, TAYLOR.c[n]);
+    return pc;
+}
+
+// A side of a flat element seen from the foot point of x0 (the origin of the
+// plane frame): the distance s >= 0 from the side's line, the direction
+// (f0, f1) of its foot, and the middle mid and half width hw of the angle
+// psi = theta - t0 over the side, measured from the foot towards its second
+// corner; wj is half the side's angle in theta (signed).  The reference's
+// R(theta) = s / cos psi, and theta's Gauss points are mid +- hw x: with the
+// sine and cosine of mid and of hw x, every point costs four products in
+// place of an angle reduction and a cosine, and the distances
+// r = sqrt(s^2 + z^2 cos^2 psi) / cos psi need no division before the sum.
+// cos psi >= cmin = s / max(rho_1, rho_2), which the points are clamped to
+// where rounding takes them below it (x0 on the side's line).
+struct PlaneSide {
+    double s, f0, f1, l0, l1, sm, cm, hw, wj, cmin;
+    __device__ __forceinline__ PlaneSide(const double c1[2], const double c2[2])
+    {
+        const double d0 = c2[0] - c1[0], d1 = c2[1] - c1[1], q = d0 * d0 + d1 * d1;
+        const double il = rsqrt(q);
+        l0 = d0 * il;
+        l1 = d1 * il;
+        const double sv = c1[0] * l1 - c1[1] * l0;
+        const double u1 = c1[0] * l0 + c1[1] * l1, u2 = c2[0] * l0 + c2[1] * l1;
+        const double sgn = sv < 0.0 ? -1.0 : 1.0;
+        f0 = sgn * l1;
+        f1 = -sgn * l0;
+        s = fmax(fabs(sv), 1e-30 * q * il);
+        cmin = s * rsqrt(fmax(u1 * u1, u2 * u2) + s * s);
+        const double a1 = atan2(u1, s), a2 = atan2(u2, s);
+        hw = 0.5 * (a2 - a1);
+        wj = sgn * hw;
+        sincos_series(0.5 * (a1 + a2), sm, cm);
+    }
+    // f(cos psi, sin psi, w) at the points of the NG-point Gauss rule
+    template <int NG, class F>
+    __device__ __forceinline__ void points(F &&f) const
+    {
+#pragma unroll 1
+        for (int q = 0; q < NG / 2; ++q) {
+            double x, w, sh, ch;
+            gauss_pt(NG, NG - 1 - q, x, w);
+            sincos_series(hw * x, sh, ch);
+            f(fmax(cm * ch - sm * sh, cmin), sm * ch + cm * sh, w);
+            f(fmax(cm * ch + sm * sh, cmin), sm * ch - cm * sh, w);
+        }
+        if (NG & 1) {
+            double x, w;
+            gauss_pt(NG, NG / 2, x, w);
+            f(fmax(cm, cmin), sm, w);
+        }
+    }
+};
+
+// the plane coordinates of a triangle's corners and the height z of x0 above
+// it from the element's precomputed frame (DevMesh::frame)
+__device__ __forceinline__ void frame_local(const double *__restrict__ frame, const double c0[3], const double x0[3],
+                                            double loc[4][2], double &z)
+{
+    const double dv[3] = {c0[0] - x0[0], c0[1] - x0[1], c0[2] - x0[2]};
+    const double u = dot3(frame, dv), v = dot3(frame + 3, dv);
+    z = -dot3(frame + 6, dv);
+    for (int a = 0; a < 3; ++a) {
+        loc[a][0] = frame[9 + 2 * a] + u;
+        loc[a][1] = frame[10 + 2 * a] + v;
+    }
 }
 
 // first column of trial element j >= j0 whose pairs include list entry p:

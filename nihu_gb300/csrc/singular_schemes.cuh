@@ -72,35 +72,34 @@ __device__ __forceinline__ void kern_on_elem(const Elem64 &e, int fam, K k, cons
 // static (Laplace) nearly singular part over a flat element: radial integral
 // analytic, angular integral with 6 Gauss points per side
 // (nihu/library/laplace_nearly_singular_integrals.hpp:62-209); adds the SLP and
-// DLP (real) results to a.sr / a.dr
-__device__ inline void near_static(const Elem64 &e, const double x0[3], bool do_s, bool do_d, Acc &a)
+// DLP (real) results to a.sr / a.dr.  frame: the element's DevMesh::frame
+// record when it is a triangle of a mesh (else NULL: the frame is formed here).
+__device__ inline void near_static(const Elem64 &e, const double *__restrict__ frame, const double x0[3], bool do_s,
+                                   bool do_d, Acc &a)
 {
     double loc[4][2], z;
-    plane_local(e, x0, loc, z);
+    if (frame) frame_local(frame, e.c[0], x0, loc, z);
+    else plane_local(e, x0, loc, z);
     const int N = e.nc;
-    double tl[4], t0[4], dr[4];
-    for (int s = 0; s < N; ++s) side_geometry(loc[s], loc[(s + 1) % N], tl[s], t0[s], dr[s], false);
     const double az = fabs(z), z2 = z * z;
     double s_sum = 0.0, d_sum = 0.0;
+#pragma unroll 1
     for (int s = 0; s < N; ++s) {
-        double t1 = tl[s], t2 = tl[(s + 1) % N];
-        wrap_limits(t1, t2);
-        const double jac = (t2 - t1) / 2.0;
-        for (int q = 0; q < 6; ++q) {
-            double xi, w;
-            gauss_pt(6, q, xi, w);
-            double th = t1 * (1.0 - xi) / 2.0 + t2 * (1.0 + xi) / 2.0;
-            double R = dr[s] / cos_angle(th - t0[s]);
-            double r2 = R * R + z2;
-            double rinv = rsqrt(r2);
-            double jw = jac * w;
-            if (do_s) s_sum += (r2 * rinv - az) * jw;  // r - |z|
-            if (do_d) d_sum += (1.0 - az * rinv) * jw;  // 1 - |z|/r
-        }
+        const PlaneSide sd(loc[s], loc[s + 1 == N ? 0 : s + 1]);
+        const double s2 = sd.s * sd.s;
+        double ss = 0.0, dd = 0.0;
+        sd.points<6>([&](double c, double, double w) {
+            const double t = fma(z2 * c, c, s2);
+            const double rinv = rsqrt(t);  // cos psi / r
+            if (do_s) ss += (t * rinv - az * c) / c * w;  // r - |z|
+            if (do_d) dd += (1.0 - az * c * rinv) * w;    // 1 - |z|/r
+        });
+        s_sum += ss * sd.wj;
+        d_sum += dd * sd.wj;
     }
     const double sg = (0.0 < z) - (z < 0.0);
-    a.sr += s_sum * INV_FOUR_PI;
-    a.dr += sg * d_sum * INV_FOUR_PI;
+    if (do_s) a.sr += s_sum * INV_FOUR_PI;
+    if (do_d) a.dr += sg * d_sum * INV_FOUR_PI;
 }
 
 // near_static with the angular point sums in FP32 (the FP32 regular
@@ -137,7 +136,7 @@ __device__ inline void near_static_f32(const Elem64 &e, const double *__restrict
         const double *c1 = loc[s], *c2 = loc[(s + 1) % N];
         const double cr = c1[0] * c2[1] - c1[1] * c2[0];
         if (fabs(cr) <= 1e-9 * scale) {
-            near_static(e, x0, do_s, do_d, a);
+            near_static(e, frame, x0, do_s, do_d, a);
             return;
         }
         if (cr > 0.0) ++pos;
@@ -371,11 +370,12 @@ __device__ inline void near_dynamic_f32(const Elem64 &e, double k, const double 
 }
 
 // full planar constant-element nearly singular integral
-__device__ inline void near_plane(const Elem64 &e, int fam, double k, const double x0[3], bool do_s, bool do_d, Acc &a,
-                           const Pt4 *__restrict__ pts42 = nullptr, bool short_series = false)
+__device__ inline void near_plane(const Elem64 &e, const double *__restrict__ frame, int fam, double k,
+                                  const double x0[3], bool do_s, bool do_d, Acc &a,
+                                  const Pt4 *__restrict__ pts42 = nullptr, bool short_series = false)
 {
     if (fam == FAM_HELMHOLTZ) near_dynamic(e, k, x0, do_s, do_d, a, pts42, short_series);
-    near_static(e, x0, do_s, do_d, a);
+    near_static(e, frame, x0, do_s, do_d, a);
 }
 
 // ------------------------------------------------------------ inverse mapping
