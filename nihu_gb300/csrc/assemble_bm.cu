@@ -34,6 +34,7 @@
 #include "bm_schemes.cuh"
 #include "classify.cuh"
 #include "kernels.h"
+#include "two_row.cuh"
 
 namespace nihu {
 
@@ -63,6 +64,36 @@ __device__ __forceinline__ void store_bm(Out *p, R r0, R i0, R c0r, R c0i, R r1,
         o.y = vi;
     }
     *p = o;
+}
+
+// HSP level 3 (1.5 <= d/D < 1.9) in FP32: degree 6 (par 0) or 7 (par 1) on the
+// flat triangle y = c0 + xi e1 + eta e2; y - x = (c_j - x) + (y - c_j), the first
+// part (dx, dy, dz) from the hi/lo centres, the second from the corners
+// relative to the centre
+template <int FAM, bool CK = false>
+__device__ __forceinline__ void hsp_level3_f32(const DevMesh &trial, int j, int par, float dx, float dy, float dz,
+                                               const float4 p, float nx0, float nx1, float nx2, float k, BmSum<float> &o,
+                                               float ki = 0.0f)
+{
+    const double *cc = trial.corners + 12 * (int64_t)j;
+    const double *cen = trial.center + 3 * (int64_t)j;
+    double e1[3], e2[3], nt[3];
+    for (int d = 0; d < 3; ++d) { e1[d] = cc[3 + d] - cc[d]; e2[d] = cc[6 + d] - cc[d]; }
+    cross3(e1, e2, nt);
+    const float Jf = (float)norm3(nt);
+    float b[3], f1[3], f2[3];
+    for (int d = 0; d < 3; ++d) {
+        b[d] = (float)(cc[d] - cen[d]);
+        f1[d] = (float)e1[d];
+        f2[d] = (float)e2[d];
+    }
+    const int np = par ? 13 : 12;
+    for (int q = 0; q < np; ++q) {
+        const float *t = par ? TRI67.p7[q] : TRI67.p6[q];
+        eval_h<FAM, float, CK>(dx + (b[0] + t[0] * f1[0] + t[1] * f2[0]), dy + (b[1] + t[0] * f1[1] + t[1] * f2[1]),
+                               dz + (b[2] + t[0] * f1[2] + t[1] * f2[2]), t[2] * Jf, p.y, p.z, p.w, nx0, nx1, nx2, k, o,
+                               ki);
+    }
 }
 
 // Work layout as the plain regular kernel: a thread owns a test row, a block
@@ -193,35 +224,17 @@ __global__ void __launch_bounds__(BM_THREADS, sizeof(R) == 4 ? 4 : 1) k_regular_
                 }
             }
             if (do_h && lh == 3) {
-                // HSP level 3 (only 1.5 <= d/D < 1.9): degree 6 (par 0) or 7 (par 1)
-                // on the flat triangle y = c0 + xi e1 + eta e2
-                const double *cc = trial.corners + 12 * (int64_t)j;
-                const double *n64 = trial.pts64 + 8 * base + 4;
-                double e1[3], e2[3], nt[3];
-                for (int d = 0; d < 3; ++d) { e1[d] = cc[3 + d] - cc[d]; e2[d] = cc[6 + d] - cc[d]; }
-                cross3(e1, e2, nt);
-                const double J = norm3(nt);
-                const int np = par ? 13 : 12;
+                // HSP level 3 (only 1.5 <= d/D < 1.9)
                 if constexpr (sizeof(R) == 4) {
-                    // y - x = (c_j - x) + (y - c_j): the first part from the hi/lo
-                    // centres, the second from the corners relative to the centre
-                    const double *cen = trial.center + 3 * (int64_t)j;
-                    float b[3], f1[3], f2[3];
-                    for (int d = 0; d < 3; ++d) {
-                        b[d] = (float)(cc[d] - cen[d]);
-                        f1[d] = (float)e1[d];
-                        f2[d] = (float)e2[d];
-                    }
-                    const float Jf = (float)J;
-                    const float4 p = s_p0[c];
-                    for (int q = 0; q < np; ++q) {
-                        const float *t = par ? TRI67.p7[q] : TRI67.p6[q];
-                        eval_h<FAM, float, CK>(dx + (b[0] + t[0] * f1[0] + t[1] * f2[0]),
-                                           dy + (b[1] + t[0] * f1[1] + t[1] * f2[1]),
-                                           dz + (b[2] + t[0] * f1[2] + t[1] * f2[2]), t[2] * Jf, p.y, p.z, p.w, nx0,
-                                           nx1, nx2, k, o, ki);
-                    }
+                    hsp_level3_f32<FAM, CK>(trial, j, par, dx, dy, dz, s_p0[c], nx0, nx1, nx2, k, o, ki);
                 } else {
+                    const double *cc = trial.corners + 12 * (int64_t)j;
+                    const double *n64 = trial.pts64 + 8 * base + 4;
+                    double e1[3], e2[3], nt[3];
+                    for (int d = 0; d < 3; ++d) { e1[d] = cc[3 + d] - cc[d]; e2[d] = cc[6 + d] - cc[d]; }
+                    cross3(e1, e2, nt);
+                    const double J = norm3(nt);
+                    const int np = par ? 13 : 12;
                     for (int q = 0; q < np; ++q) {
                         double xi, eta, w;
                         tri_pt(par ? 7 : 6, q, xi, eta, w);
@@ -245,6 +258,247 @@ __global__ void __launch_bounds__(BM_THREADS, sizeof(R) == 4 ? 4 : 1) k_regular_
     }
 }
 
+// ------------------------------------------------- two rows per thread
+// The Burton-Miller system (all four operators, A = DLP + c HSP and
+// B = SLP + c DLPt, complex64, FP32 quadrature, real wave number) through the
+// column loop of two_row.cuh.
+//
+// Bound by FP32 issue.  k_regular_bm ran the general dispatch whenever one of
+// a warp's 32 pairs was within 15.8 D, at the largest point count of the
+// warp: 240 instructions per warp and column against 80 for a far one.  Here
+// a pair costs its own points, the lists are
+//   0  15.8 <= d/D < 22.3: one point for SLP, DLP and DLPt, the level-1 rule for HSP
+//   1  3.6 <= d/D < 15.8: the level-1 rule for all but SLP, which has it below
+//      9.1 and one point above
+//   2  all others (closer, or within the FP32 guard band of a limit): classify_bm
+// and the four kernels of a point are summed as A and B at once.  Sphere of
+// 20480 triangles, k = 5, the whole system: 3.95 -> 2.82 ms (0.99 ms of stores
+// at the copy bandwidth), 206 instructions per 32 pairs on 11520 triangles,
+// 66% of the issue slots; 2 / 3 / 4 blocks per SM: 3.20 / 2.83 / 2.84 ms.
+struct Bm2Cols {
+    float4 hi[TWO_ROW_COLS], lo[TWO_ROW_COLS], p0[TWO_ROW_COLS];
+};
+
+// A += D_ DLP + H_ c HSP and B += ws S_ SLP + T_ c DLPt of one point, the
+// selected kernels; w4 = w J / (4 pi), rnx = -r.nx, rny = r.ny, nn = nx.ny
+template <int FAM, bool S_, bool D_, bool T_, bool H_>
+__device__ __forceinline__ void bm2_point(float rx, float ry, float rz, float w4, float rnx, float rny, float nn, float k,
+                                          float cr, float ci, float ws, float4 &ab)
+{
+    const float r2 = rx * rx + ry * ry + rz * rz;
+    const float rinv = rsqrtf(r2);
+    const float g = w4 * rinv, i2 = rinv * rinv, g2 = g * i2;
+    float s = 0.0f, c = 1.0f, kr = 0.0f;
+    if constexpr (FAM == FAM_HELMHOLTZ) {
+        kr = k * (r2 * rinv);
+        sincos_reduced(kr, s, c);
+    }
+    const float p = c + kr * s, q = kr * c - s;  // (1 + ikr) e^{-ikr}
+    if constexpr (D_ || H_) {
+        float vr = 0.0f, vi = 0.0f;
+        if constexpr (H_) {
+            const float aa = rnx * rny * i2, m = 3.0f * aa + nn;
+            const float u = m - aa * kr * kr, v = kr * m;
+            const float hr = u * c + v * s, hi = v * c - u * s;
+            vr = cr * hr - ci * hi;
+            vi = cr * hi + ci * hr;
+        }
+        if constexpr (D_) {
+            vr -= rny * p;
+            vi -= rny * q;
+        }
+        ab.x += g2 * vr;
+        ab.y += g2 * vi;
+    }
+    if constexpr (S_ || T_) {
+        float vr = 0.0f, vi = 0.0f;
+        if constexpr (T_) {
+            const float x = -i2 * rnx;
+            vr = x * (cr * p - ci * q);
+            vi = x * (cr * q + ci * p);
+        }
+        if constexpr (S_) {
+            vr += ws * c;
+            vi -= ws * s;
+        }
+        ab.z += g * vr;
+        ab.w += g * vi;
+    }
+}
+
+// list 2: the general dispatch of one pair; false when it is not regular.  Not
+// inlined, so that its registers are not the column loop's.
+template <int FAM>
+__device__ __noinline__ bool bm2_general(const BmArgs &a, int i, int j, float cr, float ci, float4 &ab)
+{
+    const DevMesh &test = a.test, &trial = a.trial;
+    const float4 ih = test.chi[i], il = test.clo[i], n0 = test.p0[i], pj = trial.p0[j];
+    const int par = il.w != 0.0f ? 1 : 0;
+    int ls, ld, lh;
+    float x, y, z;
+    if (classify_bm(ih, il, trial.chi[j], trial.clo[j], i, j, test.center, trial.center, trial.size, a.same_mesh, ls, ld,
+                    lh, x, y, z) != KIND_REGULAR)
+        return false;
+    const float k = a.k32;
+    const int64_t base = ((int64_t)j * 2 + par) * SLOTS;
+    BmSum<float> o;
+    for (int L = 0; L < 3; ++L) {
+        const bool bs = ls == L, bd = ld == L, bh = lh == L;
+        if (!(bs || bd || bh)) continue;
+        const float ws = bs ? 1.0f : 0.0f, wd = bd ? 1.0f : 0.0f, wh = bh ? 1.0f : 0.0f;
+        const int np = level_npts(3, par, L);
+        for (int q = 0; q < np; ++q) {
+            const float4 v = __ldg(trial.pts32 + 2 * (base + level_slot0(L) + q));
+            eval_bm<FAM, true, float>(x + v.x, y + v.y, z + v.z, v.w, pj.y, pj.z, pj.w, n0.y, n0.z, n0.w, k, ws, wd, wd,
+                                      wh, o);
+        }
+    }
+    if (lh == 3) hsp_level3_f32<FAM>(trial, j, par, x, y, z, pj, n0.y, n0.z, n0.w, k, o);
+    ab = make_float4(o.dr + cr * o.hr - ci * o.hi, o.di + cr * o.hi + ci * o.hr, o.sr + cr * o.tr - ci * o.ti,
+                     o.si + cr * o.ti + ci * o.tr);
+    return true;
+}
+
+template <int FAM>
+struct Bm2Op {
+    const BmArgs &a;
+    const Bm2Cols &cols;
+    int jb;
+    float2 *out_a, *out_b;  // of the block's first column
+    float k, cr, ci;
+
+    struct Row {
+        float4 hi, lo;
+        float nx, ny, nz;
+    };
+    __device__ __forceinline__ Row load(int i) const
+    {
+        const float4 p = a.test.p0[i];
+        return {a.test.chi[i], a.test.clo[i], p.y, p.z, p.w};
+    }
+    __device__ __forceinline__ bool far(float q) const { return q > Q_FAR_BM3; }
+    __device__ __forceinline__ int list(float q) const
+    {
+        // the FP32 guard band of classify_bm: outside it the class is the FP64 class
+        const float lo = q * (1.0f - 1e-5f), hi = q * (1.0f + 1e-5f);
+        if (hi < 2.25f) return -1;
+        if (lo >= 249.64f && hi < 497.29f) return 0;
+        if (lo >= 12.96f && (hi < 82.81f || (lo >= 82.81f && hi < 249.64f))) return 1;
+        return 2;
+    }
+    __device__ __forceinline__ void put(int i, int c, float4 ab) const
+    {
+        out_a[(int64_t)c * a.ld + i] = make_float2(ab.x, ab.y);
+        out_b[(int64_t)c * a.ld + i] = make_float2(ab.z, ab.w);
+    }
+    __device__ __forceinline__ void far_pair(const Row &r, int c, float x, float y, float z, int i) const
+    {
+        const float4 p = cols.p0[c];
+        float4 ab = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        bm2_point<FAM, true, true, true, true>(x, y, z, p.x, -(x * r.nx + y * r.ny + z * r.nz),
+                                               x * p.y + y * p.z + z * p.w, r.nx * p.y + r.ny * p.z + r.nz * p.w, k, cr,
+                                               ci, 1.0f, ab);
+        put(i, c, ab);
+    }
+    template <int LIST>
+    __device__ __forceinline__ void pair(int i, int c) const
+    {
+        constexpr float INV4PI = 0.0795774715459476679f;
+        const int j = jb + c;
+        if constexpr (LIST < 2) {
+            const Row r = load(i);
+            const float4 h = cols.hi[c], l = cols.lo[c];
+            const int par = r.lo.w != 0.0f ? 1 : 0;
+            const float x = (h.x - r.hi.x) + (l.x - r.lo.x), y = (h.y - r.hi.y) + (l.y - r.lo.y),
+                        z = (h.z - r.hi.z) + (l.z - r.lo.z);
+            const float4 p = cols.p0[c];
+            // flat trial triangles: nx.ny and r.ny are the same at every point
+            const float nn = r.nx * p.y + r.ny * p.z + r.nz * p.w, rny = x * p.y + y * p.z + z * p.w;
+            const bool far_s = LIST == 0 || (x * x + y * y + z * z) * h.w >= 82.81f;
+            float4 ab = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (LIST == 0)
+                bm2_point<FAM, true, true, true, false>(x, y, z, p.x, -(x * r.nx + y * r.ny + z * r.nz), rny, nn, k, cr,
+                                                        ci, 1.0f, ab);
+            else if (far_s)
+                bm2_point<FAM, true, false, false, false>(x, y, z, p.x, 0.0f, 0.0f, nn, k, cr, ci, 1.0f, ab);
+            const float4 *pts = a.trial.pts32 + 2 * (((int64_t)j * 2 + par) * SLOTS + level_slot0(1));
+            const int np = level_npts(3, par, 1);
+            for (int q = 0; q < np; ++q) {
+                const float4 v = __ldg(pts + 2 * q);
+                const float px = x + v.x, py = y + v.y, pz = z + v.z;
+                const float rnx = -(px * r.nx + py * r.ny + pz * r.nz);
+                if (LIST == 0)
+                    bm2_point<FAM, false, false, false, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci, 0.0f,
+                                                              ab);
+                else
+                    bm2_point<FAM, true, true, true, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci,
+                                                           far_s ? 0.0f : 1.0f, ab);
+            }
+            put(i, c, ab);
+        } else {
+            float4 ab;
+            if (bm2_general<FAM>(a, i, j, cr, ci, ab)) put(i, c, ab);
+        }
+    }
+};
+
+template <int FAM>
+__global__ void __launch_bounds__(TWO_ROW_THREADS, 3) k_regular_bm2(const __grid_constant__ BmArgs a, int cols_per_block)
+{
+    __shared__ Bm2Cols cols;
+    __shared__ TwoRowLists lists;
+    const int jb = a.j0 + blockIdx.y * cols_per_block;
+    const int ncols = min(cols_per_block, a.j1 - jb);
+    const int ib = blockIdx.x * TWO_ROW_ROWS;
+    if (threadIdx.x < ncols) {
+        cols.hi[threadIdx.x] = a.trial.chi[jb + threadIdx.x];
+        cols.lo[threadIdx.x] = a.trial.clo[jb + threadIdx.x];
+        float4 p = a.trial.p0[jb + threadIdx.x];
+        p.x *= 0.0795774715459476679f;  // the far rule's weight w J / (4 pi)
+        cols.p0[threadIdx.x] = p;
+    }
+    __syncthreads();
+    if (ib + 64 * (int)(threadIdx.x >> 5) >= a.test.n) return;
+    const int64_t off = (int64_t)(jb - a.j0) * a.ld;
+    const Bm2Op<FAM> op{a, cols, jb, reinterpret_cast<float2 *>(a.out_a) + off, reinterpret_cast<float2 *>(a.out_b) + off,
+                        a.k32, a.cre32[3], a.cim32[3]};
+    if (ib + TWO_ROW_ROWS <= a.test.n) two_row_columns<true>(op, lists, cols.hi, cols.lo, ib, a.test.n, ncols);
+    else two_row_columns<false>(op, lists, cols.hi, cols.lo, ib, a.test.n, ncols);
+}
+
+// three or four blocks of k_regular_bm2 (18 KB of shared memory each): the
+// 100 KB configuration, which the singular kernel beside it asks for as well,
+// so that an SM it starts on is configured for both
+static int bm2_carveout_percent() { return 44; }
+
+// all four operators are the Burton-Miller system: unit coefficients of SLP
+// and DLP, one coefficient c of DLPt and HSP, overwritten outputs
+static bool bm_system(const BmArgs &a)
+{
+    return !a.accumulate && a.cre[0] == 1.0 && a.cim[0] == 0.0 && a.cre[1] == 1.0 && a.cim[1] == 0.0 &&
+           a.cre[2] == a.cre[3] && a.cim[2] == a.cim[3];
+}
+
+template <int FAM>
+static cudaError_t launch_bm2(const BmArgs &a, cudaStream_t s)
+{
+    if (!bm_system(a)) return cudaErrorInvalidValue;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    static bool carveout_set[64] = {};
+    if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(k_regular_bm2<FAM>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                   bm2_carveout_percent());
+        if (e != cudaSuccess) return e;
+        carveout_set[dev] = true;
+    }
+    const int cpb = two_row_cols(a.test.n, a.j1 - a.j0, sms);
+    const dim3 grid((a.test.n + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS, (a.j1 - a.j0 + cpb - 1) / cpb);
+    k_regular_bm2<FAM><<<grid, TWO_ROW_THREADS, 0, s>>>(a, cpb);
+    return cudaGetLastError();
+}
+
 template <typename R, typename Out, int FAM>
 static void launch_bm_ops(const BmArgs &a, dim3 grid, cudaStream_t s)
 {
@@ -256,8 +510,13 @@ static void launch_bm_ops(const BmArgs &a, dim3 grid, cudaStream_t s)
             return;
         }
     }
-    if (all4) k_regular_bm<R, Out, FAM, true><<<grid, BM_THREADS, 0, s>>>(a);
-    else k_regular_bm<R, Out, FAM, false><<<grid, BM_THREADS, 0, s>>>(a);
+    if constexpr (sizeof(R) == 8 || sizeof(Out) == 16) {  // FP32 into complex64: k_regular_bm2
+        if (all4) {
+            k_regular_bm<R, Out, FAM, true><<<grid, BM_THREADS, 0, s>>>(a);
+            return;
+        }
+    }
+    k_regular_bm<R, Out, FAM, false><<<grid, BM_THREADS, 0, s>>>(a);
 }
 
 template <typename R, typename Out>
@@ -271,6 +530,9 @@ cudaError_t launch_assemble_regular_bm(const BmArgs &a, cudaStream_t s)
 {
     const int ncols = a.j1 - a.j0;
     if (a.test.n == 0 || ncols <= 0) return cudaSuccess;
+    const bool all4 = a.ops == (OP_SLP | OP_DLP | OP_DLPT | OP_HSP);
+    if (all4 && a.precision == 0 && a.dtype == 0 && a.k_im == 0.0)
+        return a.family == FAM_HELMHOLTZ ? launch_bm2<FAM_HELMHOLTZ>(a, s) : launch_bm2<FAM_LAPLACE>(a, s);
     dim3 grid((a.test.n + BM_THREADS - 1) / BM_THREADS, (ncols + BM_COLS - 1) / BM_COLS);
     if (a.precision == 0) {
         if (a.dtype == 0) launch_bm_fam<float, float2>(a, grid, s);
@@ -358,6 +620,13 @@ cudaError_t launch_assemble_singular_bm(const BmArgs &a, const NearList &near, c
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t total = (near.col_ptr ? near.nnz : 0) + (a.same_mesh ? (a.j1 - a.j0) : 0);
     if (total == 0) return cudaSuccess;
+    static bool carveout_set[64] = {};
+    if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(k_singular_bm<float2, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                             bm2_carveout_percent());
+        if (e != cudaSuccess) return e;
+        carveout_set[dev] = true;
+    }
     // at most two 4-warp blocks per SM (the FP64 pipe is the limit)
     const int64_t want = (total + BM_SING_THREADS - 1) / BM_SING_THREADS;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, 2 * (int64_t)sms));
