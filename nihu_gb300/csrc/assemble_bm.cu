@@ -272,18 +272,43 @@ __global__ void __launch_bounds__(BM_THREADS, sizeof(R) == 4 ? 4 : 1) k_regular_
 //      9.1 and one point above
 //   2  all others (closer, or within the FP32 guard band of a limit): classify_bm
 // and the four kernels of a point are summed as A and B at once.  Sphere of
-// 20480 triangles, k = 5, the whole system: 3.95 -> 2.82 ms (0.99 ms of stores
-// at the copy bandwidth), 206 instructions per 32 pairs on 11520 triangles,
-// 66% of the issue slots; 2 / 3 / 4 blocks per SM: 3.20 / 2.83 / 2.84 ms.
-struct Bm2Cols {
-    float4 hi[TWO_ROW_COLS], lo[TWO_ROW_COLS], p0[TWO_ROW_COLS];
+// 20480 triangles, k = 5, the whole system: 3.95 -> 2.72 ms (0.99 ms of stores
+// at the copy bandwidth; 7 blocks of 4 warps per SM, at 4 / 5 / 6 / 7 of them
+// 2.98 / 2.72 / 2.73 / 2.65 ms).
+// one point of all four kernels of two pairs: A = DLP + c HSP and
+// B = SLP + c DLPt; w4 = w J / (4 pi), rnx = -r.nx, nrny = -r.ny, nnn = -nx.ny
+struct Bm2Val {
+    f2 ar, ai, br, bi;
 };
+template <int FAM>
+__device__ __forceinline__ void bm2_point(f2 r2, f2 w4, f2 rnx, f2 nrny, f2 nnn, float k, float cr, float ci, Bm2Val &o)
+{
+    const f2 rinv = f2_rsqrt(r2);
+    const f2 g = w4 * rinv, i2 = rinv * rinv, g2 = g * i2;
+    const f2 naa = rnx * nrny * i2;              // -aa
+    const f2 nm = f2_fma(naa, f2_dup(3.0f), nnn);  // -m
+    f2 sn = f2_dup(0.0f), cs = f2_dup(1.0f), p = cs, q = sn, hr = nm, hi = sn;  // (hr, hi): -HSP / g2
+    if constexpr (FAM == FAM_HELMHOLTZ) {
+        const f2 r = r2 * rinv, kr = r * f2_dup(k), nkr = r * f2_dup(-k);
+        f2_sincos_reduced(nkr, sn, cs);  // e^{-ikr} = cs + i sn
+        p = f2_fma(nkr, sn, cs);          // (1 + ikr) e^{-ikr} = p + i q
+        q = f2_fma(kr, cs, sn);
+        const f2 u = f2_fma(naa * kr, nkr, nm), v = kr * nm;  // -[m - aa kr^2], -kr m
+        hr = f2_fma(v * f2_dup(-1.0f), sn, u * cs);
+        hi = f2_fma(v, cs, u * sn);
+    }
+    const f2 c_i = f2_dup(ci), nci = f2_dup(-ci), ncr = f2_dup(-cr);
+    o.ar = g2 * f2_fma(ncr, hr, f2_fma(c_i, hi, nrny * p));
+    o.ai = g2 * f2_fma(ncr, hi, f2_fma(nci, hr, nrny * q));
+    const f2 x = i2 * rnx;
+    o.br = g * f2_fma(x, f2_fma(c_i, q, ncr * p), cs);
+    o.bi = g * f2_fma(x, f2_fma(nci, p, ncr * q), sn);
+}
 
-// A += D_ DLP + H_ c HSP and B += ws S_ SLP + T_ c DLPt of one point, the
-// selected kernels; w4 = w J / (4 pi), rnx = -r.nx, rny = r.ny, nn = nx.ny
+// the same of one pair, rny = r.ny, nn = nx.ny (the listed ones)
 template <int FAM, bool S_, bool D_, bool T_, bool H_>
-__device__ __forceinline__ void bm2_point(float rx, float ry, float rz, float w4, float rnx, float rny, float nn, float k,
-                                          float cr, float ci, float ws, float4 &ab)
+__device__ __forceinline__ void bm2_point1(float rx, float ry, float rz, float w4, float rnx, float rny, float nn, float k,
+                                           float cr, float ci, float ws, float4 &ab)
 {
     const float r2 = rx * rx + ry * ry + rz * rz;
     const float rinv = rsqrtf(r2);
@@ -362,19 +387,18 @@ __device__ __noinline__ bool bm2_general(const BmArgs &a, int i, int j, float cr
 template <int FAM>
 struct Bm2Op {
     const BmArgs &a;
-    const Bm2Cols &cols;
+    const TwoRowShared &sh;
     int jb;
     float2 *out_a, *out_b;  // of the block's first column
     float k, cr, ci;
 
-    struct Row {
-        float4 hi, lo;
-        float nx, ny, nz;
+    struct Extra {  // the rows' unit normals, negated
+        f2 nx, ny, nz;
     };
-    __device__ __forceinline__ Row load(int i) const
+    __device__ __forceinline__ Extra extra(int i0, int i1) const
     {
-        const float4 p = a.test.p0[i];
-        return {a.test.chi[i], a.test.clo[i], p.y, p.z, p.w};
+        const float4 p = a.test.p0[i0], q = a.test.p0[i1];
+        return {f2_pack(-p.y, -q.y), f2_pack(-p.z, -q.z), f2_pack(-p.w, -q.w)};
     }
     __device__ __forceinline__ bool far(float q) const { return q > Q_FAR_BM3; }
     __device__ __forceinline__ int list(float q) const
@@ -386,84 +410,82 @@ struct Bm2Op {
         if (lo >= 12.96f && (hi < 82.81f || (lo >= 82.81f && hi < 249.64f))) return 1;
         return 2;
     }
-    __device__ __forceinline__ void put(int i, int c, float4 ab) const
+    __device__ __forceinline__ void put_one(int i, int c, float4 ab) const
     {
         out_a[(int64_t)c * a.ld + i] = make_float2(ab.x, ab.y);
         out_b[(int64_t)c * a.ld + i] = make_float2(ab.z, ab.w);
     }
-    __device__ __forceinline__ void far_pair(const Row &r, int c, float x, float y, float z, int i) const
+    using Val = Bm2Val;  // A and B of both rows
+    template <int H>
+    __device__ __forceinline__ void put(const Val &v, int c, int i) const
     {
-        const float4 p = cols.p0[c];
-        float4 ab = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        bm2_point<FAM, true, true, true, true>(x, y, z, p.x, -(x * r.nx + y * r.ny + z * r.nz),
-                                               x * p.y + y * p.z + z * p.w, r.nx * p.y + r.ny * p.z + r.nz * p.w, k, cr,
-                                               ci, 1.0f, ab);
-        put(i, c, ab);
+        float4 x, y;
+        f2_unpack(v.ar, x.x, y.x);
+        f2_unpack(v.ai, x.y, y.y);
+        f2_unpack(v.br, x.z, y.z);
+        f2_unpack(v.bi, x.w, y.w);
+        put_one(i, c, H == 0 ? x : y);
+    }
+    // the one-point rule of both rows
+    __device__ __forceinline__ void far_eval(const Extra &e, int c, f2 dx, f2 dy, f2 dz, f2 r2, Val &o) const
+    {
+        const TwoRowCol &t = sh.col[c];
+        bm2_point<FAM>(r2, t.w4, f2_fma(dz, e.nz, f2_fma(dy, e.ny, dx * e.nx)),
+                       f2_fma(dz, t.nz, f2_fma(dy, t.ny, dx * t.nx)) * f2_dup(-1.0f),
+                       f2_fma(e.nz, t.nz, f2_fma(e.ny, t.ny, e.nx * t.nx)), k, cr, ci, o);
     }
     template <int LIST>
     __device__ __forceinline__ void pair(int i, int c) const
     {
         constexpr float INV4PI = 0.0795774715459476679f;
-        const int j = jb + c;
-        if constexpr (LIST < 2) {
-            const Row r = load(i);
-            const float4 h = cols.hi[c], l = cols.lo[c];
-            const int par = r.lo.w != 0.0f ? 1 : 0;
-            const float x = (h.x - r.hi.x) + (l.x - r.lo.x), y = (h.y - r.hi.y) + (l.y - r.lo.y),
-                        z = (h.z - r.hi.z) + (l.z - r.lo.z);
-            const float4 p = cols.p0[c];
-            // flat trial triangles: nx.ny and r.ny are the same at every point
-            const float nn = r.nx * p.y + r.ny * p.z + r.nz * p.w, rny = x * p.y + y * p.z + z * p.w;
-            const bool far_s = LIST == 0 || (x * x + y * y + z * z) * h.w >= 82.81f;
-            float4 ab = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const TwoRowCol &t = sh.col[c];
+        const float3 d = t.diff(a.test, i);
+        const float4 p = t.p0(), n = a.test.p0[i];
+        const float nn = n.y * p.y + n.z * p.z + n.w * p.w;  // flat trial triangles: one normal
+        const bool far_s = LIST == 0 || (d.x * d.x + d.y * d.y + d.z * d.z) * t.hi().w >= 82.81f;
+        float4 ab = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (LIST == 0)
+            bm2_point1<FAM, true, true, true, false>(d.x, d.y, d.z, p.x, -(d.x * n.y + d.y * n.z + d.z * n.w),
+                                                     d.x * p.y + d.y * p.z + d.z * p.w, nn, k, cr, ci, 1.0f, ab);
+        else if (far_s)
+            bm2_point1<FAM, true, false, false, false>(d.x, d.y, d.z, p.x, 0.0f, 0.0f, nn, k, cr, ci, 1.0f, ab);
+        const int par = a.test.clo[i].w != 0.0f ? 1 : 0;
+        const float4 *pts = a.trial.pts32 + 2 * (((int64_t)(jb + c) * 2 + par) * SLOTS + level_slot0(1));
+        const int np = level_npts(3, par, 1);
+        for (int q = 0; q < np; ++q) {
+            const float4 v = __ldg(pts + 2 * q);
+            const float px = d.x + v.x, py = d.y + v.y, pz = d.z + v.z;
+            const float rnx = -(px * n.y + py * n.z + pz * n.w), rny = px * p.y + py * p.z + pz * p.w;
             if (LIST == 0)
-                bm2_point<FAM, true, true, true, false>(x, y, z, p.x, -(x * r.nx + y * r.ny + z * r.nz), rny, nn, k, cr,
-                                                        ci, 1.0f, ab);
-            else if (far_s)
-                bm2_point<FAM, true, false, false, false>(x, y, z, p.x, 0.0f, 0.0f, nn, k, cr, ci, 1.0f, ab);
-            const float4 *pts = a.trial.pts32 + 2 * (((int64_t)j * 2 + par) * SLOTS + level_slot0(1));
-            const int np = level_npts(3, par, 1);
-            for (int q = 0; q < np; ++q) {
-                const float4 v = __ldg(pts + 2 * q);
-                const float px = x + v.x, py = y + v.y, pz = z + v.z;
-                const float rnx = -(px * r.nx + py * r.ny + pz * r.nz);
-                if (LIST == 0)
-                    bm2_point<FAM, false, false, false, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci, 0.0f,
-                                                              ab);
-                else
-                    bm2_point<FAM, true, true, true, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci,
-                                                           far_s ? 0.0f : 1.0f, ab);
-            }
-            put(i, c, ab);
-        } else {
-            float4 ab;
-            if (bm2_general<FAM>(a, i, j, cr, ci, ab)) put(i, c, ab);
+                bm2_point1<FAM, false, false, false, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci, 0.0f, ab);
+            else
+                bm2_point1<FAM, true, true, true, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci,
+                                                        far_s ? 0.0f : 1.0f, ab);
         }
+        put_one(i, c, ab);
+    }
+    __device__ __forceinline__ void general(int i, int c) const
+    {
+        float4 ab;
+        if (bm2_general<FAM>(a, i, jb + c, cr, ci, ab)) put_one(i, c, ab);
     }
 };
 
 template <int FAM>
-__global__ void __launch_bounds__(TWO_ROW_THREADS, 3) k_regular_bm2(const __grid_constant__ BmArgs a, int cols_per_block)
+__global__ void __launch_bounds__(TWO_ROW_THREADS, 28 / TWO_ROW_WARPS) k_regular_bm2(const __grid_constant__ BmArgs a, int cols_per_block)
 {
-    __shared__ Bm2Cols cols;
-    __shared__ TwoRowLists lists;
+    __shared__ TwoRowShared sh;
     const int jb = a.j0 + blockIdx.y * cols_per_block;
     const int ncols = min(cols_per_block, a.j1 - jb);
     const int ib = blockIdx.x * TWO_ROW_ROWS;
-    if (threadIdx.x < ncols) {
-        cols.hi[threadIdx.x] = a.trial.chi[jb + threadIdx.x];
-        cols.lo[threadIdx.x] = a.trial.clo[jb + threadIdx.x];
-        float4 p = a.trial.p0[jb + threadIdx.x];
-        p.x *= 0.0795774715459476679f;  // the far rule's weight w J / (4 pi)
-        cols.p0[threadIdx.x] = p;
-    }
+    if (threadIdx.x < ncols) sh.stage(threadIdx.x, a.trial, jb + threadIdx.x);
     __syncthreads();
     if (ib + 64 * (int)(threadIdx.x >> 5) >= a.test.n) return;
     const int64_t off = (int64_t)(jb - a.j0) * a.ld;
-    const Bm2Op<FAM> op{a, cols, jb, reinterpret_cast<float2 *>(a.out_a) + off, reinterpret_cast<float2 *>(a.out_b) + off,
+    const Bm2Op<FAM> op{a, sh, jb, reinterpret_cast<float2 *>(a.out_a) + off, reinterpret_cast<float2 *>(a.out_b) + off,
                         a.k32, a.cre32[3], a.cim32[3]};
-    if (ib + TWO_ROW_ROWS <= a.test.n) two_row_columns<true>(op, lists, cols.hi, cols.lo, ib, a.test.n, ncols);
-    else two_row_columns<false>(op, lists, cols.hi, cols.lo, ib, a.test.n, ncols);
+    if (ib + TWO_ROW_ROWS <= a.test.n) two_row_columns<true>(op, sh, a.test, ib, ncols);
+    else two_row_columns<false>(op, sh, a.test, ib, ncols);
 }
 
 // three or four blocks of k_regular_bm2 (18 KB of shared memory each): the

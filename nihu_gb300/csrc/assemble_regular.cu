@@ -26,6 +26,7 @@
 
 #include "classify.cuh"
 #include "kernels.h"
+#include "two_row.cuh"
 
 namespace nihu {
 
@@ -466,247 +467,294 @@ __global__ void __launch_bounds__(REG_THREADS) k_regular(RegularArgs a)
 
 int regular_carveout_percent()
 {
-    // four blocks of k_regular2 (under 10 KB of shared memory each, plus the
-    // 1 KB the runtime reserves per block): the 64 KB configuration
-    return 25;
+    // four blocks of k_regular2 (18 KB of shared memory each, plus the 1 KB the
+    // runtime reserves per block): the 100 KB configuration
+    return 44;
 }
 
 // ------------------------------------------------- two rows per thread
-// The single wave number FP32 kernel for the common case (SLP and DLP, unit
-// scale, no accumulation, complex64 columns that allow 16-byte stores): each
-// thread owns two adjacent rows, so that one far vote, one set of shared
-// loads and the loop's bookkeeping serve two pairs, and each column takes one
-// 16-byte store per matrix for both rows.
+// The FP32 kernel of a single wave number into complex64 matrices, through the
+// column loop of two_row.cuh: a thread owns two rows, far columns take one
+// vote and two centroid points, the other pairs are listed by rule,
+//   0  9.1 <= d/D < 15.8: the centroid for the SLP, the level-1 points for the DLP
+//   1  2.8 <= d/D < 9.1: the level-1 points for both
+//   2  all others (closer, or within the FP32 guard band of a limit): classify_pair
+// (with one operator: its own one-point limit is "far", the pairs down to its
+// next limit list 1) and worked through one pair per lane, so that a pair
+// costs its own points and not its warp's largest count.  Points, levels and
+// their order are those of k_regular.
 //
-// A column whose 64 rows of a warp are not all far (about 13% of the warp
-// iterations on an icosphere, with some 45 of the 64 pairs not far) is not
-// evaluated in that warp: its far rows take the centroid there, certainly
-// nearly singular and self pairs are left to the singular kernel, and the
-// others are appended to the warp's list in shared memory (one 16-bit code
-// per pair: row in the block, column in the block), from the front when their
-// levels are certain without the FP64 check (SLP 1 point, DLP level 1: most
-// of them) and from the back otherwise.  Every REG2_CHUNK columns the warp
-// works through its two lists, one pair per lane, so that a pair's cost is
-// its own point count, not the largest one in its warp; warps do not wait
-// for one another.  A list holds every pair of a chunk, so it cannot
-// overflow, and a block needs under 10 KB of shared memory.  The points,
-// levels and their order are those of k_regular (the far path, the
-// certain-level path and the general dispatch).
-constexpr int REG2_THREADS = 256;
-constexpr int REG2_ROWS = 2 * REG2_THREADS;
-constexpr int REG2_CHUNK = 8;                  // columns per list flush
-constexpr int REG2_WLIST = 64 * REG2_CHUNK;    // every pair of a warp's chunk
-static_assert(REG2_ROWS <= 512 && REG_COLS <= 128, "a pair code is row (9 bits) | column << 9 in 16 bits");
+// Bound by FP32 issue, then by the stores (16 B a pair, 0.99 ms at the copy
+// bandwidth).  Sphere of 20480 triangles, SLP and DLP, the whole step with the
+// singular kernel beside it: 1.434 -> 1.386 ms against a form with scalar far
+// rows, one list for everything below 9.1 D and 512 x 32 tiles; 320 triangles,
+// this kernel: 110 -> 13 us (10 blocks before).  Tiles of 512 x 32 / 256 x 32 /
+// 256 x 16 / 256 x 8 / 128 x 32 pairs: 1.458 / 1.430 / 1.382 / 1.416 / 1.436 ms: a
+// block ends with its slowest warp, so small ones keep more warps running,
+// until the staging shows.  Listed pairs packed in twos spill (1.54 ms).
+// one point of the SLP (S_) and DLP (D_) kernels of two pairs, added to v:
+// w4 = w J / (4 pi), rn = r.n; e^{-ikr} / (4 pi r) and
+// -(1 + ikr) e^{-ikr} (r.n) / (4 pi r^3), CK: of a complex wave number k + i ki
+struct Reg2Val {
+    f2 sr, si, dr, di;
+};
+template <int FAM, bool CK, bool S_, bool D_>
+__device__ __forceinline__ void reg2_point(f2 r2, f2 w4, f2 rn, float k, float ki, Reg2Val &v)
+{
+    const f2 rinv = f2_rsqrt(r2);
+    const f2 g = w4 * rinv;
+    f2 f{};  // g (r.n) / r^2: minus the DLP's factor
+    if constexpr (D_) f = (g * (rinv * rinv)) * rn;
+    if constexpr (FAM == FAM_HELMHOLTZ) {
+        // with the sine of -kr: e^{-ikr} = cs + i sn; the DLP as -f (1 + ikr) e^{-ikr}
+        const f2 r = r2 * rinv, nkr = r * f2_dup(-k);
+        f2 sn, cs;
+        f2_sincos_reduced(nkr, sn, cs);
+        f2 na1 = f2_dup(-1.0f);
+        if constexpr (CK) {
+            float x, y;
+            f2_unpack(r * f2_dup(ki), x, y);
+            const f2 damp = f2_pack(expf(x), expf(y));
+            cs = cs * damp;
+            sn = sn * damp;
+            na1 = f2_fma(r, f2_dup(ki), na1);
+        }
+        if constexpr (S_) {
+            v.sr = f2_fma(g, cs, v.sr);
+            v.si = f2_fma(g, sn, v.si);
+        }
+        if constexpr (D_) {
+            // -(a1 + i kr)(cs + i sn) = (na1 cs + kr sn) + i (na1 sn - kr cs)
+            const f2 kr = r * f2_dup(k);
+            v.dr = f2_fma(f, f2_fma(kr, sn, na1 * cs), v.dr);
+            v.di = f2_fma(f, f2_fma(nkr, cs, na1 * sn), v.di);
+        }
+    } else {
+        if constexpr (S_) v.sr = v.sr + g;
+        if constexpr (D_) v.dr = f2_fma(f, f2_dup(-1.0f), v.dr);
+    }
+}
 
-// the far rule (the element centroid for both operators) with the weight
-// w J / (4 pi) given: e^{-ikr}/(4 pi r) and its DLP counterpart
-// -(1 + ikr) e^{-ikr} (r.n) / (4 pi r^3)
-template <int FAM>
-__device__ __forceinline__ void far_point(float rx, float ry, float rz, float w4, float nx, float ny, float nz,
-                                          float k, float &sr, float &si, float &dr, float &di)
+// the same of one pair (the listed ones: packed in twos they need more
+// registers than the loop leaves, and spill)
+template <int FAM, bool CK, bool S_, bool D_>
+__device__ __forceinline__ void reg2_point1(float rx, float ry, float rz, float w4, float rn, float k, float ki, float4 &o)
 {
     const float r2 = rx * rx + ry * ry + rz * rz;
     const float rinv = rsqrtf(r2);
     const float g = w4 * rinv;
-    const float rn = rx * nx + ry * ny + rz * nz;
-    const float f = -g * (rinv * rinv) * rn;
     if constexpr (FAM == FAM_HELMHOLTZ) {
-        const float kr = k * (r2 * rinv);
-        float sn, cs;
+        const float r = r2 * rinv, kr = k * r;
+        float sn, cs, a1 = 1.0f;
         sincos_reduced(kr, sn, cs);
-        sr = g * cs;
-        si = -g * sn;
-        dr = f * (cs + kr * sn);
-        di = f * (kr * cs - sn);
+        if constexpr (CK) {
+            const float damp = expf(ki * r);
+            sn *= damp;
+            cs *= damp;
+            a1 = 1.0f - ki * r;
+        }
+        if constexpr (S_) {
+            o.x += g * cs;
+            o.y -= g * sn;
+        }
+        if constexpr (D_) {
+            const float f = -g * (rinv * rinv) * rn;
+            o.z += f * (a1 * cs + kr * sn);
+            o.w += f * (kr * cs - a1 * sn);
+        }
     } else {
-        sr = g;
-        si = 0.0f;
-        dr = f;
-        di = 0.0f;
+        if constexpr (S_) o.x += g;
+        if constexpr (D_) o.z -= g * (rinv * rinv) * rn;
     }
 }
 
-// one pair by the general path of k_regular (classify_pair, the uniform loop
-// over the lane's points); false when the pair is not regular
-template <int FAM>
-__device__ __forceinline__ bool pair_general32(const RegularArgs &a, const float4 ih, const float4 il, int par, int i,
-                                               int j, const float4 jh, const float4 jl, int tnc, float k, float &sr,
-                                               float &si, float &dr, float &di)
+// list 2: one pair by the general dispatch (classify_pair, the uniform loop
+// over the pair's points); false when it is not regular.  Not inlined, so that
+// its registers are not the column loop's.
+template <int FAM, int OPS, bool CK>
+__device__ __noinline__ bool reg2_general(const RegularArgs &a, int i, int j, float4 &o)
 {
+    const DevMesh &test = a.test, &trial = a.trial;
+    const float4 ih = test.chi[i], il = test.clo[i], jl = trial.clo[j];
     int ls, ld;
     float dx, dy, dz;
-    const int kind = classify_pair(ih, il, jh, jl, i, j, a.test.center, a.trial.center, a.trial.size, a.same_mesh,
-                                   ls, ld, dx, dy, dz);
-    if (kind != KIND_REGULAR) return false;
-    const int nps = level_npts(tnc, par, ls);
-    const int npd = level_npts(tnc, par, ld);
+    if (classify_pair(ih, il, trial.chi[j], jl, i, j, test.center, trial.center, trial.size, a.same_mesh, ls, ld, dx, dy,
+                      dz) != KIND_REGULAR)
+        return false;
+    if (!(OPS & OP_SLP)) ls = ld;
+    if (!(OPS & OP_DLP)) ld = ls;
+    const int par = il.w != 0.0f ? 1 : 0, tnc = jl.w != 0.0f ? 4 : 3;
+    const float k = a.k32, ki = a.k_im32;
+    const int nps = level_npts(tnc, par, ls), npd = level_npts(tnc, par, ld);
     const int n_eval = ls == ld ? nps : nps + npd;
     const int64_t base = ((int64_t)j * 2 + par) * SLOTS;
-    sr = si = dr = di = 0.0f;
+    o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int q = 0; q < n_eval; ++q) {
         int slot;
         float ws, wd;
-        if (ls == ld) { slot = level_slot0(ls) + q; ws = 1.0f; wd = 1.0f; }
+        if (ls == ld) { slot = level_slot0(ls) + q; ws = wd = 1.0f; }
         else if (q < nps) { slot = level_slot0(ls) + q; ws = 1.0f; wd = 0.0f; }
         else { slot = level_slot0(ld) + q - nps; ws = 0.0f; wd = 1.0f; }
-        const float4 y = __ldg(a.trial.pts32 + 2 * (base + slot));
-        const float4 n = __ldg(a.trial.pts32 + 2 * (base + slot) + 1);
-        eval_point<FAM, float>(dx + y.x, dy + y.y, dz + y.z, y.w, n.x, n.y, n.z, k, ws, wd, sr, si, dr, di);
+        const float4 y = __ldg(trial.pts32 + 2 * (base + slot));
+        const float4 n = __ldg(trial.pts32 + 2 * (base + slot) + 1);
+        // r = (c_j - x) + (y - c_j): the hi/lo centre difference plus the point's
+        // offset from the trial centre
+        if constexpr (CK)
+            eval_point_ck<float>(dx + y.x, dy + y.y, dz + y.z, y.w, n.x, n.y, n.z, k, ki, ws, wd, o.x, o.y, o.z, o.w);
+        else
+            eval_point<FAM, float>(dx + y.x, dy + y.y, dz + y.z, y.w, n.x, n.y, n.z, k, ws, wd, o.x, o.y, o.z, o.w);
     }
     return true;
 }
 
-// one warp's deferred pairs: certain levels (the centroid for the SLP, the
-// level-1 points for the DLP) from the front of its list, the others
-// (classify_pair and the pair's own rule) from the back
-template <int FAM>
-__device__ __forceinline__ void regular2_flush(const RegularArgs &a, const unsigned short *wl, int nA, int nB,
-                                               int lane, int ib, int jb, const float4 *s_hi, const float4 *s_lo,
-                                               const int *s_nc, float2 *out_s, float2 *out_d, int64_t ldo, float k)
+// PLAIN: unit scale and no accumulation, so the stores carry no run-time checks
+template <int FAM, int OPS, bool CK, bool PLAIN>
+struct Reg2Op {
+    static constexpr bool DO_S = (OPS & OP_SLP) != 0, DO_D = (OPS & OP_DLP) != 0;
+    // (d/D)^2 of the one-point rule of every operator, and of the next limit
+    // below which list 1 ends (both: the DLP's 2.8, above the SLP's 1.8)
+    static constexpr float Q0 = DO_D ? 249.64f : 82.81f, Q1 = DO_D ? 7.84f : 3.24f;
+
+    const RegularArgs &a;
+    const TwoRowShared &sh;
+    int jb;
+    float2 *out_s, *out_d;  // of the block's first column
+    float k, ki;
+
+    struct Extra {};
+    __device__ __forceinline__ Extra extra(int, int) const { return {}; }
+    __device__ __forceinline__ bool far(float q) const { return q > Q0 * (1.0f + 1e-4f); }
+    __device__ __forceinline__ int list(float q) const
+    {
+        // the FP32 guard band of classify_pair: outside it the class is the FP64 class
+        const float lo = q * (1.0f - 1e-5f), hi = q * (1.0f + 1e-5f);
+        if (hi < 2.25f) return -1;  // certainly nearly singular
+        if (DO_S && DO_D && lo >= 82.81f && hi < Q0) return 0;
+        if (lo >= Q1 && hi < (DO_S ? 82.81f : Q0)) return 1;
+        return 2;
+    }
+    __device__ __forceinline__ void store(float2 *p, float re, float im) const
+    {
+        if constexpr (PLAIN) *p = make_float2(re, im);
+        else store_entry(p, re, im, a.alpha_re32, a.alpha_im32, a.unit_alpha != 0, a.accumulate);
+    }
+    __device__ __forceinline__ void put_one(int i, int c, const float4 &o) const
+    {
+        const int64_t off = (int64_t)c * a.ld + i;
+        if (DO_S) store(out_s + off, o.x, o.y);
+        if (DO_D) store(out_d + off, o.z, o.w);
+    }
+    using Val = Reg2Val;  // SLP and DLP of both rows
+    template <int H>
+    __device__ __forceinline__ void put(const Val &v, int c, int i) const
+    {
+        float4 x, y;
+        f2_unpack(v.sr, x.x, y.x);
+        f2_unpack(v.si, x.y, y.y);
+        f2_unpack(v.dr, x.z, y.z);
+        f2_unpack(v.di, x.w, y.w);
+        put_one(i, c, H == 0 ? x : y);
+    }
+    __device__ __forceinline__ static Val zero() { return {f2_dup(0.0f), f2_dup(0.0f), f2_dup(0.0f), f2_dup(0.0f)}; }
+    // the one-point rule of both rows
+    __device__ __forceinline__ void far_eval(const Extra &, int c, f2 dx, f2 dy, f2 dz, f2 r2, Val &v) const
+    {
+        const TwoRowCol &t = sh.col[c];
+        v = zero();
+        f2 rn{};
+        if constexpr (DO_D) rn = f2_fma(dz, t.nz, f2_fma(dy, t.ny, dx * t.nx));
+        reg2_point<FAM, CK, DO_S, DO_D>(r2, t.w4, rn, k, ki, v);
+    }
+    template <int LIST>
+    __device__ __forceinline__ void pair(int i, int c) const
+    {
+        constexpr float INV4PI = 0.0795774715459476679f;
+        if constexpr (LIST == 1 || (DO_S && DO_D)) {
+            constexpr bool PS = LIST == 1 && DO_S;  // the SLP at the level-1 points
+            const TwoRowCol &t = sh.col[c];
+            const float3 d = t.diff(a.test, i);
+            const float4 p = t.p0();
+            float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (LIST == 0) reg2_point1<FAM, CK, true, false>(d.x, d.y, d.z, p.x, 0.0f, k, ki, o);
+            const int par = a.test.clo[i].w != 0.0f ? 1 : 0;
+            const bool quad = a.trial.has_quad && a.trial.nc[jb + c] == 4;
+            const float4 *pts = a.trial.pts32 + 2 * (((int64_t)(jb + c) * 2 + par) * SLOTS + level_slot0(1));
+            const int np = level_npts(quad ? 4 : 3, par, 1);
+            for (int q = 0; q < np; ++q) {
+                const float4 v = __ldg(pts + 2 * q);
+                const float px = d.x + v.x, py = d.y + v.y, pz = d.z + v.z;
+                float rn = 0.0f;
+                if constexpr (DO_D) {
+                    // a flat triangle's points share the centre's normal (but not the
+                    // rounding of r.n, which the rule's sum averages)
+                    float4 n = make_float4(p.y, p.z, p.w, 0.0f);
+                    if (quad) n = __ldg(pts + 2 * q + 1);
+                    rn = px * n.x + py * n.y + pz * n.z;
+                }
+                reg2_point1<FAM, CK, PS, DO_D>(px, py, pz, v.w * INV4PI, rn, k, ki, o);
+            }
+            put_one(i, c, o);
+        }
+    }
+    __device__ __forceinline__ void general(int i, int c) const
+    {
+        float4 o;
+        if (reg2_general<FAM, OPS, CK>(a, i, jb + c, o)) put_one(i, c, o);
+    }
+};
+
+// 64 registers: three blocks fit beside the concurrent singular kernel's one
+template <int FAM, int OPS, bool CK, bool PLAIN>
+__global__ void __launch_bounds__(TWO_ROW_THREADS, 32 / TWO_ROW_WARPS) k_regular2(const __grid_constant__ RegularArgs a, int cols_per_block)
 {
-    const DevMesh &test = a.test;
-    const DevMesh &trial = a.trial;
-    for (int t = lane; t < nA; t += 32) {
-        const int code = wl[t];
-        const int i = ib + (code & 511), c = code >> 9, j = jb + c;
-        const float4 ih = test.chi[i], il = test.clo[i], h = s_hi[c], l = s_lo[c];
-        const int par = il.w != 0.0f ? 1 : 0;
-        const float mx = (h.x - ih.x) + (l.x - il.x), my = (h.y - ih.y) + (l.y - il.y),
-                    mz = (h.z - ih.z) + (l.z - il.z);
-        const int64_t base = ((int64_t)j * 2 + par) * SLOTS;
-        float sr = 0, si = 0, dr = 0, di = 0;
-        const float4 yc = __ldg(trial.pts32 + 2 * base), nc = __ldg(trial.pts32 + 2 * base + 1);
-        eval_point<FAM, float>(mx, my, mz, yc.w, nc.x, nc.y, nc.z, k, 1.0f, 0.0f, sr, si, dr, di);
-        const int npd = level_npts(s_nc[c], par, 1);
-        for (int q = 0; q < npd; ++q) {
-            const int64_t sl = base + level_slot0(1) + q;
-            const float4 y = __ldg(trial.pts32 + 2 * sl), n = __ldg(trial.pts32 + 2 * sl + 1);
-            eval_point<FAM, float>(mx + y.x, my + y.y, mz + y.z, y.w, n.x, n.y, n.z, k, 0.0f, 1.0f, sr, si, dr, di);
-        }
-        out_s[(int64_t)c * ldo + i] = make_float2(sr, si);
-        out_d[(int64_t)c * ldo + i] = make_float2(dr, di);
-    }
-    for (int t = lane; t < nB; t += 32) {
-        const int code = wl[REG2_WLIST - 1 - t];
-        const int i = ib + (code & 511), c = code >> 9, j = jb + c;
-        const float4 ih = test.chi[i], il = test.clo[i];
-        float sr, si, dr, di;
-        if (pair_general32<FAM>(a, ih, il, il.w != 0.0f ? 1 : 0, i, j, s_hi[c], s_lo[c], s_nc[c], k, sr, si, dr, di)) {
-            out_s[(int64_t)c * ldo + i] = make_float2(sr, si);
-            out_d[(int64_t)c * ldo + i] = make_float2(dr, di);
-        }
-    }
+    __shared__ TwoRowShared sh;
+    const int jb = a.j0 + blockIdx.y * cols_per_block;
+    const int ncols = min(cols_per_block, a.j1 - jb);
+    const int ib = blockIdx.x * TWO_ROW_ROWS;
+    if (threadIdx.x < ncols) sh.stage(threadIdx.x, a.trial, jb + threadIdx.x);
+    __syncthreads();
+    if (ib + 64 * (int)(threadIdx.x >> 5) >= a.test.n) return;
+    const int64_t off = (int64_t)(jb - a.j0) * a.ld;
+    const Reg2Op<FAM, OPS, CK, PLAIN> op{a, sh, jb, reinterpret_cast<float2 *>(a.out_s) + off,
+                                         reinterpret_cast<float2 *>(a.out_d) + off, a.k32, a.k_im32};
+    if (ib + TWO_ROW_ROWS <= a.test.n) two_row_columns<true>(op, sh, a.test, ib, ncols);
+    else two_row_columns<false>(op, sh, a.test, ib, ncols);
 }
 
-template <int FAM>
-// 64 registers: three blocks fit beside the concurrent singular kernel's one
-__global__ void __launch_bounds__(REG2_THREADS, 4) k_regular2(RegularArgs a)
+template <int FAM, int OPS, bool CK, bool PLAIN>
+static cudaError_t launch_regular2(const RegularArgs &a, cudaStream_t s)
 {
-    constexpr float INV4PI = 0.0795774715459476679f;
-    __shared__ float4 s_hi[REG_COLS], s_lo[REG_COLS], s_p0[REG_COLS];
-    __shared__ int s_nc[REG_COLS];
-    __shared__ unsigned short s_list[REG2_THREADS / 32][REG2_WLIST];
-    const DevMesh &test = a.test;
-    const DevMesh &trial = a.trial;
-    const int jb = a.j0 + blockIdx.y * REG_COLS;
-    const int ncols = min(REG_COLS, a.j1 - jb);
-    const int ib = blockIdx.x * REG2_ROWS;
-    if (threadIdx.x < ncols) {
-        s_hi[threadIdx.x] = trial.chi[jb + threadIdx.x];
-        s_lo[threadIdx.x] = trial.clo[jb + threadIdx.x];
-        s_nc[threadIdx.x] = trial.nc[jb + threadIdx.x];
-        float4 p = trial.p0[jb + threadIdx.x];
-        p.x *= INV4PI;  // the far rule's weight w J / (4 pi)
-        s_p0[threadIdx.x] = p;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    static bool carveout_set[64] = {};
+    if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(k_regular2<FAM, OPS, CK, PLAIN>,
+                                                   cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                   regular_carveout_percent());
+        if (e != cudaSuccess) return e;
+        carveout_set[dev] = true;
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int i0 = ib + 2 * threadIdx.x;
-    // warps wholly beyond the last row have nothing to do; a partial warp
-    // keeps its lanes (clamped rows, stores masked) so that the votes see
-    // every lane.  No block barrier follows.
-    if (i0 - 2 * lane >= test.n) return;
-    unsigned short *wl = s_list[threadIdx.x >> 5];
-    const float k = a.k32;
-    const int64_t ldo = a.ld;
-    float2 *const out_s = reinterpret_cast<float2 *>(a.out_s) + (int64_t)(jb - a.j0) * ldo;
-    float2 *const out_d = reinterpret_cast<float2 *>(a.out_d) + (int64_t)(jb - a.j0) * ldo;
-    const bool ok0 = i0 < test.n, ok1 = i0 + 1 < test.n;
-    const int r0 = ok0 ? i0 : test.n - 1, r1 = ok1 ? i0 + 1 : test.n - 1;
-    const float4 ih0 = test.chi[r0], il0 = test.clo[r0], ih1 = test.chi[r1], il1 = test.clo[r1];
-    const unsigned lt = (1u << lane) - 1u;
-    // FULL: every row of the block exists (all blocks but the last row
-    // block): the row checks drop out of the column loop
-    auto columns = [&](auto full_tag) {
-        constexpr bool FULL = decltype(full_tag)::value;
-        float2 *ps = out_s + i0, *pd = out_d + i0;
-        for (int c0 = 0; c0 < ncols; c0 += REG2_CHUNK) {
-            const int c1 = min(ncols, c0 + REG2_CHUNK);
-            int nA = 0, nB = 0;  // warp-uniform list lengths
-            for (int c = c0; c < c1; ++c, ps += ldo, pd += ldo) {
-                const float4 h = s_hi[c], l = s_lo[c];
-                // hi/lo centre differences of both rows (FP32 relative accuracy of r)
-                const float ax = (h.x - ih0.x) + (l.x - il0.x), ay = (h.y - ih0.y) + (l.y - il0.y),
-                            az = (h.z - ih0.z) + (l.z - il0.z);
-                const float bx = (h.x - ih1.x) + (l.x - il1.x), by = (h.y - ih1.y) + (l.y - il1.y),
-                            bz = (h.z - ih1.z) + (l.z - il1.z);
-                const float qa = (ax * ax + ay * ay + az * az) * h.w;
-                const float qb = (bx * bx + by * by + bz * bz) * h.w;
-                const bool fa = qa > Q_FAR, fb = qb > Q_FAR;
-                const float4 p = s_p0[c];
-                if (__all_sync(0xffffffffu, fa && fb)) {
-                    // far: the centroid for both operators, both rows
-                    float sr0, si0, dr0, di0, sr1, si1, dr1, di1;
-                    far_point<FAM>(ax, ay, az, p.x, p.y, p.z, p.w, k, sr0, si0, dr0, di0);
-                    far_point<FAM>(bx, by, bz, p.x, p.y, p.z, p.w, k, sr1, si1, dr1, di1);
-                    if (FULL || ok1) {
-                        *reinterpret_cast<float4 *>(ps) = make_float4(sr0, si0, sr1, si1);
-                        *reinterpret_cast<float4 *>(pd) = make_float4(dr0, di0, dr1, di1);
-                    } else if (ok0) {
-                        *ps = make_float2(sr0, si0);
-                        *pd = make_float2(dr0, di0);
-                    }
-                    continue;
-                }
-                // far rows here; the others deferred to the warp's lists
-                if (fa && (FULL || ok0)) {
-                    float sr, si, dr, di;
-                    far_point<FAM>(ax, ay, az, p.x, p.y, p.z, p.w, k, sr, si, dr, di);
-                    ps[0] = make_float2(sr, si);
-                    pd[0] = make_float2(dr, di);
-                }
-                if (fb && (FULL || ok1)) {
-                    float sr, si, dr, di;
-                    far_point<FAM>(bx, by, bz, p.x, p.y, p.z, p.w, k, sr, si, dr, di);
-                    ps[1] = make_float2(sr, si);
-                    pd[1] = make_float2(dr, di);
-                }
-                // the FP32 guard band of classify_pair: outside it the class is the FP64 class
-                const float alo = qa * (1.0f - 1e-5f), ahi = qa * (1.0f + 1e-5f);
-                const float blo = qb * (1.0f - 1e-5f), bhi = qb * (1.0f + 1e-5f);
-                const bool da = (FULL || ok0) && !fa && ahi >= 2.25f, db = (FULL || ok1) && !fb && bhi >= 2.25f;  // not certainly near
-                const bool ca = da && alo >= 82.81f && ahi < 249.64f, cb = db && blo >= 82.81f && bhi < 249.64f;
-                const unsigned mA0 = __ballot_sync(0xffffffffu, ca), mA1 = __ballot_sync(0xffffffffu, cb);
-                const unsigned mB0 = __ballot_sync(0xffffffffu, da && !ca), mB1 = __ballot_sync(0xffffffffu, db && !cb);
-                const int nA0 = __popc(mA0), nB0 = __popc(mB0);
-                const unsigned short code0 = (unsigned short)((i0 - ib) | (c << 9));
-                const unsigned short code1 = (unsigned short)((i0 + 1 - ib) | (c << 9));
-                if (ca) wl[nA + __popc(mA0 & lt)] = code0;
-                if (cb) wl[nA + nA0 + __popc(mA1 & lt)] = code1;
-                if (da && !ca) wl[REG2_WLIST - 1 - (nB + __popc(mB0 & lt))] = code0;
-                if (db && !cb) wl[REG2_WLIST - 1 - (nB + nB0 + __popc(mB1 & lt))] = code1;
-                nA += nA0 + __popc(mA1);
-                nB += nB0 + __popc(mB1);
-            }
-            if (nA + nB) {  // warp-uniform
-                __syncwarp();  // the list entries are visible to the whole warp
-                regular2_flush<FAM>(a, wl, nA, nB, lane, ib, jb, s_hi, s_lo, s_nc, out_s, out_d, ldo, k);
-                __syncwarp();  // read before the next chunk appends
-            }
-        }
-    };
-    if (ib + REG2_ROWS <= test.n) columns(std::true_type{});
-    else columns(std::false_type{});
+    const int cpb = two_row_cols(a.test.n, a.j1 - a.j0, sms);
+    const dim3 grid((a.test.n + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS, (a.j1 - a.j0 + cpb - 1) / cpb);
+    k_regular2<FAM, OPS, CK, PLAIN><<<grid, TWO_ROW_THREADS, 0, s>>>(a, cpb);
+    return cudaGetLastError();
+}
+
+template <int FAM, bool CK, bool PLAIN>
+static cudaError_t launch_regular2_ops(const RegularArgs &a, cudaStream_t s)
+{
+    if (a.ops == OP_SLP) return launch_regular2<FAM, OP_SLP, CK, PLAIN>(a, s);
+    if (a.ops == OP_DLP) return launch_regular2<FAM, OP_DLP, CK, PLAIN>(a, s);
+    return launch_regular2<FAM, OP_SLP | OP_DLP, CK, PLAIN>(a, s);
+}
+
+template <bool PLAIN>
+static cudaError_t launch_regular2_fam(const RegularArgs &a, cudaStream_t s)
+{
+    if (a.family != FAM_HELMHOLTZ) return launch_regular2_ops<FAM_LAPLACE, false, PLAIN>(a, s);
+    if (a.k_im != 0.0) return launch_regular2_ops<FAM_HELMHOLTZ, true, PLAIN>(a, s);
+    return launch_regular2_ops<FAM_HELMHOLTZ, false, PLAIN>(a, s);
 }
 
 // partial sums of the same row added in FP32 before one FP64 addition
@@ -784,12 +832,13 @@ template <typename R, typename Out>
 static void launch_fam(const RegularArgs &a, dim3 grid, cudaStream_t s)
 {
     const bool batch = a.nk > 1 || a.force_batch;
+    constexpr bool SINGLE = sizeof(R) == 8 || sizeof(Out) == 16;  // FP32 into complex64: k_regular2
     if (a.family == FAM_HELMHOLTZ) {
         if (batch) launch_ops<R, Out, FAM_HELMHOLTZ, true>(a, grid, s);
-        else launch_ops<R, Out, FAM_HELMHOLTZ, false>(a, grid, s);
+        else if constexpr (SINGLE) launch_ops<R, Out, FAM_HELMHOLTZ, false>(a, grid, s);
     } else {
         if (batch) launch_ops<R, Out, FAM_LAPLACE, true>(a, grid, s);
-        else launch_ops<R, Out, FAM_LAPLACE, false>(a, grid, s);
+        else if constexpr (SINGLE) launch_ops<R, Out, FAM_LAPLACE, false>(a, grid, s);
     }
 }
 
@@ -797,6 +846,8 @@ cudaError_t launch_assemble_regular(const RegularArgs &a, cudaStream_t s)
 {
     int ncols = a.j1 - a.j0;
     if (a.test.n == 0 || ncols <= 0) return cudaSuccess;
+    if (a.precision == 0 && a.dtype == 0 && a.nk <= 1 && !a.force_batch)
+        return a.unit_alpha && !a.accumulate ? launch_regular2_fam<true>(a, s) : launch_regular2_fam<false>(a, s);
     dim3 grid((a.test.n + REG_THREADS - 1) / REG_THREADS, (ncols + REG_COLS - 1) / REG_COLS);
     if (a.nk > 1 || a.force_batch) {
         // small meshes: split the wave numbers over gridDim.z (at least one tile of
@@ -814,27 +865,6 @@ cudaError_t launch_assemble_regular(const RegularArgs &a, cudaStream_t s)
             const int fmax = a.precision == 0 ? rhs_fmax_of<float>(a) : rhs_fmax_of<double>(a);
             grid.z = std::max<unsigned>(grid.z, (unsigned)((a.nk + fmax - 1) / fmax));
         }
-    }
-    if (a.precision == 0 && a.dtype == 0 && a.nk <= 1 && !a.force_batch && a.ops == (OP_SLP | OP_DLP) &&
-        a.unit_alpha && !a.accumulate && a.k_im == 0.0 && (a.ld & 1) == 0 &&
-        (reinterpret_cast<uintptr_t>(a.out_s) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.out_d) & 15) == 0) {
-        // two rows per thread with 16-byte stores
-        dim3 g2((a.test.n + REG2_ROWS - 1) / REG2_ROWS, grid.y);
-        int dev = 0;
-        cudaGetDevice(&dev);
-        static bool carveout_set[64] = {};
-        if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
-            cudaError_t e = cudaFuncSetAttribute(k_regular2<FAM_HELMHOLTZ>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                                 regular_carveout_percent());
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_regular2<FAM_LAPLACE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         regular_carveout_percent());
-            if (e != cudaSuccess) return e;
-            carveout_set[dev] = true;
-        }
-        if (a.family == FAM_HELMHOLTZ) k_regular2<FAM_HELMHOLTZ><<<g2, REG2_THREADS, 0, s>>>(a);
-        else k_regular2<FAM_LAPLACE><<<g2, REG2_THREADS, 0, s>>>(a);
-        return cudaGetLastError();
     }
     if (a.precision == 0) {
         if (a.dtype == 0) launch_fam<float, float2>(a, grid, s);

@@ -2,10 +2,11 @@
 // test rows: a warp owns 64 consecutive rows (lane and lane + 32, so that its
 // stores are two full 256-byte runs of a column whatever the leading
 // dimension), a block TWO_ROW_WARPS warps and up to TWO_ROW_COLS columns.
+// The two rows are the halves of packed FP32 pairs (f32x2.cuh), the column's
+// values are staged twice over, so that one instruction serves two pairs.
 //
-// A column whose 64 pairs are all far takes one vote and one evaluation per
-// row.  Otherwise its far rows are evaluated there, and the others appended
-// to the warp's lists in shared memory (a 16-bit code, row and column), each
+// Far rows of a column are evaluated in the loop.  The others are appended to
+// the warp's lists in shared memory (a 16-bit code, row and column), each
 // list one kind of work, and worked through every TWO_ROW_CHUNK columns, one
 // pair per lane: a warp runs one scheme with full lanes, where a direct
 // dispatch would make every lane wait for the largest point count of its 32
@@ -13,32 +14,82 @@
 // do not wait for one another.
 //
 // K, the operator, provides
-//   struct Row                      a test row's data, Row load(int i)
+//   struct Extra                    what it keeps of the thread's two rows; Extra extra(int i0, int i1)
 //   bool far(float q)               q = (d/D)^2 of a pair: certainly the one-point rule
 //   int list(float q)               of a pair that is not: 0, 1, 2, or -1 (left to the singular kernel)
-//   void far_pair(Row, c, dx, dy, dz, i)  evaluates and stores a far pair of column c (in the block)
-//   void pair<LIST>(i, c)           evaluates and stores a listed pair
+//   void far_eval(Extra, c, dx, dy, dz, r2, Val &)  both rows' far values in column c of the block
+//   void put<H>(Val, c, i)          stores half H (0, 1) at row i
+//   void pair<LIST>(i, c)           evaluates and stores a pair of list 0 or 1
+//   void general(i, c)              evaluates and stores a pair of list 2
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include "f32x2.cuh"
+#include "kernels.h"
+
 namespace nihu {
 
-constexpr int TWO_ROW_WARPS = 8;
+constexpr int TWO_ROW_WARPS = 4;
 constexpr int TWO_ROW_THREADS = 32 * TWO_ROW_WARPS;
 constexpr int TWO_ROW_ROWS = 64 * TWO_ROW_WARPS;
-constexpr int TWO_ROW_COLS = 32;
+constexpr int TWO_ROW_COLS = 16;
 constexpr int TWO_ROW_CHUNK = 8;
 constexpr int TWO_ROW_LIST = 64 * TWO_ROW_CHUNK;
 
+// one column's values, each as a pair of equal halves
+struct TwoRowCol {
+    f2 hx, hy, hz, iw;  // centre (hi), 1/D^2
+    f2 lx, ly, lz, w4;  // centre (lo), w J / (4 pi) of the one-point rule
+    f2 nx, ny, nz, nw4; // unit normal, -w4
+    __device__ __forceinline__ static float first(f2 x)
+    {
+        float a, b;
+        f2_unpack(x, a, b);
+        return a;
+    }
+    // the same as one scalar each
+    __device__ __forceinline__ float4 hi() const { return make_float4(first(hx), first(hy), first(hz), first(iw)); }
+    __device__ __forceinline__ float3 lo() const { return make_float3(first(lx), first(ly), first(lz)); }
+    __device__ __forceinline__ float4 p0() const { return make_float4(first(w4), first(nx), first(ny), first(nz)); }
+    // c_j - x_i from the hi/lo centres
+    __device__ __forceinline__ float3 diff(const DevMesh &test, int i) const
+    {
+        const float4 ih = test.chi[i], il = test.clo[i], h = hi();
+        const float3 l = lo();
+        return make_float3((h.x - ih.x) + (l.x - il.x), (h.y - ih.y) + (l.y - il.y), (h.z - ih.z) + (l.z - il.z));
+    }
+};
+
 // lists 0 (from the front) and 2 (from the back) share an array: together at
 // most every pair of a chunk
-struct TwoRowLists {
+struct TwoRowShared {
+    TwoRowCol col[TWO_ROW_COLS];
     unsigned short ac[TWO_ROW_WARPS][TWO_ROW_LIST], b[TWO_ROW_WARPS][TWO_ROW_LIST];
+    // stages column j of the trial mesh (call by one thread per column, then __syncthreads)
+    __device__ __forceinline__ void stage(int c, const DevMesh &trial, int j)
+    {
+        constexpr float INV4PI = 0.0795774715459476679f;
+        const float4 h = trial.chi[j], l = trial.clo[j], p = trial.p0[j];
+        TwoRowCol &t = col[c];
+        t.hx = f2_dup(h.x);
+        t.hy = f2_dup(h.y);
+        t.hz = f2_dup(h.z);
+        t.iw = f2_dup(h.w);
+        t.lx = f2_dup(l.x);
+        t.ly = f2_dup(l.y);
+        t.lz = f2_dup(l.z);
+        t.w4 = f2_dup(p.x * INV4PI);
+        t.nx = f2_dup(p.y);
+        t.ny = f2_dup(p.z);
+        t.nz = f2_dup(p.w);
+        t.nw4 = f2_dup(-p.x * INV4PI);
+    }
 };
 
 // columns per block: all TWO_ROW_COLS, or on a small mesh as few as keep
-// about four blocks per SM (one column: 320 elements, 320 blocks)
+// about four blocks per SM (320 elements: one column, 320 blocks; the regular
+// kernel 110 -> 13 us)
 inline int two_row_cols(int n_rows, int n_cols, int sms)
 {
     const int64_t rb = (n_rows + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS;
@@ -47,34 +98,47 @@ inline int two_row_cols(int n_rows, int n_cols, int sms)
 }
 
 template <bool FULL, class K>
-__device__ __forceinline__ void two_row_columns(const K &op, TwoRowLists &lists, const float4 *s_hi, const float4 *s_lo,
-                                                int ib, int n, int ncols)
+__device__ __forceinline__ void two_row_columns(const K &op, TwoRowShared &sh, const DevMesh &test, int ib, int ncols)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = test.n;
     const int i0 = ib + 64 * warp + lane, i1 = i0 + 32;
     const bool ok0 = FULL || i0 < n, ok1 = FULL || i1 < n;
-    const typename K::Row r0 = op.load(ok0 ? i0 : n - 1), r1 = op.load(ok1 ? i1 : n - 1);
-    unsigned short *la = lists.ac[warp], *lb = lists.b[warp];
+    const int r0 = ok0 ? i0 : n - 1, r1 = ok1 ? i1 : n - 1;
+    f2 nhx, nhy, nhz, nlx, nly, nlz;  // the rows' centres, negated
+    {
+        const float4 h0 = test.chi[r0], h1 = test.chi[r1], l0 = test.clo[r0], l1 = test.clo[r1];
+        nhx = f2_pack(-h0.x, -h1.x);
+        nhy = f2_pack(-h0.y, -h1.y);
+        nhz = f2_pack(-h0.z, -h1.z);
+        nlx = f2_pack(-l0.x, -l1.x);
+        nly = f2_pack(-l0.y, -l1.y);
+        nlz = f2_pack(-l0.z, -l1.z);
+    }
+    const typename K::Extra ex = op.extra(r0, r1);
+    unsigned short *la = sh.ac[warp], *lb = sh.b[warp];
     const unsigned lt = (1u << lane) - 1u;
     for (int c0 = 0; c0 < ncols; c0 += TWO_ROW_CHUNK) {
         const int c1 = min(ncols, c0 + TWO_ROW_CHUNK);
         int nA = 0, nB = 0, nC = 0;  // warp-uniform
         for (int c = c0; c < c1; ++c) {
-            const float4 h = s_hi[c], l = s_lo[c];
+            const TwoRowCol &t = sh.col[c];
             // hi/lo centre differences: FP32 relative accuracy of r
-            const float ax = (h.x - r0.hi.x) + (l.x - r0.lo.x), ay = (h.y - r0.hi.y) + (l.y - r0.lo.y),
-                        az = (h.z - r0.hi.z) + (l.z - r0.lo.z);
-            const float bx = (h.x - r1.hi.x) + (l.x - r1.lo.x), by = (h.y - r1.hi.y) + (l.y - r1.lo.y),
-                        bz = (h.z - r1.hi.z) + (l.z - r1.lo.z);
-            const float qa = (ax * ax + ay * ay + az * az) * h.w, qb = (bx * bx + by * by + bz * bz) * h.w;
+            const f2 dx = (t.hx + nhx) + (t.lx + nlx), dy = (t.hy + nhy) + (t.ly + nly), dz = (t.hz + nhz) + (t.lz + nlz);
+            // rounded in the order of the frequency batch's kernel: at large k r one
+            // more ulp of r is a visible phase
+            const f2 r2 = f2_fma(dz, dz, f2_fma(dx, dx, dy * dy));
+            float qa, qb;
+            f2_unpack(r2 * t.iw, qa, qb);
             const bool fa = op.far(qa), fb = op.far(qb);
-            if (__all_sync(0xffffffffu, fa && fb)) {
-                if (FULL || ok0) op.far_pair(r0, c, ax, ay, az, i0);
-                if (FULL || ok1) op.far_pair(r1, c, bx, by, bz, i1);
-                continue;
+            const bool all = __all_sync(0xffffffffu, fa && fb);
+            if (all || __any_sync(0xffffffffu, fa || fb)) {
+                typename K::Val v;
+                op.far_eval(ex, c, dx, dy, dz, r2, v);
+                if (fa && ok0) op.template put<0>(v, c, i0);
+                if (fb && ok1) op.template put<1>(v, c, i1);
             }
-            if (fa && ok0) op.far_pair(r0, c, ax, ay, az, i0);
-            if (fb && ok1) op.far_pair(r1, c, bx, by, bz, i1);
+            if (all) continue;
             const int ka = fa || !ok0 ? -1 : op.list(qa), kb = fb || !ok1 ? -1 : op.list(qb);
             const unsigned short ca = (unsigned short)(lane | (c << 6)), cb = (unsigned short)((lane + 32) | (c << 6));
             const unsigned a0 = __ballot_sync(0xffffffffu, ka == 0), a1 = __ballot_sync(0xffffffffu, kb == 0);
@@ -98,8 +162,7 @@ __device__ __forceinline__ void two_row_columns(const K &op, TwoRowLists &lists,
             __syncwarp();  // the entries are visible to the whole warp
             for (int t = lane; t < nA; t += 32) op.template pair<0>(wb + (la[t] & 63), la[t] >> 6);
             for (int t = lane; t < nB; t += 32) op.template pair<1>(wb + (lb[t] & 63), lb[t] >> 6);
-            for (int t = lane; t < nC; t += 32)
-                op.template pair<2>(wb + (la[TWO_ROW_LIST - 1 - t] & 63), la[TWO_ROW_LIST - 1 - t] >> 6);
+            for (int t = lane; t < nC; t += 32) op.general(wb + (la[TWO_ROW_LIST - 1 - t] & 63), la[TWO_ROW_LIST - 1 - t] >> 6);
             __syncwarp();  // read before the next chunk appends
         }
     }

@@ -64,3 +64,47 @@ def test_burton_miller_system(gpu_ctx, oracle, n, family):
     S, D, T, H = (oracle.assemble(mesh, mesh, fam, op, k, threads=8) for op in (oracle.SLP, oracle.DLP, oracle.DLPT, oracle.HSP))
     assert rel(A, D + c * H - 0.5 * np.eye(n)) <= 1e-5
     assert rel(B, S + c * T + c / 2 * np.eye(n)) <= 1e-5
+
+
+def collocation(ctx, mesh, test, family, ops, k, alpha=1.0, accumulate=0):
+    """SLP and DLP matrices through nihu_gb_assemble_c on the device; the outputs start at 7 + 3j."""
+    dm = g.api.DeviceMesh(ctx, *mesh)
+    tm = dm if test is mesh else g.api.DeviceMesh(ctx, *test)
+    return on_device(ctx, len(test[1]), len(mesh[1]), 1, lambda a, b, ld: g.lib().nihu_gb_assemble_c(
+        ctx.handle, tm.handle, dm.handle, family, ops, complex(k).real, complex(k).imag, complex(alpha).real,
+        complex(alpha).imag, g.REGULAR_FP32, g.C64, a, b, ld, accumulate, g.DEVICE))
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("k", [0.0, 3.0, 2.0 - 0.4j])
+@pytest.mark.parametrize("ops", [g.SLP, g.DLP, g.SLP | g.DLP])
+def test_collocation(gpu_ctx, oracle, n, k, ops):
+    mesh = part(n)
+    family, fam = (g.HELMHOLTZ_3D, oracle.HELMHOLTZ) if k else (g.LAPLACE_3D, oracle.LAPLACE)
+    got = collocation(gpu_ctx, mesh, mesh, family, ops, k)
+    for out, op in zip(got, (oracle.SLP, oracle.DLP)):
+        if ops & op:
+            ref = oracle.assemble(mesh, mesh, fam, op, k, threads=8)
+            assert np.abs(out - ref).max() <= 1e-5 * max(np.abs(ref).max(), 1e-3)  # one element's DLP is zero
+        else:
+            assert (out == np.complex64(7 + 3j)).all()
+
+
+@pytest.mark.parametrize("k", [3.0, 2.0 - 0.4j])
+def test_collocation_scaled_and_added(gpu_ctx, oracle, k):
+    mesh = part(319)
+    alpha = 0.5 - 2.0j
+    for out, op in zip(collocation(gpu_ctx, mesh, mesh, g.HELMHOLTZ_3D, g.SLP | g.DLP, k, alpha, 1), (oracle.SLP, oracle.DLP)):
+        ref = alpha * oracle.assemble(mesh, mesh, oracle.HELMHOLTZ, op, k, threads=8)
+        assert np.abs(out - (7 + 3j) - ref).max() <= 1e-5 * np.abs(ref).max() + 1e-6  # 7 + 3j + entry in FP32
+
+
+@pytest.mark.parametrize("quads", [False, True])
+def test_field_points(gpu_ctx, oracle, quads):
+    """Rows and columns of other meshes, one of them with both element types."""
+    trial = meshes.cube_sphere(5) if quads else part(333)
+    nodes, el = meshes.icosphere(2, radius=1.6)
+    test = (nodes, el[:75])
+    for a, b in ((test, trial), (trial, test)):
+        for out, op in zip(collocation(gpu_ctx, b, a, g.HELMHOLTZ_3D, g.SLP | g.DLP, 2.5), (oracle.SLP, oracle.DLP)):
+            assert rel(out, oracle.assemble(a, b, oracle.HELMHOLTZ, op, 2.5, same_mesh=False, threads=8)) <= 1e-5
