@@ -19,7 +19,7 @@ SOURCES = ["mesh.cu", "classify.cu", "assemble_regular.cu", "assemble_singular.c
            "noalloc.cu", "multi.cu", "gemm_tc.cu", "solve_persistent.cu", "assemble_bm.cu",
            "assemble_pairs.cu", "assemble_galerkin.cu"]
 HEADERS = ["common.cuh", "geom.cuh", "classify.cuh", "kernels.h", "linalg.h", "quad_rules.h", "solve_persistent.h",
-           "planar.cuh", "ffloat.cuh", "f32x2.cuh", "two_row.cuh", "singular_schemes.cuh", "bm_schemes.cuh"]
+           "planar.cuh", "ffloat.cuh", "static_ff.cuh", "f32x2.cuh", "two_row.cuh", "singular_schemes.cuh", "bm_schemes.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 

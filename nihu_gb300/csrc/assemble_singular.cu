@@ -27,10 +27,12 @@
 //      (nihu/library/nearly_singular_collocational_telles.hpp:85-110, telles_1987.hpp:44-113)
 // A frequency batch on a triangle evaluates the same 42-point dynamic sums
 // through their power series in k (near_moments / near_series below).
+#include <algorithm>
 #include <cmath>
 
 #include "kernels.h"
 #include "singular_schemes.cuh"
+#include "static_ff.cuh"
 
 namespace nihu {
 
@@ -465,6 +467,162 @@ __device__ __forceinline__ void singular_pairs(const RegularArgs &a, const NearL
     }
 }
 
+// the SLP self term of a constant triangle by 16 lanes: lane p < 13 takes
+// point p of the dynamic part, lane s < 3 side s of the static one
+template <bool CK>
+__device__ inline void self_tria_lanes(const Elem64 &e, int fam, cd k, const double x0[3], Acc &a, const Lanes<16> &g)
+{
+    double st = 0.0, vr = 0.0, vi = 0.0;
+    if (g.lane < 3) {
+        // side lane of corner_angles (nihu/library/plane_element_helper.hpp:42-74) and self_static
+        const int i0 = g.lane, i1 = i0 == 2 ? 0 : i0 + 1;
+        double R0[3], R1[3], C[3];
+        for (int d = 0; d < 3; ++d) {
+            R0[d] = e.c[i0][d] - x0[d];
+            R1[d] = e.c[i1][d] - x0[d];
+            C[d] = e.c[i0][d] - e.c[i1][d];
+        }
+        const double r0 = norm3(R0), r1 = norm3(R1), c = norm3(C);
+        const double cs = dot3(R0, R1) / (r0 * r1);
+        const double theta = cs >= 1.0 ? 0.0 : acos(cs), alpha = acos(dot3(R0, C) / (r0 * c));
+        st = r0 * sin(alpha) * log(tan((alpha + theta) / 2.0) / tan(alpha / 2.0));
+    }
+    if (fam == FAM_HELMHOLTZ && g.lane < 13) {
+        double e1[3], e2[3], nt[3], rv[3], xi, eta, w;
+        for (int d = 0; d < 3; ++d) { e1[d] = e.c[1][d] - e.c[0][d]; e2[d] = e.c[2][d] - e.c[0][d]; }
+        cross3(e1, e2, nt);
+        tri_pt(7, g.lane, xi, eta, w);
+        for (int d = 0; d < 3; ++d) rv[d] = e.c[0][d] + xi * e1[d] + eta * e2[d] - x0[d];
+        const double r = norm3(rv), wj = w * norm3(nt);
+        if constexpr (CK) {
+            const cd v = self_slp_point_ck(k, r);
+            vr = v.re * wj;
+            vi = v.im * wj;
+        } else {
+            // (e^{-ikr} - 1)/r = -ik e^{-ikr/2} sinc(kr/2)
+            double s, c;
+            sincos_bounded(k.re * r / 2.0, &s, &c, false);
+            const double sc = sinc_ref(k.re * r / 2.0);
+            vr = -k.re * s * sc * wj;
+            vi = -k.re * c * sc * wj;
+        }
+    }
+    a.sr += (g.sum(st) + g.sum(vr)) * INV_FOUR_PI;
+    a.si += g.sum(vi) * INV_FOUR_PI;
+}
+
+// The nearly singular and self pairs of a single wave number on triangles
+// under FP32 quadrature, G lanes per nearly singular pair and 16 (G = 1: one)
+// per self pair.  One thread per pair is the cheapest in instructions, but
+// its chain (about 4 000 dependent instructions, of which the FP64 set-up
+// takes 16 SM cycles each) is 93 us long however few pairs there are; with
+// the points and sides over four lanes it is 35 us.
+template <typename Out, bool CK, int G>
+__global__ void __launch_bounds__(SING_THREADS, 4) k_singular_tria(const __grid_constant__ RegularArgs a, NearList near)
+{
+    const int64_t p_begin = near.col_ptr ? near.col_ptr[a.j0] : 0;
+    const int64_t n_near = (near.col_ptr ? near.col_ptr[a.j1] : 0) - p_begin;
+    const int64_t n_self = a.same_mesh ? (int64_t)(min(a.j1, a.test.n) - a.j0) : 0;
+    const bool do_s = (a.ops & OP_SLP) != 0, do_d = (a.ops & OP_DLP) != 0;
+    const int fam = a.family;
+    const cd kc{a.k, a.k_im};
+    Out *out_s = reinterpret_cast<Out *>(a.out_s), *out_d = reinterpret_cast<Out *>(a.out_d);
+    const int64_t thread = (int64_t)blockIdx.x * SING_THREADS + threadIdx.x, threads = (int64_t)gridDim.x * SING_THREADS;
+    auto put = [&](int i, int j, const Acc &v) {
+        const int64_t off = (int64_t)(j - a.j0) * a.ld + i;
+        if (do_s) store64(out_s + off, v.sr, v.si, a.alpha_re, a.alpha_im, a.accumulate);
+        if (do_d) store64(out_d + off, v.dr, v.di, a.alpha_re, a.alpha_im, a.accumulate);
+    };
+    auto centre = [&](int i, double x0[3]) {
+        for (int d = 0; d < 3; ++d) x0[d] = a.test.center[3 * (int64_t)i + d];
+    };
+    const Lanes<G> g;
+    for (int64_t item = thread / G; item < n_near; item += threads / G) {
+        const int64_t p = p_begin + item;
+        const int i = near.rows[p], j = near_column(near.col_ptr, a.j0, a.j1, p);
+        double x0[3];
+        centre(i, x0);
+        Elem64 e;
+        load_elem(a.trial, j, e);
+        const double *frame = a.trial.frame + 16 * (int64_t)j;
+        Acc acc;
+        if constexpr (CK) {
+            near_dynamic_ck_ff<G>(e, kc, x0, do_s, do_d, acc, g);
+            Acc4 st;
+            near_static4_ff<G>(frame, e.c[0], x0, x0, OpSet{do_s, do_d, false, false}, st, g);
+            if (do_s) acc.sr += st.sr;
+            if (do_d) acc.dr += st.dr;
+        } else {
+            if (fam == FAM_HELMHOLTZ) near_dynamic_f32<G>(e, a.k, x0, do_s, do_d, acc, g);
+            near_static_f32<G>(e, frame, x0, do_s, do_d, acc, g);
+        }
+        if (g.lane == 0) put(i, j, acc);
+    }
+    // self terms: the DLP of a flat triangle over itself is zero
+    if constexpr (G > 1) {
+        const Lanes<16> h;
+        for (int64_t item = thread / 16; item < n_self; item += threads / 16) {
+            const int j = a.j0 + (int)item;
+            double x0[3];
+            centre(j, x0);
+            Elem64 e;
+            load_elem(a.trial, j, e);
+            Acc acc;
+            if (do_s) self_tria_lanes<CK>(e, fam, kc, x0, acc, h);
+            if (h.lane == 0) put(j, j, acc);
+        }
+    } else {
+        for (int64_t item = thread; item < n_self; item += threads) {
+            const int j = a.j0 + (int)item;
+            double x0[3];
+            centre(j, x0);
+            Elem64 e;
+            load_elem(a.trial, j, e);
+            Acc acc;
+            if (do_s) {
+                if constexpr (CK) self_tria_ck(e, fam, kc, x0, acc);
+                else self_tria(e, fam, a.k, x0, acc);
+            }
+            put(j, j, acc);
+        }
+    }
+}
+
+template <typename Out, bool CK, int G>
+static cudaError_t launch_singular_tria(const RegularArgs &a, const NearList &near, int64_t items, int sms, int dev,
+                                        cudaStream_t s)
+{
+    // the carveout of the regular kernel beside it, so that an SM this kernel
+    // starts on is configured for both
+    static bool carveout_set[64] = {};
+    if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(k_singular_tria<Out, CK, G>,
+                                                   cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                   regular_carveout_percent());
+        if (e != cudaSuccess) return e;
+        carveout_set[dev] = true;
+    }
+    const int64_t near_n = near.col_ptr ? near.nnz : 0, self_n = items - near_n;
+    const int64_t want = (std::max(near_n * G, self_n * (G > 1 ? 16 : 1)) + SING_THREADS - 1) / SING_THREADS;
+    // one block per SM beside the regular kernel, which bounds a large mesh
+    // (20480 triangles, 1 / 2 / 4 blocks: 1.368 / 1.385 / 1.439 ms a call); two
+    // where this kernel bounds: a complex wave number (4493 triangles:
+    // 0.364 / 0.279 / 0.283 ms), fewer than four items a thread, or several lanes per item
+    const int per_sm = G > 1 ? 4 : (CK || items <= 4 * (int64_t)sms * SING_THREADS ? 2 : 1);
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * per_sm));
+    k_singular_tria<Out, CK, G><<<blocks, SING_THREADS, 0, s>>>(a, near);
+    return cudaGetLastError();
+}
+
+template <typename Out, bool CK>
+static cudaError_t launch_singular_tria_g(const RegularArgs &a, const NearList &near, int64_t items, int g, int sms,
+                                          int dev, cudaStream_t s)
+{
+    if (g == 4) return launch_singular_tria<Out, CK, 4>(a, near, items, sms, dev, s);
+    if (g == 2) return launch_singular_tria<Out, CK, 2>(a, near, items, sms, dev, s);
+    return launch_singular_tria<Out, CK, 1>(a, near, items, sms, dev, s);
+}
+
 // held to 128 registers so that three blocks of the concurrent regular kernel
 // keep every SM beside this kernel's one (it would take 164 by itself, with
 // the FP32 dynamic part beside the FP64 schemes, which left room for two)
@@ -529,6 +687,21 @@ cudaError_t launch_assemble_singular(const RegularArgs &a, const NearList &near,
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t items = (near.col_ptr ? near.nnz : 0) + (a.same_mesh ? (a.j1 - a.j0) : 0);
+    if (items == 0) return cudaSuccess;
+    // triangles under FP32 quadrature (a complex wave number's float-float
+    // sums take |k| r <= 64, r < 3 D)
+    if (a.precision == 0 && a.dtype == 0 && a.nk <= 1 && !a.force_batch && !a.trial.has_quad &&
+        (a.k_im == 0.0 || (fabs(a.k) + fabs(a.k_im)) * 3.0 * a.trial_size_max <= 64.0)) {
+        // as many lanes per pair as still leave two blocks per SM: few pairs are
+        // bound by one pair's chain, many by the instructions (320 triangles, 4 800
+        // items, 1 / 2 / 4 / 8 lanes: 110 / 56 / 50 / 60 us a call; 5120 triangles,
+        // 78 000 items, this kernel: 161 / 182 / 229 / 348 us)
+        const int64_t room = 2 * (int64_t)sms * SING_THREADS;
+        const int g = items * 4 <= room ? 4 : (items * 2 <= room ? 2 : 1);
+        return a.k_im != 0.0 ? launch_singular_tria_g<float2, true>(a, near, items, g, sms, dev, s)
+                             : launch_singular_tria_g<float2, false>(a, near, items, g, sms, dev, s);
+    }
     // this kernel needs no shared memory, but the regular kernel's blocks
     // beside it do: the same carveout preference as theirs, so that an SM
     // this kernel starts on is configured for both (set once per device)
@@ -545,8 +718,7 @@ cudaError_t launch_assemble_singular(const RegularArgs &a, const NearList &near,
     // one 4-warp block per SM keeps the narrow FP64 pipe busy (a warp-wide
     // FP64 instruction occupies it for many cycles) and leave most of every SM
     // to the concurrently running regular kernel
-    int64_t total = (near.col_ptr ? near.nnz : 0) + (a.same_mesh ? (a.j1 - a.j0) : 0);
-    int64_t want = (total + SING_THREADS - 1) / SING_THREADS;
+    int64_t want = (items + SING_THREADS - 1) / SING_THREADS;
     // quads: the pairs' FP32 sums need more warps than the FP64 pipe does;
     // up to four blocks per SM once the regular kernel's blocks drain
     const int per_sm = (a.trial.has_quad && a.precision == 0 && a.nk <= 1 && !a.force_batch) ? 4 : 1;

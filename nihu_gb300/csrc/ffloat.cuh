@@ -175,6 +175,66 @@ __device__ __forceinline__ ff ff_log(ff v, int e)
     return ff_add(ff_add(ln, ff{t.y, t.z}), ff_quick(r.h, __fadd_rn(r.l, tail)));
 }
 
+// sin and cos of any x of moderate size: x less the nearest multiple n of pi/2
+// in three parts (exact products for |n| < 2^9), then ff_sincos and the quadrant
+__device__ __forceinline__ void ff_sincos_any(ff x, ff &s, ff &c)
+{
+    constexpr double HP = 1.57079632679489661923;
+    constexpr float P1 = 1.5703125f;  // 201 / 128
+    constexpr float P2 = (float)(HP - 1.5703125);
+    constexpr float P3 = (float)(HP - 1.5703125 - (double)P2);
+    const float n = rintf(x.h * 0.636619772367581343f);
+    ff r = ff_add(x, ff{__fmul_rn(-n, P1), 0.0f});
+    r = ff_add(r, ff_two_prod(-n, P2));
+    r = ff_add(r, ff{__fmul_rn(-n, P3), 0.0f});
+    ff sr, cr;
+    ff_sincos(r, sr, cr);
+    const int q = (int)n & 3;
+    s = (q & 1) ? cr : sr;
+    c = (q & 1) ? sr : cr;
+    if (q & 2) s = ff_neg(s);
+    if (q == 1 || q == 2) c = ff_neg(c);
+}
+
+// e^x for |x| < 80: x = n ln 2 / 16 + f, |f| <= ln 2 / 32, the 16 powers
+// 2^{j/16} from a table, the series of f with its small terms in FP32
+struct FfExp2 {
+    float h[16], l[16];
+    constexpr FfExp2() : h(), l()
+    {
+        for (int j = 0; j < 16; ++j) {
+            const double x = 0.69314718055994530942 * j / 16.0;
+            double v = 0.0, t = 1.0;
+            for (int k = 0; k < 30; ++k) {
+                v += t;
+                t *= x / (k + 1);
+            }
+            h[j] = (float)v;
+            l[j] = (float)(v - (double)(float)v);
+        }
+    }
+};
+static __device__ const FfExp2 FF_EXP2{};
+
+__device__ __forceinline__ ff ff_exp(ff x)
+{
+    constexpr double L = 0.69314718055994530942 / 16.0;
+    constexpr float L1 = 0.043304443359375f;  // 1419 / 32768
+    constexpr float L2 = (float)(L - 0.043304443359375);
+    constexpr float L3 = (float)(L - 0.043304443359375 - (double)L2);
+    const float n = rintf(x.h * 23.0831206542234142f);
+    ff f = ff_add(x, ff{__fmul_rn(-n, L1), 0.0f});
+    f = ff_add(f, ff_two_prod(-n, L2));
+    f = ff_add(f, ff{__fmul_rn(-n, L3), 0.0f});
+    const ff f2 = ff_mul(f, f);
+    const float tail = __fmul_rn(__fmul_rn(f2.h, f.h),
+                                 __fmaf_rn(f.h, __fmaf_rn(f.h, 1.0f / 120.0f, 1.0f / 24.0f), 1.0f / 6.0f));
+    const ff em1 = ff_add(f, ff_quick(0.5f * f2.h, __fadd_rn(0.5f * f2.l, tail)));  // e^f - 1
+    const int i = (int)n, j = i & 15;
+    const ff t{FF_EXP2.h[j], FF_EXP2.l[j]};
+    return ff_scale(ff_add(t, ff_mul(t, em1)), __int_as_float(((i >> 4) + 127) << 23));
+}
+
 // an n-point Gauss-Legendre rule's non-negative half as float-float:
 // nodes x (decreasing) and weights, the last node 0 when n is odd
 template <int N>
@@ -194,6 +254,27 @@ struct GaussHalfFF {
         }
     }
 };
+// the 42-point degree-14 triangle rule: (xi hi, xi lo, eta hi, eta lo) and (w hi, w lo)
+struct Tri14FF {
+    float4 x[42];
+    float2 w[42];
+    constexpr Tri14FF() : x(), w()
+    {
+        constexpr double d[NIHU_TRI_DATA_LEN] = NIHU_TRI_DATA;
+        constexpr int off[15] = NIHU_TRI_OFFSETS;
+        for (int q = 0; q < 42; ++q) {
+            const double a = d[3 * (off[14] + q)], b = d[3 * (off[14] + q) + 1], c = d[3 * (off[14] + q) + 2];
+            x[q].x = (float)a;
+            x[q].y = (float)(a - (double)(float)a);
+            x[q].z = (float)b;
+            x[q].w = (float)(b - (double)(float)b);
+            w[q].x = (float)c;
+            w[q].y = (float)(c - (double)(float)c);
+        }
+    }
+};
+static __device__ const Tri14FF TRI14_FF{};
+
 static __device__ const GaussHalfFF<6> GAUSS6_FF{};
 static __device__ const GaussHalfFF<21> GAUSS21_FF{};
 

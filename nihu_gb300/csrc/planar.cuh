@@ -195,6 +195,28 @@ __device__ __forceinline__ void frame_local(const double *__restrict__ frame, co
     }
 }
 
+// G lanes of a warp (a power of two, consecutive) that share one pair: each
+// takes every G-th point or side, sum() adds their parts in a fixed order and
+// gives every lane the total.  G = 1: one thread per pair.
+template <int G>
+struct Lanes {
+    int lane;
+    unsigned mask;
+    __device__ __forceinline__ Lanes()
+    {
+        const int l = threadIdx.x & 31;
+        lane = l & (G - 1);
+        mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (l & ~(G - 1));
+    }
+    template <class T>
+    __device__ __forceinline__ T sum(T v) const
+    {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+};
+
 // first column of trial element j >= j0 whose pairs include list entry p:
 // the largest j < j1 with col_ptr[j] <= p
 __device__ __forceinline__ int near_column(const int64_t *col_ptr, int j0, int j1, int64_t p)
@@ -275,44 +297,47 @@ __device__ __forceinline__ double sinc_ref(double x)
     return 1.0 - x * x / 6.0 * (1.0 - x * x / 20.0);
 }
 
-// the dynamic part sum_13 w J (e^{-ikr} - 1)/r of a constant triangle's SLP
-// self term for a complex (lossy) wave number, in the reference's form
+// one point, and the sum_13 w J (e^{-ikr} - 1)/r of the dynamic part of a
+// constant triangle's SLP self term for a complex (lossy) wave number, in the reference's form
 // -ik e^{-ikr/2} sinc(kr/2) (finite at r = 0: the rule holds the centroid),
 // with z = kr/2 complex:
 //   e^{-iz} = e^{Im z} (cos Re z - i sin Re z),
 //   sin z = sin Re z cosh Im z + i cos Re z sinh Im z,
 //   sinc z = sin z / z, or 1 - z^2/6 (1 - z^2/20) for |z| <= 1e-3 (nihu/util/math_functions.hpp:54-61)
+__device__ inline cd self_slp_point_ck(cd k, double r)
+{
+    const cd z{0.5 * k.re * r, 0.5 * k.im * r};
+    double sr, cr;
+    sincos(z.re, &sr, &cr);
+    const double ez = exp(z.im);
+    const cd em{ez * cr, -ez * sr};  // e^{-iz}
+    cd sc;
+    if (sqrt(z.re * z.re + z.im * z.im) > 1e-3) {
+        const cd sz{sr * cosh(z.im), cr * sinh(z.im)};
+        const double den = z.re * z.re + z.im * z.im;  // sz / z = sz conj(z) / |z|^2
+        sc = {(sz.re * z.re + sz.im * z.im) / den, (sz.im * z.re - sz.re * z.im) / den};
+    } else {
+        const cd z2 = cmul(z, z);
+        const cd t = {1.0 - z2.re / 20.0, -z2.im / 20.0};
+        const cd u = cmul(z2, t);
+        sc = {1.0 - u.re / 6.0, -u.im / 6.0};
+    }
+    return cmul(cd{k.im, -k.re}, cmul(em, sc));  // times -i k
+}
+
 __device__ inline cd tria_self_slp_dynamic_ck(const Elem64 &e, cd k, const double x0[3])
 {
     double e1[3], e2[3], nt[3];
     for (int d = 0; d < 3; ++d) { e1[d] = e.c[1][d] - e.c[0][d]; e2[d] = e.c[2][d] - e.c[0][d]; }
     cross3(e1, e2, nt);
     const double J = norm3(nt);
-    const cd mik{k.im, -k.re};  // -i k
     cd sum{0.0, 0.0};
     for (int p = 0; p < 13; ++p) {
         double xi, eta, w;
         tri_pt(7, p, xi, eta, w);
         double rv[3];
         for (int d = 0; d < 3; ++d) rv[d] = e.c[0][d] + xi * e1[d] + eta * e2[d] - x0[d];
-        const double r = norm3(rv);
-        const cd z{0.5 * k.re * r, 0.5 * k.im * r};
-        double sr, cr;
-        sincos(z.re, &sr, &cr);
-        const double ez = exp(z.im);
-        const cd em{ez * cr, -ez * sr};  // e^{-iz}
-        cd sc;
-        if (sqrt(z.re * z.re + z.im * z.im) > 1e-3) {
-            const cd sz{sr * cosh(z.im), cr * sinh(z.im)};
-            const double den = z.re * z.re + z.im * z.im;  // sz / z = sz conj(z) / |z|^2
-            sc = {(sz.re * z.re + sz.im * z.im) / den, (sz.im * z.re - sz.re * z.im) / den};
-        } else {
-            const cd z2 = cmul(z, z);
-            const cd t = {1.0 - z2.re / 20.0, -z2.im / 20.0};
-            const cd u = cmul(z2, t);
-            sc = {1.0 - u.re / 6.0, -u.im / 6.0};
-        }
-        sum = cadd(sum, cscale(cmul(mik, cmul(em, sc)), w * J));
+        sum = cadd(sum, cscale(self_slp_point_ck(k, norm3(rv)), w * J));
     }
     return sum;
 }

@@ -73,3 +73,24 @@ def test_static_parts_of_near_pairs(gpu_ctx, oracle, name, ops):
         # entries of coplanar elements vanish: the floor is then the element's own scale
         scale = max(big, {g.DLP: 1e-1, g.DLPT: 1e-1}.get(ops, 0.0))
         assert (err <= rel * np.abs(ref[ok]) + floor * scale).all(), (precision, err.max() / scale)
+
+
+@pytest.mark.parametrize("k", [2.0 - 0.4j, 7.0 + 1.0j, 20.0 - 4.0j, 150.0 - 1.0j])
+@pytest.mark.parametrize("n", [1, 20, 80, 319, 640, 1280])
+def test_near_entries_of_a_complex_wave_number(gpu_ctx, oracle, n, k):
+    """The nearly singular and self entries with their dynamic part: float-float
+    up to |k| r = 64, FP64 beyond; one, two or four lanes per pair by the number
+    of pairs.  Tolerance as above; E - 1 is formed from E, so the floor is
+    1e-8 of the largest entry here too."""
+    nodes, el = meshes.icosphere(3 if n > 320 else 2)
+    mesh = (nodes, np.ascontiguousarray(el[:n]))
+    m = g.create_mesh(*mesh)
+    sp = g.constant_view(m)
+    kind = oracle.classify(mesh, mesh, same_mesh=True)
+    rows, cols = (x.astype(np.int32) for x in np.nonzero(kind < 0))
+    for op, make in ((oracle.SLP, g.helmholtz_3d_SLP_kernel), (oracle.DLP, g.helmholtz_3d_DLP_kernel)):
+        got = np.zeros((n, n), np.complex64, order="F")
+        (g.dirac(sp) * g.create_integral_operator(make(k))[sp]).eval_into(got, ctx=gpu_ctx)
+        ref = oracle.assemble_pairs(mesh, mesh, oracle.HELMHOLTZ, op, k, rows, cols, same_mesh=True, threads=8)
+        err = np.abs(got[rows, cols] - ref)
+        assert (err <= 2e-7 * np.abs(ref) + 1e-8 * max(np.abs(ref).max(), 1e-3)).all(), err.max()
