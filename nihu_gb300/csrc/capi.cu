@@ -1,5 +1,6 @@
 // C ABI of the GB300 collocation BEM library (declared in include/nihu_gb300.h).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -1281,138 +1282,94 @@ nihu_gb_status nihu_gb_matvec(nihu_gb_ctx *ctx, int dtype_a, const void *A, int6
 
 namespace {
 
-struct Cplx {
-    double re, im;
-};
-
+// Restarted GMRES of one system with everything but the matvec in one
+// cooperative launch per step (gmres_step.cu): the host enqueues matvec and
+// step, one step ahead of the status word the device writes into mapped memory.
 nihu_gb_status gmres_device(nihu_gb_ctx *ctx, int dtype_a, const void *A, int64_t n, int64_t lda, const double2 *b,
                             double2 *x, int restart, int max_iters, double tol, int *iters_out, double *res_out)
 {
-    typedef std::complex<double> C;
     nihu_gb_status st;
     const int m = restart;
-    void *pV, *pw, *pt, *ppart, *pdot, *ph;
+    // the bound of restart times vector blocks that this solver has always had
+    if ((m + 1) * std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, 64)) > 4096)
+        return fail(ctx, NIHU_GB_ERR_INVALID_ARGUMENT, "GMRES restart too large");
+    const int splits = gemv_splits(n, n, dtype_a);
+    GmresPlan plan;
+    CK(gmres_step_plan(n, m, ctx->device, &plan));
+    void *pV, *ppart, *psmall, *pstate, *psums;
     if ((st = scratch(ctx, "gm_V", 16 * (size_t)n * (m + 1), &pV))) return st;
-    if ((st = scratch(ctx, "gm_w", 16 * (size_t)n, &pw))) return st;
-    if ((st = scratch(ctx, "gm_t", 16 * (size_t)n, &pt))) return st;
-    int splits = gemv_splits(n, n, dtype_a);
     if ((st = scratch(ctx, "mv_part", 16 * (size_t)splits * n, &ppart))) return st;
-    const int dblocks = dot_blocks(n);
-    if ((st = scratch(ctx, "gm_dot", 16 * (size_t)dblocks * (m + 1), &pdot))) return st;
-    if ((st = scratch(ctx, "gm_h", 16 * (size_t)(m + 1), &ph))) return st;
-    double2 *V = (double2 *)pV, *w = (double2 *)pw, *t = (double2 *)pt, *part = (double2 *)ppart;
-    double2 *dot = (double2 *)pdot, *dh = (double2 *)ph;
-    Cplx *hsm = (Cplx *)ctx->h_small;  // pinned host scratch, (m + 1) * dblocks <= 4096 entries
-    if ((size_t)(m + 1) * dblocks * sizeof(Cplx) > (1 << 16)) return fail(ctx, NIHU_GB_ERR_INVALID_ARGUMENT, "GMRES restart too large");
-
-    auto norm_of = [&](const double2 *v, double *out) -> nihu_gb_status {
-        CK(launch_multidot(v, n, 1, v, dot, dblocks, ctx->stream));
-        ctx->launches += 1;
-        CK(cudaMemcpyAsync(hsm, dot, 16 * dblocks, cudaMemcpyDeviceToHost, ctx->stream));
-        if ((st = sync(ctx))) return st;
-        double s = 0;
-        for (int q = 0; q < dblocks; ++q) s += hsm[q].re;
-        *out = std::sqrt(s);
-        return NIHU_GB_OK;
-    };
-    auto project = [&](int nv, std::vector<C> &h) -> nihu_gb_status {
-        // h = V[0..nv)^H w ; w -= V h
-        CK(launch_multidot(V, n, nv, w, dot, dblocks, ctx->stream));
-        ctx->launches += 1;
-        CK(cudaMemcpyAsync(hsm, dot, 16 * (size_t)dblocks * nv, cudaMemcpyDeviceToHost, ctx->stream));
-        if ((st = sync(ctx))) return st;
-        std::vector<double2> hv(nv);
-        for (int v = 0; v < nv; ++v) {
-            double sr = 0, si = 0;
-            for (int q = 0; q < dblocks; ++q) { sr += hsm[v * dblocks + q].re; si += hsm[v * dblocks + q].im; }
-            h[v] += C(sr, si);
-            hv[v] = make_double2(sr, si);
+    if ((st = scratch(ctx, "gm_small", 16 * gmres_small_entries(m), &psmall))) return st;
+    if ((st = scratch(ctx, "gm_state", 64, &pstate))) return st;
+    if ((st = scratch(ctx, "gm_sums", 16 * 2 * (size_t)(m + 1) * plan.ctas, &psums))) return st;
+    GmresHost *hs = (GmresHost *)ctx->h_small;  // pinned, mapped
+    hs->seq = 0;
+    hs->flag = GMRES_GO;
+    GmresStep a;
+    a.n = n;
+    a.restart = m;
+    a.max_iters = max_iters;
+    a.tol = tol;
+    a.splits = splits;
+    a.partial = (const double2 *)ppart;
+    a.V = (double2 *)pV;
+    a.small = (double2 *)psmall;
+    a.sums = (double2 *)psums;
+    a.state = (GmresState *)pstate;
+    a.active = (int *)((char *)pstate + 32);
+    a.host = hs;
+    int seq = 0;
+    // one matvec and one step (of the residual when rhs is given)
+    auto enqueue = [&](const double2 *v, const double2 *rhs, int k) -> nihu_gb_status {
+        {
+            Phase ph(ctx, dtype_a == 0 ? "gemv_c64" : "gemv_c128");
+            CK(launch_gemv_partial(dtype_a, A, n, n, lda, v, (double2 *)ppart, splits, ctx->stream, a.active));
         }
-        CK(cudaMemcpyAsync(dh, hv.data(), 16 * nv, cudaMemcpyHostToDevice, ctx->stream));
-        CK(launch_subtract_combo(V, n, nv, dh, w, ctx->stream));
-        ctx->launches += 1;
+        Phase ph(ctx, "gmres_step");
+        a.b = rhs;
+        a.k = k;
+        a.seq = ++seq;
+        CK(launch_gmres_step(a, plan, ctx->stream));
+        ctx->launches += 2;
         return NIHU_GB_OK;
     };
-
-    // r0 = b - A x ; reference normalises by the initial residual norm
-    CK(timed_gemv(ctx, dtype_a, A, n, n, lda, x, t, 1.0, 0.0, 0.0, 0.0, part, splits));
-    CK(launch_sub(b, t, w, n, ctx->stream));
-    ctx->launches += 1;
-    double r0norm;
-    if ((st = norm_of(w, &r0norm))) return st;
-    int iters = 0;
-    double rel = 0.0;
-    if (r0norm == 0.0) {
-        if (iters_out) *iters_out = 0;
-        if (res_out) *res_out = 0.0;
+    // wait until the device has done step `want`; an idle or failed stream ends the wait
+    auto wait = [&](int want) -> nihu_gb_status {
+        for (int64_t spin = 1; hs->seq < want; ++spin) {
+            if (spin % 1024) continue;
+            const cudaError_t e = cudaStreamQuery(ctx->stream);
+            if (e == cudaErrorNotReady) continue;
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "GMRES");
+            if (hs->seq < want) return fail(ctx, NIHU_GB_ERR_CUDA, "GMRES: the step's status did not arrive");
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);  // seq is the last word the device writes
         return NIHU_GB_OK;
-    }
-    double beta = r0norm;
-    std::vector<std::vector<C>> H(m + 1, std::vector<C>(m, C(0)));
-    std::vector<C> g(m + 1), cs(m), sn(m);
+    };
     bool converged = false;
+    a.first = 1;
     while (true) {
-        CK(launch_scale_copy(w, V, n, 1.0 / beta, ctx->stream));
-        ctx->launches += 1;
-        std::fill(g.begin(), g.end(), C(0));
-        g[0] = beta;
-        int kdone = 0;
-        bool stop = false;
+        // the cycle's residual (of the guess x, or after a restart)
+        CK(cudaMemsetAsync(a.active, 1, sizeof(int), ctx->stream));
+        if ((st = enqueue(x, b, 0))) return st;
+        a.first = 0;
         for (int k = 0; k < m; ++k) {
-            ++iters;
-            // w = A v_k
-            CK(timed_gemv(ctx, dtype_a, A, n, n, lda, V + (size_t)k * n, w, 1.0, 0.0, 0.0, 0.0, part, splits));
-            std::vector<C> h(k + 2, C(0));
-            if ((st = project(k + 1, h))) return st;
-            if ((st = project(k + 1, h))) return st;  // reorthogonalisation (CGS2)
-            double hn;
-            if ((st = norm_of(w, &hn))) return st;
-            h[k + 1] = hn;
-            if (hn > 0.0) {
-                CK(launch_scale_copy(w, V + (size_t)(k + 1) * n, n, 1.0 / hn, ctx->stream));
-                ctx->launches += 1;
-            }
-            // apply previous Givens rotations, then a new one
-            for (int i = 0; i < k; ++i) {
-                C a0 = h[i], a1 = h[i + 1];
-                h[i] = std::conj(cs[i]) * a0 + std::conj(sn[i]) * a1;
-                h[i + 1] = -sn[i] * a0 + cs[i] * a1;
-            }
-            double den = std::sqrt(std::norm(h[k]) + std::norm(h[k + 1]));
-            if (den == 0.0) { cs[k] = 1.0; sn[k] = 0.0; }
-            else { cs[k] = h[k] / den; sn[k] = h[k + 1] / den; }
-            C a0 = h[k], a1 = h[k + 1];
-            h[k] = std::conj(cs[k]) * a0 + std::conj(sn[k]) * a1;
-            h[k + 1] = 0.0;
-            C g0 = g[k], g1 = g[k + 1];
-            g[k] = std::conj(cs[k]) * g0 + std::conj(sn[k]) * g1;
-            g[k + 1] = -sn[k] * g0 + cs[k] * g1;
-            for (int i = 0; i <= k; ++i) H[i][k] = h[i];
-            kdone = k + 1;
-            rel = std::abs(g[k + 1]) / r0norm;
-            if (rel < tol || iters >= max_iters || hn == 0.0 || kdone == n) { stop = true; break; }
+            if ((st = enqueue(a.V + (size_t)k * n, nullptr, k))) return st;
+            if ((st = wait(seq - 1))) return st;
+            if (hs->flag != GMRES_GO) break;
         }
-        // y = H^{-1} g, x += V y
-        std::vector<C> yv(kdone);
-        for (int i = kdone - 1; i >= 0; --i) {
-            C s = g[i];
-            for (int j = i + 1; j < kdone; ++j) s -= H[i][j] * yv[j];
-            yv[i] = s / H[i][i];
+        if ((st = wait(seq))) return st;
+        const int flag = hs->flag;
+        if (flag == GMRES_ZERO) {  // the residual is zero
+            converged = true;
+            break;
         }
-        std::vector<double2> yd(kdone);
-        for (int i = 0; i < kdone; ++i) yd[i] = make_double2(yv[i].real(), yv[i].imag());
-        CK(cudaMemcpyAsync(dh, yd.data(), 16 * kdone, cudaMemcpyHostToDevice, ctx->stream));
-        CK(launch_add_combo(V, n, kdone, dh, x, ctx->stream));
+        CK(launch_gmres_update(a, x, ctx->stream));
         ctx->launches += 1;
-        if (rel < tol) converged = true;
-        if (stop) break;
-        // restart: w = b - A x
-        CK(timed_gemv(ctx, dtype_a, A, n, n, lda, x, t, 1.0, 0.0, 0.0, 0.0, part, splits));
-        CK(launch_sub(b, t, w, n, ctx->stream));
-        ctx->launches += 1;
-        if ((st = norm_of(w, &beta))) return st;
-        if (beta == 0.0) { converged = true; rel = 0.0; break; }
+        converged = hs->rel < tol;
+        if (flag == GMRES_STOP) break;
     }
+    const int iters = hs->iters;
+    const double rel = hs->rel;
     if ((st = sync(ctx))) return st;
     if (iters_out) *iters_out = iters;
     if (res_out) *res_out = rel;

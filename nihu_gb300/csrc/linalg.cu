@@ -1,5 +1,5 @@
-// Dense linear algebra of the solve: identity shift, streamed complex matvec,
-// GMRES building blocks (FP64 Gram-Schmidt) and an FP64 LU factorisation.
+// Dense linear algebra of the solve: identity shift, streamed complex matvec
+// and an LU factorisation.
 #include <algorithm>
 
 #include "kernels.h"
@@ -166,6 +166,7 @@ __global__ void k_gemv_reduce(const double2 *__restrict__ partial, int splits, i
     y += (int64_t)blockIdx.y * m;
     if (i >= m) return;
     double sr = 0.0, si = 0.0;
+#pragma unroll 8
     for (int s = 0; s < splits; ++s) {
         double2 v = partial[(int64_t)s * m + i];
         sr += v.x;
@@ -185,16 +186,17 @@ int gemv_splits(int64_t m, int64_t n, int dtype)
     int64_t row_blocks = (m + rows_per_block - 1) / rows_per_block;
     int64_t want = (int64_t)sms * 4;
     int64_t splits = (want + row_blocks - 1) / row_blocks;
-    // at least 256 columns per split keeps the partial traffic negligible
-    splits = min(splits, max((int64_t)1, n / 256));
+    // at least 32 columns per split: the partial sums (16 B a row) then stay below
+    // a sixteenth of the matrix, and a small or middling one fills the GPU (5120
+    // unknowns: 200 blocks and 46 us a product with 256 columns at least, 610
+    // blocks and 35 us now)
+    splits = min(splits, max((int64_t)1, n / 32));
     return (int)max((int64_t)1, min(splits, (int64_t)1024));
 }
 
-cudaError_t launch_gemv_batched(int dtype, const void *A, int64_t m, int64_t n, int64_t lda, int64_t a_stride,
-                                int batch, const double2 *x, double2 *y, double are, double aim, double bre,
-                                double bim, double2 *partial, int splits, cudaStream_t s, const int *active)
+static void gemv_partial(int dtype, const void *A, int64_t m, int64_t n, int64_t lda, int64_t a_stride, int batch,
+                         const double2 *x, double2 *partial, int splits, cudaStream_t s, const int *active)
 {
-    if (m == 0 || batch == 0) return cudaSuccess;
     int cols_per_split = (int)((n + splits - 1) / splits);
     if (n == 0) cols_per_split = 0;
     if (dtype == 0) {
@@ -206,6 +208,22 @@ cudaError_t launch_gemv_batched(int dtype, const void *A, int64_t m, int64_t n, 
         k_gemv_c128<<<grid, GEMV_THREADS, 0, s>>>((const double2 *)A, m, n, lda, x, partial, cols_per_split,
                                                    a_stride, active);
     }
+}
+
+cudaError_t launch_gemv_partial(int dtype, const void *A, int64_t m, int64_t n, int64_t lda, const double2 *x,
+                                double2 *partial, int splits, cudaStream_t s, const int *active)
+{
+    if (m == 0) return cudaSuccess;
+    gemv_partial(dtype, A, m, n, lda, 0, 1, x, partial, splits, s, active);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gemv_batched(int dtype, const void *A, int64_t m, int64_t n, int64_t lda, int64_t a_stride,
+                                int batch, const double2 *x, double2 *y, double are, double aim, double bre,
+                                double bim, double2 *partial, int splits, cudaStream_t s, const int *active)
+{
+    if (m == 0 || batch == 0) return cudaSuccess;
+    gemv_partial(dtype, A, m, n, lda, a_stride, batch, x, partial, splits, s, active);
     dim3 rgrid((unsigned)((m + 255) / 256), batch);
     k_gemv_reduce<<<rgrid, 256, 0, s>>>(partial, splits, m, y, are, aim, bre, bim, active);
     return cudaGetLastError();
@@ -257,126 +275,6 @@ cudaError_t launch_permute_segments(const double2 *src, double2 *dst, const int6
     if (count == 0 || max_len == 0) return cudaSuccess;
     dim3 g((unsigned)std::min(64, (max_len + 255) / 256), count);
     k_permute_segments<<<g, 256, 0, s>>>(src, dst, src_off, dst_off, len);
-    return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------ GMRES
-//
-// Classical Gram-Schmidt with one reorthogonalisation (CGS2) on FP64 basis
-// vectors V[0..k] (each n complex128, contiguous).  Dot products produce
-// per-block partial sums that the host adds (it needs them for the Givens
-// rotations anyway).
-
-constexpr int DOT_THREADS = 256;
-
-// partial[(v * gridDim.x + b)] = sum over the block's rows of conj(V[v]) . w
-__global__ void __launch_bounds__(DOT_THREADS) k_multidot(const double2 *__restrict__ V, int64_t n, int nv,
-                                                           const double2 *__restrict__ w, double2 *partial)
-{
-    __shared__ double sr[DOT_THREADS / 32], si[DOT_THREADS / 32];
-    const int v = blockIdx.y;
-    const double2 *vec = V + (int64_t)v * n;
-    double ar = 0.0, ai = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * DOT_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * DOT_THREADS) {
-        double2 a = vec[i], b = w[i];
-        ar += a.x * b.x + a.y * b.y;
-        ai += a.x * b.y - a.y * b.x;
-    }
-    ar = warp_sum(ar);
-    ai = warp_sum(ai);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { sr[wid] = ar; si[wid] = ai; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double tr = 0.0, ti = 0.0;
-        for (int k = 0; k < DOT_THREADS / 32; ++k) { tr += sr[k]; ti += si[k]; }
-        partial[(int64_t)v * gridDim.x + blockIdx.x] = make_double2(tr, ti);
-    }
-}
-
-// w -= sum_v V[v] h[v]
-__global__ void k_subtract_combo(const double2 *__restrict__ V, int64_t n, int nv, const double2 *__restrict__ h,
-                                 double2 *w)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double2 acc = w[i];
-    for (int v = 0; v < nv; ++v) {
-        double2 a = V[(int64_t)v * n + i], c = h[v];
-        acc.x -= a.x * c.x - a.y * c.y;
-        acc.y -= a.x * c.y + a.y * c.x;
-    }
-    w[i] = acc;
-}
-
-// x += sum_v V[v] y[v]
-__global__ void k_add_combo(const double2 *__restrict__ V, int64_t n, int nv, const double2 *__restrict__ yv,
-                            double2 *x)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double2 acc = x[i];
-    for (int v = 0; v < nv; ++v) {
-        double2 a = V[(int64_t)v * n + i], c = yv[v];
-        acc.x += a.x * c.x - a.y * c.y;
-        acc.y += a.x * c.y + a.y * c.x;
-    }
-    x[i] = acc;
-}
-
-// dst = src * s (real scale)
-__global__ void k_scale_copy(const double2 *__restrict__ src, double2 *dst, int64_t n, double s)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double2 v = src[i];
-    dst[i] = make_double2(v.x * s, v.y * s);
-}
-
-// dst = a - b
-__global__ void k_sub(const double2 *__restrict__ a, const double2 *__restrict__ b, double2 *dst, int64_t n)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double2 u = a[i], v = b[i];
-    dst[i] = make_double2(u.x - v.x, u.y - v.y);
-}
-
-int dot_blocks(int64_t n)
-{
-    int64_t b = (n + DOT_THREADS * 4 - 1) / (DOT_THREADS * 4);
-    return (int)max((int64_t)1, min(b, (int64_t)64));
-}
-
-cudaError_t launch_multidot(const double2 *V, int64_t n, int nv, const double2 *w, double2 *partial, int blocks,
-                            cudaStream_t s)
-{
-    dim3 grid(blocks, nv);
-    k_multidot<<<grid, DOT_THREADS, 0, s>>>(V, n, nv, w, partial);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_subtract_combo(const double2 *V, int64_t n, int nv, const double2 *h, double2 *w, cudaStream_t s)
-{
-    k_subtract_combo<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(V, n, nv, h, w);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_add_combo(const double2 *V, int64_t n, int nv, const double2 *y, double2 *x, cudaStream_t s)
-{
-    k_add_combo<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(V, n, nv, y, x);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_scale_copy(const double2 *src, double2 *dst, int64_t n, double sc, cudaStream_t s)
-{
-    k_scale_copy<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n, sc);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_sub(const double2 *a, const double2 *b, double2 *dst, int64_t n, cudaStream_t s)
-{
-    k_sub<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, dst, n);
     return cudaGetLastError();
 }
 

@@ -25,13 +25,44 @@ cudaError_t launch_add_identity_batched(int n, double are, double aim, int dtype
 cudaError_t launch_permute_segments(const double2 *src, double2 *dst, const int64_t *src_off, const int64_t *dst_off,
                                     const int *len, int count, int max_len, cudaStream_t s);
 
-int dot_blocks(int64_t n);
-cudaError_t launch_multidot(const double2 *V, int64_t n, int nv, const double2 *w, double2 *partial, int blocks,
-                            cudaStream_t s);
-cudaError_t launch_subtract_combo(const double2 *V, int64_t n, int nv, const double2 *h, double2 *w, cudaStream_t s);
-cudaError_t launch_add_combo(const double2 *V, int64_t n, int nv, const double2 *y, double2 *x, cudaStream_t s);
-cudaError_t launch_scale_copy(const double2 *src, double2 *dst, int64_t n, double sc, cudaStream_t s);
-cudaError_t launch_sub(const double2 *a, const double2 *b, double2 *dst, int64_t n, cudaStream_t s);
+// the matvec's partial sums alone (splits x n); active (device, may be NULL):
+// nothing is done when it is 0
+cudaError_t launch_gemv_partial(int dtype, const void *A, int64_t m, int64_t n, int64_t lda, const double2 *x,
+                                double2 *partial, int splits, cudaStream_t s, const int *active);
+
+// gmres_step.cu ---------------------------------------------------------
+// what the host watches (mapped memory): seq is written last
+constexpr int GMRES_GO = 0, GMRES_CYCLE = 1, GMRES_STOP = 2, GMRES_ZERO = 3;
+struct GmresHost {
+    volatile double rel;
+    volatile int iters, flag, seq;
+};
+struct GmresState {
+    double r0, rel;
+    int iters, kdone;
+};
+struct GmresStep {
+    int64_t n = 0;
+    int restart = 0, k = 0, first = 0, max_iters = 0, splits = 0, seq = 0;
+    double tol = 0.0;
+    const double2 *partial = nullptr;  // of A V_k, or (b set) of A x
+    const double2 *b = nullptr;        // set: begin a cycle from b - A x (first: of the solve)
+    double2 *V = nullptr;              // restart + 1 vectors
+    double2 *small = nullptr;          // H [(restart + 1) x restart], cs, sn [restart], g [restart + 1]
+    double2 *sums = nullptr;           // 2 x (restart + 1) x plan.ctas
+    GmresState *state = nullptr;
+    int *active = nullptr;  // 1 while the cycle runs
+    GmresHost *host = nullptr;
+};
+struct GmresPlan {
+    int ctas = 0;
+    size_t smem = 0;
+};
+inline size_t gmres_small_entries(int m) { return (size_t)(m + 1) * m + 2 * m + (m + 1); }
+cudaError_t gmres_step_plan(int64_t n, int restart, int device, GmresPlan *plan);
+cudaError_t launch_gmres_step(const GmresStep &a, const GmresPlan &plan, cudaStream_t s);
+// x += V H^{-1} g over the steps done
+cudaError_t launch_gmres_update(const GmresStep &a, double2 *x, cudaStream_t s);
 
 cudaError_t launch_lu_factor(double2 *A, int64_t n, int64_t lda, int *piv, int *info, int64_t *launches,
                              cudaStream_t s);
