@@ -386,6 +386,7 @@ __device__ __noinline__ bool bm2_general(const BmArgs &a, int i, int j, float cr
 
 template <int FAM>
 struct Bm2Op {
+    static constexpr int GENERAL_LANES = 1;
     const BmArgs &a;
     const TwoRowShared &sh;
     int jb;
@@ -400,7 +401,7 @@ struct Bm2Op {
         const float4 p = a.test.p0[i0], q = a.test.p0[i1];
         return {f2_pack(-p.y, -q.y), f2_pack(-p.z, -q.z), f2_pack(-p.w, -q.w)};
     }
-    __device__ __forceinline__ bool far(float q) const { return q > Q_FAR_BM3; }
+    __device__ __forceinline__ bool far(const Extra &, int, float q, float) const { return q > Q_FAR_BM3; }
     __device__ __forceinline__ int list(float q) const
     {
         // the FP32 guard band of classify_bm: outside it the class is the FP64 class

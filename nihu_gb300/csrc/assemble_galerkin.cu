@@ -26,12 +26,14 @@
 // vectors relative to the common node (matched pairs) or to the element
 // centres (unmatched pairs), which keeps FP32 relative accuracy as r -> 0.
 #include <algorithm>
+#include <initializer_list>
 #include <mutex>
 #include <vector>
 
 #include "classify.cuh"
 #include "kernels.h"
 #include "singular_schemes.cuh"
+#include "two_row.cuh"
 
 namespace nihu {
 
@@ -478,6 +480,549 @@ __global__ void __launch_bounds__(GAL_THREADS) k_galerkin_regular(GalArgs a)
     }
 }
 
+// ------------------------------------------------- two rows per thread
+// The FP32 kernel into complex64 matrices of a real wave number with unit
+// scale and no accumulation, through the column loop of two_row.cuh: far pairs
+// (both one-point rules) in the loop, the others listed by rule,
+//   0  9.1 <= d/D < 15.8: the centroids for the SLP, the level-1 product for the DLP
+//   1  2.8 <= d/D < 9.1: the level-1 product (9 points on triangles) for both
+//   2  all others: k_galerkin_regular's dispatch
+// A far pair also has to be out of its elements' reach (2 (D_i + D_j), within
+// which they may share a node), tested against the largest of the warp's rows;
+// lists 0 and 1 compare node ids within it.
+//
+// Bound by FP32 issue: the one-row kernel ran every lane of a warp through the
+// largest product of its 32 pairs.  5120 triangles, k = 5, both operators:
+// with the near pairs' kernel 1269 us before, 888 us now; alone 635 us (45% of
+// the issue slots; 96 registers, spill-free only up to 20 warps per SM, which
+// measured 30 us less than 28).
+struct Gal2Val {
+    f2 sr, si, dr, di;
+};
+// one point of two pairs; w4: the product of both weights and Jacobians over 4 pi
+template <int FAM, bool S_, bool D_>
+__device__ __forceinline__ void gal2_point(f2 rx, f2 ry, f2 rz, f2 w4, f2 nx, f2 ny, f2 nz, float k, Gal2Val &v)
+{
+    const f2 r2 = f2_fma(rz, rz, f2_fma(rx, rx, ry * ry));
+    const f2 rinv = f2_rsqrt(r2);
+    const f2 g = w4 * rinv;
+    f2 f{};  // g (r.n) / r^2: minus the DLP's factor
+    if constexpr (D_) f = (g * (rinv * rinv)) * f2_fma(rz, nz, f2_fma(ry, ny, rx * nx));
+    if constexpr (FAM == FAM_HELMHOLTZ) {
+        const f2 r = r2 * rinv, kr = r * f2_dup(k), nkr = r * f2_dup(-k);
+        f2 sn, cs;
+        f2_sincos_reduced(nkr, sn, cs);  // e^{-ikr} = cs + i sn
+        if constexpr (S_) {
+            v.sr = f2_fma(g, cs, v.sr);
+            v.si = f2_fma(g, sn, v.si);
+        }
+        if constexpr (D_) {
+            const f2 nf = f * f2_dup(-1.0f);
+            v.dr = f2_fma(nf, f2_fma(nkr, sn, cs), v.dr);
+            v.di = f2_fma(nf, f2_fma(kr, cs, sn), v.di);
+        }
+    } else {
+        if constexpr (S_) v.sr = v.sr + g;
+        if constexpr (D_) v.dr = f2_fma(f, f2_dup(-1.0f), v.dr);
+    }
+}
+
+constexpr int GAL2_LANES = 4;  // lanes per pair of list 2, whose products have up to 45 points
+struct Gal2Sums {
+    float sr = 0.0f, si = 0.0f, dr = 0.0f, di = 0.0f;
+};
+
+// one point of one pair
+template <int FAM, bool S_, bool D_>
+__device__ __forceinline__ void gal2_point1(float rx, float ry, float rz, float w4, float nx, float ny, float nz, float k,
+                                            Gal2Sums &o)
+{
+    const float r2 = rx * rx + ry * ry + rz * rz;
+    const float rinv = rsqrtf(r2);
+    const float g = w4 * rinv;
+    float sn = 0.0f, cs = 1.0f, kr = 0.0f;
+    if constexpr (FAM == FAM_HELMHOLTZ) {
+        kr = k * (r2 * rinv);
+        sincos_reduced(kr, sn, cs);
+    }
+    if constexpr (S_) {
+        o.sr += g * cs;
+        o.si -= g * sn;
+    }
+    if constexpr (D_) {
+        const float f = -g * (rinv * rinv) * (rx * nx + ry * ny + rz * nz);
+        o.dr += f * (cs + kr * sn);
+        o.di += f * (kr * cs - sn);
+    }
+}
+
+// k_galerkin_regular's general dispatch of one pair by GAL2_LANES lanes (each
+// takes every GAL2_LANES-th test point; every lane gets the sums); false when
+// it is left to the near kernel or listed as an extra pair
+template <int FAM, int OPS>
+__device__ __noinline__ bool gal2_general(const GalArgs &a, int i, int j, Gal2Sums &o)
+{
+    constexpr bool DO_S = (OPS & OP_SLP) != 0, DO_D = (OPS & OP_DLP) != 0;
+    const Lanes<GAL2_LANES> lanes;
+    const DevMesh &test = a.test, &trial = a.trial;
+    const float4 ih = test.chi[i], il = test.clo[i], jh = trial.chi[j], jl = trial.clo[j];
+    int ls, ld;
+    float dx, dy, dz;
+    if (classify_pair(ih, il, jh, jl, i, j, test.center, trial.center, trial.size, a.same_mesh, ls, ld, dx, dy, dz) !=
+        KIND_REGULAR)
+        return false;
+    const int inc = test.nc[i], jnc = trial.nc[j];
+    int ind1, ind2;
+    if (a.same_mesh && common_nodes(test.nid[i], inc, trial.nid[j], jnc, ind1, ind2) > 0) {
+        // a node shared beyond 1.5 D (strongly graded mesh): singular rule
+        if (lanes.lane == 0) {
+            const unsigned slot = atomicAdd(a.n_extra, 1u);
+            if (slot < (unsigned)a.extra_cap) a.extra[slot] = make_int2(i, j);
+            else atomicCAS(a.err, 0, -1);
+        }
+        return false;
+    }
+    if (!DO_S) ls = ld;
+    if (!DO_D) ld = ls;
+    const int cmax = (il.w != 0.0f || jl.w != 0.0f) ? 1 : 0;
+    const int64_t bi = ((int64_t)i * 2 + cmax) * SLOTS, bj = ((int64_t)j * 2 + cmax) * SLOTS;
+    for (int pass = 0; pass < (ls == ld ? 1 : 2); ++pass) {
+        const int L = pass == 0 ? ls : ld;
+        const float ws = (DO_S && ls == L) ? 1.0f : 0.0f, wd = (DO_D && ld == L) ? 1.0f : 0.0f;
+        const int npi = level_npts(inc, cmax, L), npj = level_npts(jnc, cmax, L);
+        for (int p = lanes.lane; p < npi; p += GAL2_LANES) {
+            const float4 x = __ldg(test.pts32 + 2 * (bi + level_slot0(L) + p));
+            for (int q = 0; q < npj; ++q) {
+                const float4 y = __ldg(trial.pts32 + 2 * (bj + level_slot0(L) + q));
+                const float4 n = __ldg(trial.pts32 + 2 * (bj + level_slot0(L) + q) + 1);
+                eval_point<FAM, float>(dx + (y.x - x.x), dy + (y.y - x.y), dz + (y.z - x.z), y.w, n.x, n.y, n.z, a.k32,
+                                       ws * x.w, wd * x.w, o.sr, o.si, o.dr, o.di);
+            }
+        }
+    }
+    o.sr = lanes.sum(o.sr);
+    o.si = lanes.sum(o.si);
+    o.dr = lanes.sum(o.dr);
+    o.di = lanes.sum(o.di);
+    return true;
+}
+
+template <int FAM, int OPS>
+struct Gal2Op {
+    static constexpr bool DO_S = (OPS & OP_SLP) != 0, DO_D = (OPS & OP_DLP) != 0;
+    static constexpr float Q0 = DO_D ? 249.64f : 82.81f, Q1 = DO_D ? 7.84f : 3.24f;  // as Reg2Op
+    static constexpr int GENERAL_LANES = GAL2_LANES;
+
+    const GalArgs &a;
+    const TwoRowShared &sh;
+    int jb;
+    float2 *out_s, *out_d;
+    float k;
+
+    struct Extra {
+        f2 area;
+        float size;  // the largest of the warp's rows
+    };
+    __device__ __forceinline__ Extra extra(int i0, int i1) const
+    {
+        float d = fmaxf(rsqrtf(a.test.chi[i0].w), rsqrtf(a.test.chi[i1].w));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) d = fmaxf(d, __shfl_xor_sync(0xffffffffu, d, o));
+        return {f2_pack(a.test.p0[i0].x, a.test.p0[i1].x), d};
+    }
+    // beyond the distance at which elements of sizes 1/sqrt(iw) and d may share a node
+    __device__ __forceinline__ bool apart(float iw, float d, float r2) const
+    {
+        const float reach = 2.0f * (rsqrtf(iw) + d);
+        return !a.same_mesh || r2 > 1.01f * reach * reach;
+    }
+    __device__ __forceinline__ bool far(const Extra &e, int c, float q, float r2) const
+    {
+        return q > Q0 * (1.0f + 1e-4f) && apart(TwoRowCol::first(sh.col[c].iw), e.size, r2);
+    }
+    __device__ __forceinline__ int list(float q) const
+    {
+        const float lo = q * (1.0f - 1e-5f), hi = q * (1.0f + 1e-5f);  // classify_pair's guard band
+        if (hi < 2.25f) return -1;
+        if (DO_S && DO_D && lo >= 82.81f && hi < Q0) return 0;
+        if (lo >= Q1 && hi < (DO_S ? 82.81f : Q0)) return 1;
+        return 2;
+    }
+    __device__ __forceinline__ void put_one(int i, int c, float sr, float si, float dr, float di) const
+    {
+        const int64_t off = (int64_t)c * a.ld + i;
+        if (DO_S) out_s[off] = make_float2(sr, si);
+        if (DO_D) out_d[off] = make_float2(dr, di);
+    }
+    using Val = Gal2Val;
+    template <int H>
+    __device__ __forceinline__ void put(const Val &v, int c, int i) const
+    {
+        float x[4], y[4];
+        f2_unpack(v.sr, x[0], y[0]);
+        f2_unpack(v.si, x[1], y[1]);
+        f2_unpack(v.dr, x[2], y[2]);
+        f2_unpack(v.di, x[3], y[3]);
+        if (H == 0) put_one(i, c, x[0], x[1], x[2], x[3]);
+        else put_one(i, c, y[0], y[1], y[2], y[3]);
+    }
+    __device__ __forceinline__ static Val zero() { return {f2_dup(0.0f), f2_dup(0.0f), f2_dup(0.0f), f2_dup(0.0f)}; }
+    __device__ __forceinline__ void far_eval(const Extra &e, int c, f2 dx, f2 dy, f2 dz, f2, Val &v) const
+    {
+        const TwoRowCol &t = sh.col[c];
+        v = zero();
+        gal2_point<FAM, DO_S, DO_D>(dx, dy, dz, t.w4 * e.area, t.nx, t.ny, t.nz, k, v);
+    }
+    template <int LIST>
+    __device__ __forceinline__ void pair(int i, int c) const
+    {
+        if constexpr (LIST == 1 || (DO_S && DO_D)) {
+            constexpr float INV4PI = 0.0795774715459476679f;
+            constexpr bool PS = LIST == 1 && DO_S;  // the SLP at the level-1 points
+            const TwoRowCol &t = sh.col[c];
+            const int j = jb + c;
+            const float3 d = t.diff(a.test, i);
+            const float4 p = t.p0();
+            Gal2Sums o;
+            if (LIST == 0) gal2_point1<FAM, true, false>(d.x, d.y, d.z, p.x * a.test.p0[i].x, p.y, p.z, p.w, k, o);
+            if (!a.test.has_quad && !a.trial.has_quad) {
+                // 3 x 3 points, one normal
+                const float4 *px = a.test.pts32 + 2 * ((int64_t)i * 2 * SLOTS + level_slot0(1));
+                const float4 *py = a.trial.pts32 + 2 * ((int64_t)j * 2 * SLOTS + level_slot0(1));
+                const float4 y0 = __ldg(py), y1 = __ldg(py + 2), y2 = __ldg(py + 4);
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    const float4 x = __ldg(px + 2 * u);
+                    const float ux = d.x - x.x, uy = d.y - x.y, uz = d.z - x.z, w = x.w * INV4PI;
+                    gal2_point1<FAM, PS, DO_D>(ux + y0.x, uy + y0.y, uz + y0.z, y0.w * w, p.y, p.z, p.w, k, o);
+                    gal2_point1<FAM, PS, DO_D>(ux + y1.x, uy + y1.y, uz + y1.z, y1.w * w, p.y, p.z, p.w, k, o);
+                    gal2_point1<FAM, PS, DO_D>(ux + y2.x, uy + y2.y, uz + y2.z, y2.w * w, p.y, p.z, p.w, k, o);
+                }
+            } else {
+                const int inc = a.test.nc[i], jnc = a.trial.nc[j], cmax = inc == 4 || jnc == 4 ? 1 : 0;
+                const float4 *px = a.test.pts32 + 2 * (((int64_t)i * 2 + cmax) * SLOTS + level_slot0(1));
+                const float4 *py = a.trial.pts32 + 2 * (((int64_t)j * 2 + cmax) * SLOTS + level_slot0(1));
+                const int npi = level_npts(inc, cmax, 1), npj = level_npts(jnc, cmax, 1);
+                for (int u = 0; u < npi; ++u) {
+                    const float4 x = __ldg(px + 2 * u);
+                    const float ux = d.x - x.x, uy = d.y - x.y, uz = d.z - x.z, w = x.w * INV4PI;
+                    for (int v = 0; v < npj; ++v) {
+                        const float4 y = __ldg(py + 2 * v), n = __ldg(py + 2 * v + 1);
+                        gal2_point1<FAM, PS, DO_D>(ux + y.x, uy + y.y, uz + y.z, y.w * w, n.x, n.y, n.z, k, o);
+                    }
+                }
+            }
+            // within reach the elements may share a node: the singular rule's pairs are listed
+            if (clear(i, j, t, d)) put_one(i, c, o.sr, o.si, o.dr, o.di);
+        }
+    }
+    // false: a pair that shares a node, which goes to the extra list
+    __device__ __forceinline__ bool clear(int i, int j, const TwoRowCol &t, float3 d) const
+    {
+        if (apart(TwoRowCol::first(t.iw), rsqrtf(a.test.chi[i].w), d.x * d.x + d.y * d.y + d.z * d.z)) return true;
+        int ind1, ind2;
+        if (common_nodes(a.test.nid[i], a.test.nc[i], a.trial.nid[j], a.trial.nc[j], ind1, ind2) == 0) return true;
+        const unsigned slot = atomicAdd(a.n_extra, 1u);
+        if (slot < (unsigned)a.extra_cap) a.extra[slot] = make_int2(i, j);
+        else atomicCAS(a.err, 0, -1);
+        return false;
+    }
+    __device__ __forceinline__ void general(int i, int c) const
+    {
+        Gal2Sums o;
+        if (gal2_general<FAM, OPS>(a, i, jb + c, o) && (threadIdx.x & (GAL2_LANES - 1)) == 0)
+            put_one(i, c, o.sr, o.si, o.dr, o.di);
+    }
+};
+
+template <int FAM, int OPS>
+__global__ void __launch_bounds__(TWO_ROW_THREADS, 20 / TWO_ROW_WARPS) k_galerkin_regular2(const __grid_constant__ GalArgs a,
+                                                                                          int cols_per_block)
+{
+    __shared__ TwoRowShared sh;
+    const int jb = a.j0 + blockIdx.y * cols_per_block;
+    const int ncols = min(cols_per_block, a.j1 - jb);
+    if (threadIdx.x < ncols) sh.stage(threadIdx.x, a.trial, jb + threadIdx.x);
+    __syncthreads();
+    const int ib = blockIdx.x * TWO_ROW_ROWS;
+    if (ib + 64 * (threadIdx.x >> 5) >= a.test.n) return;
+    const int64_t off = (int64_t)(jb - a.j0) * a.ld;
+    const Gal2Op<FAM, OPS> op{a, sh, jb, reinterpret_cast<float2 *>(a.out_s) + off,
+                              reinterpret_cast<float2 *>(a.out_d) + off, a.k32};
+    if (ib + TWO_ROW_ROWS <= a.test.n) two_row_columns<true>(op, sh, a.test, ib, ncols);
+    else two_row_columns<false>(op, sh, a.test, ib, ncols);
+}
+
+template <int FAM>
+static cudaError_t launch_galerkin_regular2(const GalArgs &a, cudaStream_t s)
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int cpb = two_row_cols(a.test.n, a.j1 - a.j0, sms);
+    const dim3 grid((a.test.n + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS, (a.j1 - a.j0 + cpb - 1) / cpb);
+    const auto kernel = a.ops == OP_SLP   ? k_galerkin_regular2<FAM, OP_SLP>
+                        : a.ops == OP_DLP ? k_galerkin_regular2<FAM, OP_DLP>
+                                          : k_galerkin_regular2<FAM, OP_SLP | OP_DLP>;
+    kernel<<<grid, TWO_ROW_THREADS, 0, s>>>(a, cpb);
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------- near pairs, FP32 triangles
+
+// sin and cos in FP32: the Taylor series to x^11 and x^12 for |x| <= pi/2
+// (truncation below 4e-8), when the caller's bound allows (warp-uniform), else
+// the library's
+__device__ __forceinline__ void sincos_short(float x, bool bounded, float &s, float &c)
+{
+    if (!bounded) {
+        sincosf(x, &s, &c);
+        return;
+    }
+    const float u = x * x;
+    float p = -1.0f / 39916800.0f, q = 1.0f / 479001600.0f;
+    p = fmaf(p, u, 1.0f / 362880.0f);
+    q = fmaf(q, u, -1.0f / 3628800.0f);
+    p = fmaf(p, u, -1.0f / 5040.0f);
+    q = fmaf(q, u, 1.0f / 40320.0f);
+    p = fmaf(p, u, 1.0f / 120.0f);
+    q = fmaf(q, u, -1.0f / 720.0f);
+    p = fmaf(p, u, -1.0f / 6.0f);
+    q = fmaf(q, u, 1.0f / 24.0f);
+    q = fmaf(q, u, -0.5f);
+    s = fmaf(p * u, x, x);
+    c = fmaf(q, u, 1.0f);
+}
+
+// k_galerkin_near for triangles under FP32 quadrature and a real wave number:
+// the same rules and points.  That kernel runs every warp through FP64 copies
+// of the pair's corners on all lanes (46% of its time the FP64 pipe, two
+// blocks per SM at 128 registers); here 21 lanes form one corner or centre
+// difference each in FP64, rounded to FP32 and shared by shuffles.
+// 5120 triangles (94 100 pairs), alone: 250 us.
+template <typename Out, int FAM>
+__global__ void __launch_bounds__(GAL_WARPS * 32) k_galerkin_near_tria(const __grid_constant__ GalArgs a, NearList near,
+                                                                       int extra)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    int64_t n_near = 0, p_begin = 0, total = 0;
+    if (extra) {
+        total = min((int64_t)*a.n_extra, (int64_t)a.extra_cap);
+    } else {
+        p_begin = near.col_ptr ? near.col_ptr[a.j0] : 0;
+        n_near = (near.col_ptr ? near.col_ptr[a.j1] : 0) - p_begin;
+        total = n_near + (a.same_mesh ? (int64_t)(a.j1 - a.j0) : 0);
+    }
+    const bool do_s = (a.ops & OP_SLP) != 0, do_d = (a.ops & OP_DLP) != 0;
+    Out *out_s = reinterpret_cast<Out *>(a.out_s);
+    Out *out_d = reinterpret_cast<Out *>(a.out_d);
+    const float kf = a.k32;
+    for (int64_t item = warp; item < total; item += nwarps) {
+        int i, j;
+        if (extra) {
+            const int2 e = a.extra[item];
+            i = e.x;
+            j = e.y;
+        } else if (item < n_near) {
+            const int64_t p = p_begin + item;
+            i = near.rows[p];
+            j = near_column(near.col_ptr, a.j0, a.j1, p);
+        } else {
+            j = a.j0 + (int)(item - n_near);
+            i = j;
+            if (i >= a.test.n) continue;
+        }
+        int match = -1, ind1 = 0, ind2 = 0;
+        if (a.same_mesh) {
+            if (i == j) {
+                match = 2;
+            } else {
+                const int num = common_nodes(a.test.nid[i], 3, a.trial.nid[j], 3, ind1, ind2);
+                match = num > 1 ? 1 : (num == 1 ? 0 : -1);
+            }
+        }
+        // lane 3 q + d (9 + 3 q + d): coordinate d of corner q of the test (trial)
+        // element, relative to test corner 0 (matched), or of its sides and of
+        // corner 0 relative to its centre (unmatched); 18 + d: the centres' difference
+        float mine = 0.0f;
+        if (lane < 21) {
+            const int d = lane % 3, q = (lane / 3) % 3;
+            const bool on_trial = lane >= 9;
+            const double *ci = a.test.corners + 12 * (int64_t)i, *cj = a.trial.corners + 12 * (int64_t)j;
+            const double *xi = a.test.center + 3 * (int64_t)i, *xj = a.trial.center + 3 * (int64_t)j;
+            double from, to;
+            if (lane >= 18) {
+                to = xj[d];
+                from = xi[d];
+            } else {
+                to = (on_trial ? cj : ci)[3 * q + d];
+                from = match >= 0 ? ci[d] : (q == 0 ? (on_trial ? xj : xi)[d] : (on_trial ? cj : ci)[d]);
+            }
+            mine = (float)(to - from);
+        }
+        float tc[3][3], rc[3][3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                tc[q][d] = __shfl_sync(0xffffffffu, mine, 3 * q + d);
+                rc[q][d] = __shfl_sync(0xffffffffu, mine, 9 + 3 * q + d);
+            }
+        // sides of both elements (in their own orientation), normals
+        float e1[3], e2[3], f1[3], f2v[3], ntv[3], nrv[3], nrm[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            e1[d] = match >= 0 ? tc[1][d] - tc[0][d] : tc[1][d];
+            e2[d] = match >= 0 ? tc[2][d] - tc[0][d] : tc[2][d];
+            f1[d] = match >= 0 ? rc[1][d] - rc[0][d] : rc[1][d];
+            f2v[d] = match >= 0 ? rc[2][d] - rc[0][d] : rc[2][d];
+        }
+        ntv[0] = e1[1] * e2[2] - e1[2] * e2[1];
+        ntv[1] = e1[2] * e2[0] - e1[0] * e2[2];
+        ntv[2] = e1[0] * e2[1] - e1[1] * e2[0];
+        nrv[0] = f1[1] * f2v[2] - f1[2] * f2v[1];
+        nrv[1] = f1[2] * f2v[0] - f1[0] * f2v[2];
+        nrv[2] = f1[0] * f2v[1] - f1[1] * f2v[0];
+        const float Jt = sqrtf(ntv[0] * ntv[0] + ntv[1] * ntv[1] + ntv[2] * ntv[2]);
+        const float Jr = sqrtf(nrv[0] * nrv[0] + nrv[1] * nrv[1] + nrv[2] * nrv[2]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) nrm[d] = nrv[d] / Jr;
+        const float wscale = Jt * Jr * (float)(1.0 / FOUR_PI);
+        // a corner is at most D from its centre (the longest side is below 1.5 D), a
+        // listed pair's centres at most 1.5 D_j apart: r <= D_i + 2.5 D_j
+        const float r_max = rsqrtf(a.test.chi[i].w) + 2.5f * rsqrtf(a.trial.chi[j].w);
+        const bool bounded = !extra && fabsf(kf) * r_max <= 1.57f;
+        float fsr = 0, fsi = 0, fdr = 0, fdi = 0;
+        auto point = [&](const float rv[3], float w, bool use_s, bool use_d) {
+            const float r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
+            const float rinv = rsqrtf(r2);
+            const float g = w * wscale * rinv;  // w Jt Jr / (4 pi r)
+            float sn = 0.0f, cs = 1.0f, kr = 0.0f;
+            if constexpr (FAM == FAM_HELMHOLTZ) {
+                kr = kf * (r2 * rinv);
+                sincos_short(kr, bounded, sn, cs);
+            }
+            if (use_s) {
+                fsr += g * cs;
+                fsi -= g * sn;
+            }
+            if (use_d) {
+                const float f = -g * rinv * (rv[0] * nrm[0] + rv[1] * nrm[1] + rv[2] * nrm[2]) * rinv;
+                fdr += f * (cs + kr * sn);
+                fdi += f * (kr * cs - sn);
+            }
+        };
+        if (match >= 0) {
+            // both rotated triangles start at the common node: r_vec from their
+            // sides there and the rule's FP64-formed coordinate differences
+            int pt[3], pr[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                pt[q] = match == 2 ? q : (ind1 + q) % 3;
+                pr[q] = match == 2 ? q : (match == 1 ? (ind2 + 1 + 3 - q) % 3 : (ind2 + q) % 3);
+            }
+            auto pick = [](const float (&c)[3][3], int idx, int d) {
+                return idx == 0 ? c[0][d] : (idx == 1 ? c[1][d] : c[2][d]);
+            };
+            float at[3], bt[3], ar[3], br[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                at[d] = pick(tc, pt[1], d) - pick(tc, pt[0], d);
+                bt[d] = pick(tc, pt[2], d) - pick(tc, pt[0], d);
+                ar[d] = pick(rc, pr[1], d) - pick(rc, pr[0], d);
+                br[d] = pick(rc, pr[2], d) - pick(rc, pr[0], d);
+            }
+            const float4 *rule = reinterpret_cast<const float4 *>(g_gal_rule32) + 2 * (size_t)gal_offset(match);
+            const int np = gal_npts(match);
+            // q0 = (xi1, xi2, eta1, eta2), q1 = (w, eta1 - xi1, eta2 - xi2, 0)
+            auto sum = [&](auto form) {
+#pragma unroll 2
+                for (int p = lane; p < np; p += 32) {
+                    const float4 q0 = __ldg(rule + 2 * p), q1 = __ldg(rule + 2 * p + 1);
+                    float rv[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) rv[d] = form(q0, q1, d);
+                    point(rv, q1.x, do_s, do_d);
+                }
+            };
+            if (match == 2) sum([&](float4, float4 q1, int d) { return q1.y * at[d] + q1.z * bt[d]; });
+            else if (match == 1)
+                sum([&](float4 q0, float4 q1, int d) { return q1.y * at[d] + q0.w * br[d] - q0.y * bt[d]; });
+            else
+                sum([&](float4 q0, float4, int d) {
+                    return q0.z * ar[d] + q0.w * br[d] - q0.x * at[d] - q0.y * bt[d];
+                });
+        } else {
+            // the product rules of the degrees of d/D, decided in FP32 with the
+            // FP64 guard band of the classification
+            float c0[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) c0[d] = __shfl_sync(0xffffffffu, mine, 18 + d);
+            const float ratio = sqrtf(c0[0] * c0[0] + c0[1] * c0[1] + c0[2] * c0[2]) / (float)a.trial.size[j];
+            double rx = (double)ratio;
+            if (fabsf(ratio - 1.1f) < 1e-4f || fabsf(ratio - 1.5f) < 1e-4f || fabsf(ratio - 1.8f) < 1e-4f) {
+                double dcd[3];
+                for (int d = 0; d < 3; ++d)
+                    dcd[d] = a.trial.center[3 * (int64_t)j + d] - a.test.center[3 * (int64_t)i + d];
+                rx = norm3(dcd) / a.trial.size[j];
+            }
+            const int deg_s = rx < 11.0 / 10.0 ? 6 : (rx < T_S1 ? 4 : (rx < T_S0 ? 2 : 0));
+            const int deg_d = rx < 11.0 / 10.0 ? 8 : (rx < T_NEAR ? 6 : (rx < T_D1 ? 4 : (rx < T_D0 ? 2 : 0)));
+            const bool one_pass = !do_s || !do_d || deg_s == deg_d;
+            for (int pass = 0; pass < (one_pass ? 1 : 2); ++pass) {
+                const bool use_s = one_pass ? do_s : pass == 0;
+                const bool use_d = one_pass ? do_d : pass == 1;
+                const int deg = use_s ? deg_s : deg_d;
+                const int npt = g_tri_npts[deg];
+                const float *rule = TRI_F32.v + 3 * g_tri_off[deg];
+                for (int p = lane; p < npt * npt; p += 32) {
+                    const float *qa = rule + 3 * (p / npt), *qb = rule + 3 * (p % npt);
+                    const float fxa = qa[0], fea = qa[1], wa = qa[2], fxb = qb[0], feb = qb[1], wb = qb[2];
+                    float rv[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        rv[d] = c0[d] + (rc[0][d] + fxb * f1[d] + feb * f2v[d]) - (tc[0][d] + fxa * e1[d] + fea * e2[d]);
+                    point(rv, wa * wb, use_s, use_d);
+                }
+            }
+        }
+        // the four sums over the lanes in FP64, two, then one value per lane: after
+        // two exchanges lanes 0-7 hold sr, 8-15 si, 16-23 dr, 24-31 di
+        const bool up = lane & 16, odd = lane & 8;
+        double va = (double)(up ? fdr : fsr), vb = (double)(up ? fdi : fsi);
+        va += (double)__shfl_xor_sync(0xffffffffu, up ? fsr : fdr, 16);
+        vb += (double)__shfl_xor_sync(0xffffffffu, up ? fsi : fdi, 16);
+        double v = odd ? vb : va;
+        v += __shfl_xor_sync(0xffffffffu, odd ? va : vb, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const double im = __shfl_down_sync(0xffffffffu, v, 8);
+        if (lane == 0 || lane == 16) {
+            const bool slp = lane == 0;
+            if (slp ? do_s : do_d)
+                store64((slp ? out_s : out_d) + (int64_t)(j - a.j0) * a.ld + i, v, im, a.alpha_re, a.alpha_im,
+                        a.accumulate);
+        }
+    }
+}
+
+template <typename Out>
+static cudaError_t launch_galerkin_near_tria(const GalArgs &a, const NearList &near, int extra, int64_t max_items, int sms,
+                                             cudaStream_t s)
+{
+    const auto kernel = a.family == FAM_HELMHOLTZ ? k_galerkin_near_tria<Out, FAM_HELMHOLTZ>
+                                                  : k_galerkin_near_tria<Out, FAM_LAPLACE>;
+    const int64_t want = (max_items + GAL_WARPS - 1) / GAL_WARPS;
+    // as many blocks as an SM holds at 72 registers: the regular kernel, launched
+    // beside this one, follows into the SMs as they drain (5120 triangles, both
+    // together: 4, 6, 7 blocks per SM 952, 900, 888 us; one after the other 950)
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, 7 * (int64_t)sms));
+    kernel<<<blocks, GAL_WARPS * 32, 0, s>>>(a, near, extra);
+    return cudaGetLastError();
+}
+
 // point p of the product rule of a given degree on an element: reference
 // coordinates and weight (Dunavant on triangles, Gauss tensor on quads)
 __device__ __forceinline__ void product_point(int nc, int degree, int p, double &xi, double &eta, double &w)
@@ -909,7 +1454,7 @@ static void launch_gal_ops(const GalArgs &a, dim3 grid, cudaStream_t s)
             return;
         }
     }
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (sizeof(R) == 4 && sizeof(Out) == 16) {  // into complex64: k_galerkin_regular2
         if (a.alpha_re == 1.0 && a.alpha_im == 0.0 && !a.accumulate) {
             if (a.ops == OP_SLP) k_galerkin_regular<R, Out, FAM, OP_SLP, true><<<grid, GAL_THREADS, 0, s>>>(a);
             else if (a.ops == OP_DLP) k_galerkin_regular<R, Out, FAM, OP_DLP, true><<<grid, GAL_THREADS, 0, s>>>(a);
@@ -933,6 +1478,9 @@ cudaError_t launch_galerkin_regular(const GalArgs &a, cudaStream_t s)
 {
     const int ncols = a.j1 - a.j0;
     if (a.test.n == 0 || ncols <= 0) return cudaSuccess;
+    if (a.precision == 0 && a.dtype == 0 && a.k_im == 0.0 && a.alpha_re == 1.0 && a.alpha_im == 0.0 && !a.accumulate)
+        return a.family == FAM_HELMHOLTZ ? launch_galerkin_regular2<FAM_HELMHOLTZ>(a, s)
+                                         : launch_galerkin_regular2<FAM_LAPLACE>(a, s);
     dim3 grid((a.test.n + GAL_THREADS - 1) / GAL_THREADS, (ncols + GAL_COLS - 1) / GAL_COLS);
     if (a.precision == 0) {
         if (a.dtype == 0) launch_gal_fam<float, float2>(a, grid, s);
@@ -950,6 +1498,9 @@ cudaError_t launch_galerkin_near(const GalArgs &a, const NearList &near, int ext
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (a.precision == 0 && a.k_im == 0.0 && !a.test.has_quad && !a.trial.has_quad)
+        return a.dtype == 0 ? launch_galerkin_near_tria<float2>(a, near, extra, max_items, sms, s)
+                            : launch_galerkin_near_tria<double2>(a, near, extra, max_items, sms, s);
     // two 4-warp blocks per SM: the kernel runs beside the regular one and
     // must leave it most of the register file
     const int64_t want = (max_items + GAL_WARPS - 1) / GAL_WARPS;

@@ -610,6 +610,7 @@ __device__ __noinline__ bool reg2_general(const RegularArgs &a, int i, int j, fl
 // PLAIN: unit scale and no accumulation, so the stores carry no run-time checks
 template <int FAM, int OPS, bool CK, bool PLAIN>
 struct Reg2Op {
+    static constexpr int GENERAL_LANES = 1;
     static constexpr bool DO_S = (OPS & OP_SLP) != 0, DO_D = (OPS & OP_DLP) != 0;
     // (d/D)^2 of the one-point rule of every operator, and of the next limit
     // below which list 1 ends (both: the DLP's 2.8, above the SLP's 1.8)
@@ -623,7 +624,7 @@ struct Reg2Op {
 
     struct Extra {};
     __device__ __forceinline__ Extra extra(int, int) const { return {}; }
-    __device__ __forceinline__ bool far(float q) const { return q > Q0 * (1.0f + 1e-4f); }
+    __device__ __forceinline__ bool far(const Extra &, int, float q, float) const { return q > Q0 * (1.0f + 1e-4f); }
     __device__ __forceinline__ int list(float q) const
     {
         // the FP32 guard band of classify_pair: outside it the class is the FP64 class

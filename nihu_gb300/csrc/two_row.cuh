@@ -15,12 +15,12 @@
 //
 // K, the operator, provides
 //   struct Extra                    what it keeps of the thread's two rows; Extra extra(int i0, int i1)
-//   bool far(float q)               q = (d/D)^2 of a pair: certainly the one-point rule
+//   bool far(Extra, c, q, r2)       q = (d/D)^2 of a pair, r2 = d^2: certainly the one-point rule
 //   int list(float q)               of a pair that is not: 0, 1, 2, or -1 (left to the singular kernel)
 //   void far_eval(Extra, c, dx, dy, dz, r2, Val &)  both rows' far values in column c of the block
 //   void put<H>(Val, c, i)          stores half H (0, 1) at row i
 //   void pair<LIST>(i, c)           evaluates and stores a pair of list 0 or 1
-//   void general(i, c)              evaluates and stores a pair of list 2
+//   void general(i, c)              evaluates and stores a pair of list 2, called by GENERAL_LANES lanes
 #pragma once
 
 #include <cuda_runtime.h>
@@ -130,7 +130,9 @@ __device__ __forceinline__ void two_row_columns(const K &op, TwoRowShared &sh, c
             const f2 r2 = f2_fma(dz, dz, f2_fma(dx, dx, dy * dy));
             float qa, qb;
             f2_unpack(r2 * t.iw, qa, qb);
-            const bool fa = op.far(qa), fb = op.far(qb);
+            float ra, rb;
+            f2_unpack(r2, ra, rb);
+            const bool fa = op.far(ex, c, qa, ra), fb = op.far(ex, c, qb, rb);
             const bool all = __all_sync(0xffffffffu, fa && fb);
             if (all || __any_sync(0xffffffffu, fa || fb)) {
                 typename K::Val v;
@@ -162,7 +164,12 @@ __device__ __forceinline__ void two_row_columns(const K &op, TwoRowShared &sh, c
             __syncwarp();  // the entries are visible to the whole warp
             for (int t = lane; t < nA; t += 32) op.template pair<0>(wb + (la[t] & 63), la[t] >> 6);
             for (int t = lane; t < nB; t += 32) op.template pair<1>(wb + (lb[t] & 63), lb[t] >> 6);
-            for (int t = lane; t < nC; t += 32) op.general(wb + (la[TWO_ROW_LIST - 1 - t] & 63), la[TWO_ROW_LIST - 1 - t] >> 6);
+            // G lanes per entry of list 2
+            constexpr int G = K::GENERAL_LANES;
+            for (int t0 = 0; t0 < nC; t0 += 32 / G) {
+                const int t = t0 + lane / G;
+                if (t < nC) op.general(wb + (la[TWO_ROW_LIST - 1 - t] & 63), la[TWO_ROW_LIST - 1 - t] >> 6);
+            }
             __syncwarp();  // read before the next chunk appends
         }
     }
