@@ -55,7 +55,7 @@ struct nihu_gb_ctx {
     cudaGraphExec_t lu_exec = nullptr;
     int lu_n = 0;
     int64_t lu_launches = 0;
-    void *lu_F = nullptr, *lu_piv = nullptr;
+    void *lu_F = nullptr, *lu_aux = nullptr;
 };
 
 struct nihu_gb_mesh {
@@ -1429,7 +1429,7 @@ namespace {
 // x_0 = 0, then d = (LU)^{-1} r, x += d, r = b - A x (FP64 matvec) until the
 // correction is within 64 FP64 roundings of x (|d| <= 64 eps |x|, the
 // accuracy of an FP64 factorisation).  *refined = false (and nothing solved)
-// when the order is beyond the FP32 kernels' shared memory or the
+// when the order is beyond the FP32 kernels' shared memory and registers or the
 // corrections stop shrinking (cond(A) near 1 / eps32): the caller then
 // factorises in FP64.  A is left unchanged.
 nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int64_t lda, const double2 *b, double2 *x,
@@ -1440,26 +1440,24 @@ nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
     if (!lu32_fits((int)n, (size_t)smem_optin)) return NIHU_GB_OK;
     nihu_gb_status st;
-    void *pf, *ppiv, *pd, *pr, *psums, *ppart;
+    void *pf, *paux, *pd, *pr, *psums, *ppart;
     const int splits = gemv_splits(n, n, NIHU_GB_C128);
     if ((st = scratch(ctx, "lu32_F", 8 * (size_t)n * n, &pf))) return st;
-    if ((st = scratch(ctx, "lu_piv", sizeof(int) * n, &ppiv))) return st;
+    if ((st = scratch(ctx, "lu32_aux", lu32_aux_bytes((int)n), &paux))) return st;
     if ((st = scratch(ctx, "lu32_d", 16 * (size_t)n, &pd))) return st;
     if ((st = scratch(ctx, "lu32_r", 16 * (size_t)n, &pr))) return st;
     if ((st = scratch(ctx, "lu32_sums", 2 * sizeof(double), &psums))) return st;
     if ((st = scratch(ctx, "lu32_part", 16 * (size_t)splits * n, &ppart))) return st;
     double2 *d = (double2 *)pd, *r = (double2 *)pr;
-    size_t panel_smem = 0;
-    CK(lu32_prepare((int)n, (size_t)smem_optin, &panel_smem));
-    if (!(ctx->lu_exec && ctx->lu_n == n && ctx->lu_F == pf && ctx->lu_piv == ppiv)) {
+    CK(lu32_prepare((int)n, (size_t)smem_optin));
+    if (!(ctx->lu_exec && ctx->lu_n == n && ctx->lu_F == pf && ctx->lu_aux == paux)) {
         // record the panel sequence once per order and buffers
         if (ctx->lu_exec) cudaGraphExecDestroy(ctx->lu_exec);
         ctx->lu_exec = nullptr;
         cudaGraph_t graph = nullptr;
         int64_t counted = 0;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = launch_lu32_factor((float2 *)pf, (int)n, (int *)ppiv, ctx->d_flag + 1, panel_smem, &counted,
-                                           ctx->stream);
+        cudaError_t e = launch_lu32_factor((float2 *)pf, (int)n, paux, ctx->d_flag + 1, &counted, ctx->stream);
         cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
         if (e == cudaSuccess) e = e2;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&ctx->lu_exec, graph, 0);
@@ -1470,13 +1468,13 @@ nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int
         }
         ctx->lu_n = (int)n;
         ctx->lu_F = pf;
-        ctx->lu_piv = ppiv;
+        ctx->lu_aux = paux;
         ctx->lu_launches = counted;
     }
     CK(cudaMemsetAsync(ctx->d_flag + 1, 0, sizeof(int), ctx->stream));
     {
         Phase ph(ctx, "lu_factor");
-        CK(launch_to_c64(A, lda, (int)n, (float2 *)pf, ctx->stream));
+        CK(launch_to_c64(A, lda, (int)n, (float2 *)pf, paux, ctx->stream));
         CK(cudaGraphLaunch(ctx->lu_exec, ctx->stream));
         ctx->launches += 1 + ctx->lu_launches;
     }
@@ -1490,7 +1488,7 @@ nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int
     double sums[2] = {0.0, 0.0}, prev = 0.0;
     const double eps = 2.220446049250313e-16;
     for (int it = 0; it < 12; ++it) {
-        CK(launch_lu32_solve((const float2 *)pf, (int)n, (const int *)ppiv, r, d, ctx->stream));
+        CK(launch_lu32_solve((const float2 *)pf, (int)n, paux, r, d, ctx->stream));
         CK(launch_lu32_update_x(x, d, (int)n, (double *)psums, ctx->stream));
         CK(cudaMemcpyAsync(r, b, 16 * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
         CK(launch_gemv(NIHU_GB_C128, A, n, n, lda, x, r, -1.0, 0.0, 1.0, 0.0, (double2 *)ppart, splits, ctx->stream));
