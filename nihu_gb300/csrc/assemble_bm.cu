@@ -109,8 +109,9 @@ __global__ void __launch_bounds__(BM_THREADS, sizeof(R) == 4 ? 4 : 1) k_regular_
     const DevMesh &test = a.test;
     const DevMesh &trial = a.trial;
     const int i = blockIdx.x * BM_THREADS + threadIdx.x;
-    const int jb = a.j0 + blockIdx.y * BM_COLS;
-    const int ncols = min(BM_COLS, a.j1 - jb);
+    const int cpb = (a.j1 - a.j0 + gridDim.y - 1) / gridDim.y;
+    const int jb = a.j0 + blockIdx.y * cpb;
+    const int ncols = min(cpb, a.j1 - jb);
     if (threadIdx.x < ncols) {
         s_hi[threadIdx.x] = trial.chi[jb + threadIdx.x];
         s_lo[threadIdx.x] = trial.clo[jb + threadIdx.x];
@@ -556,7 +557,8 @@ cudaError_t launch_assemble_regular_bm(const BmArgs &a, cudaStream_t s)
     const bool all4 = a.ops == (OP_SLP | OP_DLP | OP_DLPT | OP_HSP);
     if (all4 && a.precision == 0 && a.dtype == 0 && a.k_im == 0.0)
         return a.family == FAM_HELMHOLTZ ? launch_bm2<FAM_HELMHOLTZ>(a, s) : launch_bm2<FAM_LAPLACE>(a, s);
-    dim3 grid((a.test.n + BM_THREADS - 1) / BM_THREADS, (ncols + BM_COLS - 1) / BM_COLS);
+    dim3 grid((a.test.n + BM_THREADS - 1) / BM_THREADS);
+    grid.y = column_blocks(grid.x, ncols, BM_COLS);
     if (a.precision == 0) {
         if (a.dtype == 0) launch_bm_fam<float, float2>(a, grid, s);
         else launch_bm_fam<float, double2>(a, grid, s);

@@ -319,8 +319,9 @@ __global__ void __launch_bounds__(GAL_THREADS) k_galerkin_regular(GalArgs a)
     const DevMesh &test = a.test;
     const DevMesh &trial = a.trial;
     const int i = blockIdx.x * GAL_THREADS + threadIdx.x;
-    const int jb = a.j0 + blockIdx.y * GAL_COLS;
-    const int ncols = min(GAL_COLS, a.j1 - jb);
+    const int cpb = (a.j1 - a.j0 + gridDim.y - 1) / gridDim.y;
+    const int jb = a.j0 + blockIdx.y * cpb;
+    const int ncols = min(cpb, a.j1 - jb);
     if (threadIdx.x < ncols) {
         const int j = jb + threadIdx.x;
         s_hi[threadIdx.x] = trial.chi[j];
@@ -1481,7 +1482,8 @@ cudaError_t launch_galerkin_regular(const GalArgs &a, cudaStream_t s)
     if (a.precision == 0 && a.dtype == 0 && a.k_im == 0.0 && a.alpha_re == 1.0 && a.alpha_im == 0.0 && !a.accumulate)
         return a.family == FAM_HELMHOLTZ ? launch_galerkin_regular2<FAM_HELMHOLTZ>(a, s)
                                          : launch_galerkin_regular2<FAM_LAPLACE>(a, s);
-    dim3 grid((a.test.n + GAL_THREADS - 1) / GAL_THREADS, (ncols + GAL_COLS - 1) / GAL_COLS);
+    dim3 grid((a.test.n + GAL_THREADS - 1) / GAL_THREADS);
+    grid.y = column_blocks(grid.x, ncols, GAL_COLS);
     if (a.precision == 0) {
         if (a.dtype == 0) launch_gal_fam<float, float2>(a, grid, s);
         else launch_gal_fam<float, double2>(a, grid, s);

@@ -190,8 +190,10 @@ __global__ void __launch_bounds__(REG_THREADS) k_regular(RegularArgs a)
     const DevMesh &test = a.test;
     const DevMesh &trial = a.trial;
     const int i = blockIdx.x * REG_THREADS + threadIdx.x;
-    const int jb = a.j0 + blockIdx.y * REG_COLS;
-    const int ncols = min(REG_COLS, a.j1 - jb);
+    // the launch's split of the columns; frequency batches: whole column blocks (rhs_part)
+    const int cpb = BATCH ? REG_COLS : (int)((a.j1 - a.j0 + gridDim.y - 1) / gridDim.y);
+    const int jb = a.j0 + blockIdx.y * cpb;
+    const int ncols = min(cpb, a.j1 - jb);
     // frequency batch: this block's wave numbers [f_lo, f_hi) (gridDim.z chunks)
     const int f_per = (a.nk + gridDim.z - 1) / gridDim.z;
     const int f_lo = min(a.nk, (int)blockIdx.z * f_per), f_hi = min(a.nk, f_lo + f_per);
@@ -866,6 +868,8 @@ cudaError_t launch_assemble_regular(const RegularArgs &a, cudaStream_t s)
             const int fmax = a.precision == 0 ? rhs_fmax_of<float>(a) : rhs_fmax_of<double>(a);
             grid.z = std::max<unsigned>(grid.z, (unsigned)((a.nk + fmax - 1) / fmax));
         }
+    } else {
+        grid.y = column_blocks(grid.x, ncols, REG_COLS);
     }
     if (a.precision == 0) {
         if (a.dtype == 0) launch_fam<float, float2>(a, grid, s);
