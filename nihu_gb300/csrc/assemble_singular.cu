@@ -445,7 +445,8 @@ __device__ __forceinline__ void singular_pairs(const RegularArgs &a, const NearL
                             // FP32 regular quadrature: the schemes' sums in FP32 as well
                             near_polar_sum_f32(e, fam, kf, x0, r5[0], r5[1], do_s, polar_d, acc);
                             if (fam == FAM_HELMHOLTZ) near_dynamic_quad_f32(lin, kf, x0, do_s, polar_d, acc);
-                            near_static(lin, nullptr, x0, do_s, polar_d, acc);
+                            if constexpr (sizeof(Out) == 8) near_static_quad_ff(lin, x0, do_s, polar_d, acc);
+                            else near_static(lin, nullptr, x0, do_s, polar_d, acc);
                         } else {
                             near_polar_sum(e, lin, fam, kf, x0, r5[0], r5[1], do_s, polar_d, acc);
                             near_plane(lin, nullptr, fam, kf, x0, do_s, polar_d, acc);

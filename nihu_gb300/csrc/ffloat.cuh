@@ -276,6 +276,7 @@ struct Tri14FF {
 static __device__ const Tri14FF TRI14_FF{};
 
 static __device__ const GaussHalfFF<6> GAUSS6_FF{};
+static __device__ const GaussHalfFF<8> GAUSS8_FF{};
 static __device__ const GaussHalfFF<21> GAUSS21_FF{};
 
 }  // namespace nihu

@@ -473,8 +473,8 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
         ex(e, res[0], res[1], y);
         edx(e, res[0], res[1], dxi, deta);
         cross3(dxi, deta, n);
-        double sq = sqrt(norm3(n));
-        for (int d = 0; d < 3; ++d) n[d] /= sq;
+        const double isq = rsqrt(norm3(n));  // one reciprocal a step for what is divided by it
+        for (int d = 0; d < 3; ++d) n[d] *= isq;
         double f[3];
         for (int d = 0; d < 3; ++d) f[d] = y[d] + n[d] * res[2] - x0[d];
         double err = norm3(f);
@@ -487,12 +487,12 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
             for (int d = 0; d < 3; ++d) r6[d] = res[d];
             return got5;
         }
-        // d n / d xi = (x_xixi x x_eta + x_xi x x_xieta) / sq, x_xixi = x_etaeta = 0
+        // d n / d xi = (x_xixi x x_eta + x_xi x x_xieta) / sqrt|n|, x_xixi = x_etaeta = 0
         double t2[3], dnxi[3], dneta[3];
         cross3(dxi, dxe, t2);
-        for (int d = 0; d < 3; ++d) dnxi[d] = t2[d] / sq;
+        for (int d = 0; d < 3; ++d) dnxi[d] = t2[d] * isq;
         cross3(dxe, deta, t2);
-        for (int d = 0; d < 3; ++d) dneta[d] = t2[d] / sq;
+        for (int d = 0; d < 3; ++d) dneta[d] = t2[d] * isq;
         double M[3][4];
         for (int d = 0; d < 3; ++d) {
             M[d][0] = dxi[d] + dnxi[d] * res[2];
@@ -500,14 +500,16 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
             M[d][2] = n[d];
             M[d][3] = f[d];
         }
+        double ip[3];  // 1 / pivot
         for (int c = 0; c < 3; ++c) {
             int p = c;
             for (int r = c + 1; r < 3; ++r)
                 if (fabs(M[r][c]) > fabs(M[p][c])) p = r;
             if (p != c)
                 for (int q = 0; q < 4; ++q) { double t = M[c][q]; M[c][q] = M[p][q]; M[p][q] = t; }
+            ip[c] = 1.0 / M[c][c];
             for (int r = c + 1; r < 3; ++r) {
-                double fct = M[r][c] / M[c][c];
+                double fct = M[r][c] * ip[c];
                 for (int q = c; q < 4; ++q) M[r][q] -= fct * M[c][q];
             }
         }
@@ -515,7 +517,7 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
         for (int r = 2; r >= 0; --r) {
             double v = M[r][3];
             for (int q = r + 1; q < 3; ++q) v -= M[r][q] * s[q];
-            s[r] = v / M[r][r];
+            s[r] = v * ip[r];
         }
         for (int d = 0; d < 3; ++d) res[d] -= s[d];
     }
@@ -705,50 +707,64 @@ __device__ __forceinline__ void kern32(int fam, float k, const float rv[3], cons
     }
 }
 
-// near_polar_sum with the FP32 sums (quads)
+// near_polar_sum with the FP32 sums (quads).  The parameter domain is the
+// square [-1, 1]^2, so a side's foot point and direction are exact, and with the
+// angle psi measured from the foot (tan psi the position along the side over
+// its distance s) a point at the side is rho = s / cos psi away in the
+// direction f cos psi + l sin psi (f to the foot, l along the side).  psi and its
+// sines in float-float, one pair of them for two points of the symmetric rule:
+// FP64 angles, sines and quotients per point, and the FP64 rule's conversions,
+// were a third of the singular kernel's time on quads (with the static part in
+// float-float and fewer divisions in the inverse mapping, closed cylinder of
+// 9 792 quads, SLP and DLP: 1997 -> 1200 us; entries' error unchanged).
 static __device__ __noinline__ void near_polar_sum_f32(const Elem64 &e, int fam, double k, const double x0[3], double xi0,
                                           double eta0, bool do_s, bool do_d, Acc &a)
 {
-    const int N = e.nc;
-    double tl[4], t0[4], dr[4];
-    for (int n = 0; n < N; ++n) {
-        double c1[2], c2[2];
-        domain_corner(N, n, c1[0], c1[1]);
-        domain_corner(N, (n + 1) % N, c2[0], c2[1]);
-        c1[0] -= xi0; c1[1] -= eta0;
-        c2[0] -= xi0; c2[1] -= eta0;
-        side_geometry(c1, c2, tl[n], t0[n], dr[n], true);
-    }
     QuadAround32 q;
     quad_around32(e, x0, xi0, eta0, q);
     const float kf = (float)k;
+    const ff xm = ff_from(-1.0 - xi0), xp = ff_from(1.0 - xi0), em = ff_from(-1.0 - eta0), ep = ff_from(1.0 - eta0);
     float sr = 0, si = 0, dsr = 0, dsi = 0;
-    for (int n = 0; n < N; ++n) {
-        double t1 = tl[n], t2 = tl[(n + 1) % N];
-        wrap_limits(t1, t2);
-        if (fabs(t2 - t1) < 1e-3) continue;
+#pragma unroll 1
+    for (int n = 0; n < 4; ++n) {
+        // along the side (corners n and n + 1 counter-clockwise) and across it
+        const bool back = n >= 2, vertical = n & 1;
+        const ff lo = vertical ? em : xm, hi = vertical ? ep : xp;
+        const ff u1 = back ? ff_neg(hi) : lo, u2 = back ? ff_neg(lo) : hi;
+        const ff across = n == 0 ? em : (n == 1 ? xp : (n == 2 ? ep : xm));  // signed, outwards + at 1 and 2
+        const bool plus = n == 1 || n == 2;
+        const bool inside = plus ? across.h >= 0.0f : across.h <= 0.0f;
+        ff s = across.h < 0.0f ? ff_neg(across) : across;
+        s.h = fmaxf(s.h, 1e-14f);
+        const ff q1 = ff_angle(u1, s), q2 = ff_angle(u2, s);
+        const ff mid = ff_scale(ff_add(q1, q2), 0.5f), hw = ff_scale(ff_sub(q2, q1), 0.5f);
+        if (2.0f * hw.h < 1e-3f) continue;
+        const float cmin = s.h * rsqrtf(fmaxf(u1.h * u1.h, u2.h * u2.h) + s.h * s.h);
+        ff sm, cm;
+        ff_sincos(mid, sm, cm);
+        const float l = back ? -1.0f : 1.0f, f = across.h < 0.0f ? -1.0f : 1.0f;  // along u (v), towards the side
+#pragma unroll 1
         for (int ia = 0; ia < 8; ++ia) {
-            double xx, wa;
-            gauss_pt(8, ia, xx, wa);
-            const double th = ((1.0 - xx) * t1 + (1.0 + xx) * t2) / 2.0;
-            double cth, sth;
-            sincos(th, &sth, &cth);
-            const float wth = (float)(wa * (t2 - t1) / 2.0);
-            const float rho_lim = (float)(dr[n] / cos_angle(th - t0[n]));
-            const float cf = (float)cth, sf = (float)sth;
+            ff sh, ch;
+            ff_sincos(ff_mul(hw, ff{GAUSS8_FF.xh[ia & 3], GAUSS8_FF.xl[ia & 3]}), sh, ch);
+            if (ia & 4) sh = ff_neg(sh);
+            const float c = fmaxf(ff_sub(ff_mul(cm, ch), ff_mul(sm, sh)).h, cmin);
+            const float sn = ff_add(ff_mul(sm, ch), ff_mul(cm, sh)).h;
+            const float wth = GAUSS8_FF.wh[ia & 3] * (inside ? hw.h : -hw.h);
+            const float rho_lim = s.h / c;
+            const float cf = vertical ? f * c : l * sn, sf = vertical ? l * sn : f * c;
             float ps = 0, pi = 0, pds = 0, pdi = 0;
             for (int ib = 0; ib < 8; ++ib) {
-                double xr, wb;
-                gauss_pt(8, ib, xr, wb);
-                const float rho = (1.0f + (float)xr) * rho_lim * 0.5f;
-                const float wt = (float)wb * rho_lim * 0.5f * rho;
+                const float xr = ib & 4 ? -GAUSS8_FF.xh[ib & 3] : GAUSS8_FF.xh[ib & 3];
+                const float rho = (1.0f + xr) * rho_lim * 0.5f;
+                const float wt = GAUSS8_FF.wh[ib & 3] * rho_lim * 0.5f * rho;
                 const float u = rho * cf, v = rho * sf, uv = u * v;
                 float rl[3], re[3], ne[3];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    rl[c] = q.p[c] + u * q.t1[c] + v * q.t2[c];
-                    re[c] = rl[c] + uv * q.d[c];
-                    ne[c] = q.n0[c] + u * q.nu[c] + v * q.nv[c];
+                for (int d = 0; d < 3; ++d) {
+                    rl[d] = q.p[d] + u * q.t1[d] + v * q.t2[d];
+                    re[d] = rl[d] + uv * q.d[d];
+                    ne[d] = q.n0[d] + u * q.nu[d] + v * q.nv[d];
                 }
                 float fsr, fsi, fdr, fdi, lsr, lsi, ldr, ldi;
                 kern32(fam, kf, re, ne, do_s, do_d, fsr, fsi, fdr, fdi);
@@ -801,16 +817,16 @@ static __device__ __noinline__ void near_telles_sum_f32(const Elem64 &e, int fam
     for (int b = 0; b < 16; ++b) {
         double x, w;
         gauss_pt(16, b, x, w);
-        vv[b] = (float)(ca[1] * x * x * x + cb[1] * x * x + cc[1] * x + cdd[1] - im[1]);
-        tw[b] = (float)(w * (3.0 * ca[1] * x * x + 2.0 * cb[1] * x + cc[1]));
+        vv[b] = (float)(fma(fma(fma(ca[1], x, cb[1]), x, cc[1]), x, cdd[1] - im[1]));
+        tw[b] = (float)(w * fma(fma(3.0 * ca[1], x, 2.0 * cb[1]), x, cc[1]));
     }
     const float kf = (float)k;
     float sdr = 0, sdi = 0;
     for (int ia = 0; ia < 16; ++ia) {
         double x, w;
         gauss_pt(16, ia, x, w);
-        const float u = (float)(ca[0] * x * x * x + cb[0] * x * x + cc[0] * x + cdd[0] - im[0]);
-        const float w0 = (float)(w * (3.0 * ca[0] * x * x + 2.0 * cb[0] * x + cc[0]));
+        const float u = (float)(fma(fma(fma(ca[0], x, cb[0]), x, cc[0]), x, cdd[0] - im[0]));
+        const float w0 = (float)(w * fma(fma(3.0 * ca[0], x, 2.0 * cb[0]), x, cc[0]));
         float pr = 0, pim = 0;
         for (int ib = 0; ib < 16; ++ib) {
             const float v = vv[ib], uv = u * v;
@@ -846,10 +862,10 @@ static __device__ __noinline__ void near_dynamic_quad_f32(const Elem64 &e, doubl
     const float kf = (float)k;
     float sr = 0, si = 0, dr = 0, di = 0;
     for (int p = 0; p < 64; ++p) {
-        double xi, eta, w0, w1;
-        gauss_pt(8, p / 8, xi, w0);
-        gauss_pt(8, p % 8, eta, w1);
-        const float u = (float)xi, v = (float)eta, uv = u * v;
+        const int qa = (p >> 3) & 3, qb = p & 3;
+        const float u = p & 32 ? -GAUSS8_FF.xh[qa] : GAUSS8_FF.xh[qa], v = p & 4 ? -GAUSS8_FF.xh[qb] : GAUSS8_FF.xh[qb];
+        const float uv = u * v;
+        const float w = ff_mul(ff{GAUSS8_FF.wh[qa], GAUSS8_FF.wl[qa]}, ff{GAUSS8_FF.wh[qb], GAUSS8_FF.wl[qb]}).h;
         float rv[3], nv[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -865,7 +881,7 @@ static __device__ __noinline__ void near_dynamic_quad_f32(const Elem64 &e, doubl
         const float cm1 = -2.0f * hs * hs;  // cos kr - 1 without cancellation
         const float sn = 2.0f * hs * hc;
         const float cs = 1.0f + cm1;
-        const float t = (float)(w0 * w1) * J * rinv * INV4PI;
+        const float t = w * J * rinv * INV4PI;
         if (do_s) {
             sr += t * cm1;
             si -= t * sn;

@@ -45,7 +45,7 @@ struct OpSet {
 // cancels between the sides by more than three digits: |z| small against the
 // in-plane part of nx times the side, a folded pair whose collocation point
 // nearly lies in the element's plane; those take FP64.
-template <int G = 1>
+template <int G = 1, int SIDES = 3>
 __device__ inline bool near_static4_ff(const double *__restrict__ frame, const double c0[3], const double x0[3],
                                        const double nxg[3], OpSet ops, Acc4 &a, const Lanes<G> &g = Lanes<G>())
 {
@@ -64,8 +64,8 @@ __device__ inline bool near_static4_ff(const double *__restrict__ frame, const d
     const bool six = ops.s || ops.d || ops.t;
     double s_sum = 0.0, d_sum = 0.0, t_sum = 0.0, h_sum = 0.0;
 #pragma unroll 1
-    for (int sd = g.lane; sd < 3; sd += G) {
-        const int e1 = sd, e2 = sd == 2 ? 0 : sd + 1;
+    for (int sd = g.lane; sd < SIDES; sd += G) {
+        const int e1 = sd, e2 = sd == SIDES - 1 ? 0 : sd + 1;
         const double a0 = frame[9 + 2 * e1], a1 = frame[10 + 2 * e1], b0 = frame[9 + 2 * e2], b1 = frame[10 + 2 * e2];
         const double d0 = b0 - a0, d1 = b1 - a1, il = rsqrt(d0 * d0 + d1 * d1);
         const double l0 = d0 * il, l1 = d1 * il;
@@ -157,6 +157,27 @@ __device__ inline bool near_static4_ff(const double *__restrict__ frame, const d
     a.tr += t_sum * INV_FOUR_PI;
     if (ops.h) a.hr += (in_plane ? h_sum : h_sum / (z * (double)sc)) * (INV_FOUR_PI * sc);
     return true;
+}
+
+// near_static on a flat quadrilateral, for results that are stored in FP32: its
+// plane frame in FP64 (DevMesh::frame's layout, four corners), the rest as above
+static __device__ __noinline__ void near_static_quad_ff(const Elem64 &e, const double x0[3], bool do_s, bool do_d, Acc &a)
+{
+    double loc[4][2], z, T[3][3], frame[17];
+    plane_local_frame(e, x0, loc, z, T);
+    for (int d = 0; d < 3; ++d) {
+        frame[d] = T[0][d];
+        frame[3 + d] = T[1][d];
+        frame[6 + d] = T[2][d];
+    }
+    for (int c = 0; c < 4; ++c) {
+        frame[9 + 2 * c] = loc[c][0] - loc[0][0];
+        frame[10 + 2 * c] = loc[c][1] - loc[0][1];
+    }
+    Acc4 st;
+    near_static4_ff<1, 4>(frame, e.c[0], x0, x0, OpSet{do_s, do_d, false, false}, st);
+    if (do_s) a.sr += st.sr;
+    if (do_d) a.dr += st.dr;
 }
 
 }  // namespace nihu
