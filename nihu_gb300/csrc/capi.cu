@@ -1831,6 +1831,20 @@ nihu_gb_status gmres_cycle_multi(nihu_gb_ctx *ctx, const ApplyFn &apply, int64_t
     double2 *V = (double2 *)pV, *W = (double2 *)pW, *part = (double2 *)ppart, *hd = (double2 *)ph;
     double *scd = (double *)psc;
     const size_t blk = (size_t)n * nrhs;
+    // the FP32 copy of the basis that the Gram-Schmidt passes read; not under a
+    // memory budget or short of memory, which the copy must not use up: they then
+    // round the FP64 one as they read it
+    void *pV32 = nullptr;
+    const size_t bytes32 = 8 * blk * (m + 1);
+    const auto have = ctx->scratch.find("mr_V32");
+    if (have != ctx->scratch.end() && have->second.second >= bytes32) {
+        pV32 = have->second.first;
+    } else if (!ctx->budget) {
+        size_t free_mem = 0, all_mem = 0;
+        CK(cudaMemGetInfo(&free_mem, &all_mem));
+        if (bytes32 <= free_mem / 4 && (st = scratch(ctx, "mr_V32", bytes32, &pV32))) return st;
+    }
+    float2 *V32 = (float2 *)pV32;
     std::vector<double2> hh((size_t)(m + 1) * nrhs);
     std::vector<double> sc(nrhs);
 
@@ -1851,7 +1865,7 @@ nihu_gb_status gmres_cycle_multi(nihu_gb_ctx *ctx, const ApplyFn &apply, int64_t
         sc[r] = act[r] ? 1.0 / beta[r] : 0.0;
     }
     CK(cudaMemcpyAsync(scd, sc.data(), 8 * (size_t)nrhs, cudaMemcpyHostToDevice, ctx->stream));
-    CK(launch_bscale(R, V, n, nrhs, scd, ctx->stream));
+    CK(launch_bscale(R, V, V32, n, nrhs, scd, ctx->stream));
     ctx->launches += 1;
     std::vector<std::vector<C>> H(nrhs, std::vector<C>((size_t)(m + 1) * m, C(0)));
     std::vector<std::vector<C>> g(nrhs, std::vector<C>(m + 1, C(0))), cs(nrhs, std::vector<C>(m)), sn(nrhs, std::vector<C>(m));
@@ -1876,19 +1890,19 @@ nihu_gb_status gmres_cycle_multi(nihu_gb_ctx *ctx, const ApplyFn &apply, int64_t
         // inner solve of a refinement (inner tolerance 1e-3 or so), whose
         // residual the outer loop forms in FP64; the FP64 pipe stays free
         for (int pass = 0; pass < 2; ++pass) {
-            CK(launch_bdot(V, k + 1, W, n, nrhs, part, hd, ctx->stream, true));
+            CK(launch_bdot32(V, V32, k + 1, W, n, nrhs, part, hd, ctx->stream));
             CK(cudaMemcpyAsync(hh.data(), hd, 16 * (size_t)(k + 1) * nrhs, cudaMemcpyDeviceToHost, ctx->stream));
             if ((st = sync(ctx))) return st;
             for (int v = 0; v <= k; ++v)
                 for (int r = 0; r < nrhs; ++r) h[r][v] += C(hh[(size_t)v * nrhs + r].x, hh[(size_t)v * nrhs + r].y);
-            CK(launch_bcombo(V, n, nrhs, k + 1, hd, -1.0, W, ctx->stream, true));
+            CK(launch_bcombo32(V, V32, n, nrhs, k + 1, hd, -1.0, W, ctx->stream));
             ctx->launches += 3;
         }
         std::vector<double> hn(nrhs);
         if ((st = norms(W, hn))) return st;
         for (int r = 0; r < nrhs; ++r) sc[r] = (run[r] && hn[r] > 0.0) ? 1.0 / hn[r] : 0.0;
         CK(cudaMemcpyAsync(scd, sc.data(), 8 * (size_t)nrhs, cudaMemcpyHostToDevice, ctx->stream));
-        CK(launch_bscale(W, V + (size_t)(k + 1) * blk, n, nrhs, scd, ctx->stream));
+        CK(launch_bscale(W, V + (size_t)(k + 1) * blk, V32 ? V32 + (size_t)(k + 1) * blk : nullptr, n, nrhs, scd, ctx->stream));
         ctx->launches += 1;
         for (int r = 0; r < nrhs; ++r) {
             if (!run[r]) continue;

@@ -101,13 +101,19 @@ cudaError_t launch_gemm_tc(int parts, const void *A, int64_t m, int64_t n, int64
                            int64_t nrhs, double2 *Y, int64_t ldy, double are, double aim, double bre, double bim,
                            void *scratch, int *err, cudaStream_t s);
 int bdot_blocks(int64_t n);
-// fp32: products and partial sums in FP32 on the FP64-stored vectors (the
-// inner Arnoldi of a refinement), else FP64
 cudaError_t launch_bdot(const double2 *V, int nv, const double2 *W, int64_t n, int nrhs, double2 *part, double2 *out,
-                        cudaStream_t s, bool fp32 = false);
+                        cudaStream_t s);
 cudaError_t launch_bcombo(const double2 *V, int64_t n, int nrhs, int nv, const double2 *h, double sign, double2 *W,
-                          cudaStream_t s, bool fp32 = false);
-cudaError_t launch_bscale(const double2 *src, double2 *dst, int64_t n, int nrhs, const double *sc, cudaStream_t s);
+                          cudaStream_t s);
+// the same with products and partial sums in FP32 (the inner Arnoldi of a
+// refinement); V32: the basis V rounded to FP32, or NULL (rounded as it is read)
+cudaError_t launch_bdot32(const double2 *V, const float2 *V32, int nv, const double2 *W, int64_t n, int nrhs,
+                          double2 *part, double2 *out, cudaStream_t s);
+cudaError_t launch_bcombo32(const double2 *V, const float2 *V32, int64_t n, int nrhs, int nv, const double2 *h,
+                            double sign, double2 *W, cudaStream_t s);
+// dst = src * sc per right-hand side, and its FP32 copy dst32 (may be NULL)
+cudaError_t launch_bscale(const double2 *src, double2 *dst, float2 *dst32, int64_t n, int nrhs, const double *sc,
+                          cudaStream_t s);
 cudaError_t launch_rsub(const double2 *B, double2 *R, size_t count, cudaStream_t s);
 
 }  // namespace nihu

@@ -91,31 +91,47 @@ cudaError_t launch_gemm_c64(void *cublas, int mode, const void *A, int64_t m, in
 constexpr int BT = 256;
 
 // part[((v * nrhs + r) * blocks + b)] = sum over the block's rows of conj(V_v[:, r]) . W[:, r];
-// F32: products and the thread's and warp's sums in FP32 (the block's in FP64)
-template <bool F32>
-__global__ void __launch_bounds__(BT) k_bdot(const double2 *__restrict__ V, const double2 *__restrict__ W, int64_t n,
-                                             int nrhs, double2 *part)
+// F32: products and the thread's and warp's sums in FP32 (the block's in FP64),
+// four basis vectors to a block, which convert W once.  V2: float2 reads a copy
+// of the basis that was rounded once, with the same products: the conversions
+// of the FP64 one, four a point and vector on the narrow FP64 pipe, bounded the
+// Gram-Schmidt passes (15 680 unknowns, 64 right-hand sides, 16 steps: the
+// solve 15.5 ms, here 14.0).
+template <bool F32, class V2>
+__global__ void __launch_bounds__(BT) k_bdot(const V2 *__restrict__ V, const double2 *__restrict__ W, int64_t n,
+                                             int nrhs, int nv, double2 *part)
 {
-    __shared__ double sr[BT / 32], si[BT / 32];
-    const int v = blockIdx.z, r = blockIdx.y;
-    const double2 *a = V + ((int64_t)v * nrhs + r) * n;
+    constexpr int NV = F32 ? 4 : 1;
+    __shared__ double sr[NV][BT / 32], si[NV][BT / 32];
+    const int v0 = blockIdx.z * NV, r = blockIdx.y;
+    const V2 *a = V + ((int64_t)v0 * nrhs + r) * n;
     const double2 *b = W + (int64_t)r * n;
+    const int64_t next = (int64_t)nrhs * n;
     using T = std::conditional_t<F32, float, double>;
-    T ar = 0, ai = 0;
+    T ar[NV] = {}, ai[NV] = {};
     for (int64_t i = (int64_t)blockIdx.x * BT + threadIdx.x; i < n; i += (int64_t)gridDim.x * BT) {
-        const double2 x = a[i], y = b[i];
-        const T xr = (T)x.x, xi = (T)x.y, yr = (T)y.x, yi = (T)y.y;
-        ar += xr * yr + xi * yi;
-        ai += xr * yi - xi * yr;
+        const double2 y = b[i];
+        const T yr = (T)y.x, yi = (T)y.y;
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+            if (v0 + u >= nv) break;
+            const V2 x = a[u * next + i];
+            const T xr = (T)x.x, xi = (T)x.y;
+            ar[u] += xr * yr + xi * yi;
+            ai[u] += xr * yi - xi * yr;
+        }
     }
-    ar = warp_sum(ar);
-    ai = warp_sum(ai);
-    if ((threadIdx.x & 31) == 0) { sr[threadIdx.x >> 5] = ar; si[threadIdx.x >> 5] = ai; }
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+        const T wr = warp_sum(ar[u]), wi = warp_sum(ai[u]);
+        if ((threadIdx.x & 31) == 0) { sr[u][threadIdx.x >> 5] = wr; si[u][threadIdx.x >> 5] = wi; }
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    const int u = threadIdx.x;
+    if (u < NV && v0 + u < nv) {
         double tr = 0.0, ti = 0.0;
-        for (int k = 0; k < BT / 32; ++k) { tr += sr[k]; ti += si[k]; }
-        part[((int64_t)v * nrhs + r) * gridDim.x + blockIdx.x] = make_double2(tr, ti);
+        for (int k = 0; k < BT / 32; ++k) { tr += sr[u][k]; ti += si[u][k]; }
+        part[((int64_t)(v0 + u) * nrhs + r) * gridDim.x + blockIdx.x] = make_double2(tr, ti);
     }
 }
 
@@ -134,36 +150,53 @@ __global__ void k_bdot_reduce(const double2 *__restrict__ part, int count, int b
 }
 
 // W[:, r] += sign * sum_{v < nv} V_v[:, r] h[v * nrhs + r]; F32: the sum in FP32
-template <bool F32>
-__global__ void k_bcombo(const double2 *__restrict__ V, int64_t n, int nrhs, int nv, const double2 *__restrict__ h,
+template <bool F32, class V2>
+__global__ void k_bcombo(const V2 *__restrict__ V, int64_t n, int nrhs, int nv, const double2 *__restrict__ h,
                          double sign, double2 *W)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int r = blockIdx.y;
-    if (i >= n) return;
     using T = std::conditional_t<F32, float, double>;
+    constexpr int TILE = 64;  // coefficients staged at a time
+    __shared__ T hr[TILE], hi[TILE];
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = blockIdx.y;
     T sr = 0, si = 0;
-    for (int v = 0; v < nv; ++v) {
-        const double2 a = V[((int64_t)v * nrhs + r) * n + i], c = h[v * nrhs + r];
-        const T ar = (T)a.x, ai = (T)a.y, cr = (T)c.x, ci = (T)c.y;
-        sr += ar * cr - ai * ci;
-        si += ar * ci + ai * cr;
+    for (int v0 = 0; v0 < nv; v0 += TILE) {
+        const int nt = min(TILE, nv - v0);
+        __syncthreads();
+        if (threadIdx.x < nt) {
+            const double2 c = h[(v0 + threadIdx.x) * nrhs + r];
+            hr[threadIdx.x] = (T)c.x;
+            hi[threadIdx.x] = (T)c.y;
+        }
+        __syncthreads();
+        if (i < n)
+#pragma unroll 4
+            for (int v = 0; v < nt; ++v) {
+                const V2 a = V[((int64_t)(v0 + v) * nrhs + r) * n + i];
+                const T ar = (T)a.x, ai = (T)a.y, cr = hr[v], ci = hi[v];
+                sr += ar * cr - ai * ci;
+                si += ar * ci + ai * cr;
+            }
     }
+    if (i >= n) return;
     double2 acc = W[(int64_t)r * n + i];
     acc.x += sign * (double)sr;
     acc.y += sign * (double)si;
     W[(int64_t)r * n + i] = acc;
 }
 
-// dst[:, r] = src[:, r] * s[r]
-__global__ void k_bscale(const double2 *__restrict__ src, double2 *dst, int64_t n, const double *__restrict__ s)
+// dst[:, r] = src[:, r] * s[r], and its FP32 copy dst32 (may be NULL)
+__global__ void k_bscale(const double2 *__restrict__ src, double2 *dst, float2 *dst32, int64_t n,
+                         const double *__restrict__ s)
 {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int r = blockIdx.y;
     if (i >= n) return;
     double2 v = src[(int64_t)r * n + i];
     double f = s[r];
-    dst[(int64_t)r * n + i] = make_double2(v.x * f, v.y * f);
+    v = make_double2(v.x * f, v.y * f);
+    dst[(int64_t)r * n + i] = v;
+    if (dst32) dst32[(int64_t)r * n + i] = make_float2((float)v.x, (float)v.y);
 }
 
 // R = B - R (element-wise, count complex values)
@@ -188,31 +221,51 @@ int bdot_blocks(int64_t n)
     return (int)max((int64_t)1, min(b, (int64_t)16));
 }
 
-cudaError_t launch_bdot(const double2 *V, int nv, const double2 *W, int64_t n, int nrhs, double2 *part, double2 *out,
-                        cudaStream_t s, bool fp32)
+static cudaError_t bdot_reduce(const double2 *part, int count, int blocks, double2 *out, cudaStream_t s)
 {
-    int blocks = bdot_blocks(n);
-    dim3 g(blocks, nrhs, nv);
-    if (fp32) k_bdot<true><<<g, BT, 0, s>>>(V, W, n, nrhs, part);
-    else k_bdot<false><<<g, BT, 0, s>>>(V, W, n, nrhs, part);
-    int count = nv * nrhs;
     k_bdot_reduce<<<(count + 255) / 256, 256, 0, s>>>(part, count, blocks, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_bcombo(const double2 *V, int64_t n, int nrhs, int nv, const double2 *h, double sign, double2 *W,
-                          cudaStream_t s, bool fp32)
+cudaError_t launch_bdot(const double2 *V, int nv, const double2 *W, int64_t n, int nrhs, double2 *part, double2 *out,
+                        cudaStream_t s)
 {
-    dim3 g((unsigned)((n + 255) / 256), nrhs);
-    if (fp32) k_bcombo<true><<<g, 256, 0, s>>>(V, n, nrhs, nv, h, sign, W);
-    else k_bcombo<false><<<g, 256, 0, s>>>(V, n, nrhs, nv, h, sign, W);
+    const int blocks = bdot_blocks(n);
+    k_bdot<false><<<dim3(blocks, nrhs, nv), BT, 0, s>>>(V, W, n, nrhs, nv, part);
+    return bdot_reduce(part, nv * nrhs, blocks, out, s);
+}
+
+cudaError_t launch_bdot32(const double2 *V, const float2 *V32, int nv, const double2 *W, int64_t n, int nrhs,
+                          double2 *part, double2 *out, cudaStream_t s)
+{
+    const int blocks = bdot_blocks(n);
+    const dim3 g(blocks, nrhs, (nv + 3) / 4);
+    if (V32) k_bdot<true><<<g, BT, 0, s>>>(V32, W, n, nrhs, nv, part);
+    else k_bdot<true><<<g, BT, 0, s>>>(V, W, n, nrhs, nv, part);
+    return bdot_reduce(part, nv * nrhs, blocks, out, s);
+}
+
+cudaError_t launch_bcombo(const double2 *V, int64_t n, int nrhs, int nv, const double2 *h, double sign, double2 *W,
+                          cudaStream_t s)
+{
+    k_bcombo<false><<<dim3((unsigned)((n + 255) / 256), nrhs), 256, 0, s>>>(V, n, nrhs, nv, h, sign, W);
     return cudaGetLastError();
 }
 
-cudaError_t launch_bscale(const double2 *src, double2 *dst, int64_t n, int nrhs, const double *sc, cudaStream_t s)
+cudaError_t launch_bcombo32(const double2 *V, const float2 *V32, int64_t n, int nrhs, int nv, const double2 *h,
+                            double sign, double2 *W, cudaStream_t s)
+{
+    const dim3 g((unsigned)((n + 255) / 256), nrhs);
+    if (V32) k_bcombo<true><<<g, 256, 0, s>>>(V32, n, nrhs, nv, h, sign, W);
+    else k_bcombo<true><<<g, 256, 0, s>>>(V, n, nrhs, nv, h, sign, W);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bscale(const double2 *src, double2 *dst, float2 *dst32, int64_t n, int nrhs, const double *sc,
+                          cudaStream_t s)
 {
     dim3 g((unsigned)((n + 255) / 256), nrhs);
-    k_bscale<<<g, 256, 0, s>>>(src, dst, n, sc);
+    k_bscale<<<g, 256, 0, s>>>(src, dst, dst32, n, sc);
     return cudaGetLastError();
 }
 
