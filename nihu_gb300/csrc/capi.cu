@@ -1430,8 +1430,8 @@ namespace {
 // correction is within 64 FP64 roundings of x (|d| <= 64 eps |x|, the
 // accuracy of an FP64 factorisation).  *refined = false (and nothing solved)
 // when the order is beyond the FP32 kernels' shared memory and registers or the
-// corrections stop shrinking (cond(A) near 1 / eps32): the caller then
-// factorises in FP64.  A is left unchanged.
+// corrections stop shrinking (cond(A) near 1 / eps32), or a memory budget has no
+// room for the inverses: the caller then factorises in FP64.  A is left unchanged.
 nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int64_t lda, const double2 *b, double2 *x,
                               bool *refined)
 {
@@ -1443,7 +1443,15 @@ nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int
     void *pf, *paux, *pd, *pr, *psums, *ppart;
     const int splits = gemv_splits(n, n, NIHU_GB_C128);
     if ((st = scratch(ctx, "lu32_F", 8 * (size_t)n * n, &pf))) return st;
-    if ((st = scratch(ctx, "lu32_aux", lu32_aux_bytes((int)n), &paux))) return st;
+    {
+        // the diagonal blocks' inverses are 1 KB a row: where a memory budget has no room
+        // for them the caller's FP64 factorisation, which needs none, still runs
+        const std::string msg = ctx->err;
+        if (scratch(ctx, "lu32_aux", lu32_aux_bytes((int)n), &paux)) {
+            ctx->err = msg;
+            return NIHU_GB_OK;
+        }
+    }
     if ((st = scratch(ctx, "lu32_d", 16 * (size_t)n, &pd))) return st;
     if ((st = scratch(ctx, "lu32_r", 16 * (size_t)n, &pr))) return st;
     if ((st = scratch(ctx, "lu32_sums", 2 * sizeof(double), &psums))) return st;

@@ -67,3 +67,12 @@ def test_zero_column_is_named(gpu_ctx, n, col):
     A[:, col] = 0
     with pytest.raises(g.NihuError, match=re.escape(f"zero pivot in column {col})")):
         g.lu_solve(A, rand_c(rng, n), ctx=gpu_ctx)
+
+
+def test_budget_without_room_for_the_inverses(gpu_ctx):
+    # FP64 matrix, FP32 factors and the vectors fit, 1 KB a row more does not
+    n = 600
+    rng = np.random.default_rng(n)
+    A, b = rand_c(rng, n, n), rand_c(rng, n)
+    ctx = g.api.Context(hbm_budget_bytes=24 * n * n + 200 * n)
+    assert backward_error(A, g.lu_solve(A, b, ctx=ctx), b) <= 1e-13
