@@ -6,8 +6,8 @@
 // Laplace 3D SLP/DLP kernels (nihu/library/helmholtz_kernel.hpp:180-195,
 // laplace_kernel.hpp:137-147, normal_derivative_kernel.hpp:131-175).
 //
-// Work layout: a block owns REG_THREADS consecutive test rows and REG_COLS
-// consecutive trial columns.  A thread owns one row; for each column it
+// Work layout (k_regular): a block owns REG_THREADS consecutive test rows and up
+// to REG_COLS consecutive trial columns.  A thread owns one row; for each column it
 // classifies the pair (classify.cuh), evaluates the selected rule(s) and
 // writes the entry.  Writes of a warp are 32 consecutive entries of one
 // column of the column-major matrix (256 B for complex64), so the dominant

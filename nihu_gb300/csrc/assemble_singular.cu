@@ -1,8 +1,9 @@
 // FP64 singular (self) and nearly singular collocational entries.
 //
-// One thread evaluates one (test, trial) pair.  GB300's FP64 pipe is narrow,
-// so the per-pair set-up (plane transform, side angles, inverse mapping) is
-// done exactly once per pair -- never replicated across lanes -- and every
+// One thread evaluates one (test, trial) pair (k_singular_tria, k_singular_quad: a
+// few lanes where there are few pairs).  GB300's FP64 pipe is narrow, so
+// the per-pair set-up (plane transform, side angles, inverse mapping) is done
+// once per pair where there are many, and every
 // quadrature point shares one sincos and one reciprocal square root between
 // the SLP and the DLP and between the Helmholtz and Laplace parts of the
 // kernel difference.  Threads of a warp take consecutive pairs of the
@@ -624,6 +625,84 @@ static cudaError_t launch_singular_tria_g(const RegularArgs &a, const NearList &
     return launch_singular_tria<Out, CK, 1>(a, near, items, sms, dev, s);
 }
 
+// The same on meshes with quads, real wave number, into complex64: the rules of
+// singular_pairs under FP32 quadrature with their points over G lanes.  The
+// FP64 set-up (inverse mapping, Telles coefficients: about 3 000 operations a
+// pair) is repeated on each lane, so few lanes where there are many pairs.
+template <int G>
+__global__ void __launch_bounds__(SING_THREADS, 4) k_singular_quad(const __grid_constant__ RegularArgs a, NearList near, int *err)
+{
+    const int64_t p_begin = near.col_ptr ? near.col_ptr[a.j0] : 0;
+    const int64_t n_near = (near.col_ptr ? near.col_ptr[a.j1] : 0) - p_begin;
+    const int64_t n_self = a.same_mesh ? (int64_t)(min(a.j1, a.test.n) - a.j0) : 0;
+    const bool do_s = (a.ops & OP_SLP) != 0, do_d = (a.ops & OP_DLP) != 0;
+    const int fam = a.family;
+    const bool telles = fam == FAM_HELMHOLTZ && do_d, polar_d = fam == FAM_LAPLACE && do_d;
+    float2 *out_s = reinterpret_cast<float2 *>(a.out_s), *out_d = reinterpret_cast<float2 *>(a.out_d);
+    const int64_t thread = (int64_t)blockIdx.x * SING_THREADS + threadIdx.x, threads = (int64_t)gridDim.x * SING_THREADS;
+    auto put = [&](int i, int j, const Acc &v) {
+        const int64_t off = (int64_t)(j - a.j0) * a.ld + i;
+        if (do_s) store64(out_s + off, v.sr, v.si, a.alpha_re, a.alpha_im, a.accumulate);
+        if (do_d) store64(out_d + off, v.dr, v.di, a.alpha_re, a.alpha_im, a.accumulate);
+    };
+    const Lanes<G> g;
+    for (int64_t item = thread / G; item < n_near; item += threads / G) {
+        const int64_t p = p_begin + item;
+        const int i = near.rows[p], j = near_column(near.col_ptr, a.j0, a.j1, p);
+        double x0[3];
+        for (int d = 0; d < 3; ++d) x0[d] = a.test.center[3 * (int64_t)i + d];
+        Elem64 e;
+        load_elem(a.trial, j, e);
+        Acc acc;
+        if (e.nc == 3) {
+            if (fam == FAM_HELMHOLTZ) near_dynamic_f32<G>(e, a.k, x0, do_s, do_d, acc, g);
+            near_static_f32<G>(e, a.trial.frame + 16 * (int64_t)j, x0, do_s, do_d, acc, g);
+        } else {
+            double r5[3] = {0, 0, 0}, r6[3] = {0, 0, 0};
+            if (!inverse_mapping(e, x0, telles, r5, r6)) {
+                if (g.lane == 0) atomicCAS(err, 0, (int)min(item + 1, (int64_t)0x7fffffff));
+                continue;
+            }
+            if (do_s || polar_d) {
+                Elem64 lin;
+                linearized(e, r5[0], r5[1], lin);
+                near_polar_sum_f32<G>(e, fam, a.k, x0, r5[0], r5[1], do_s, polar_d, acc, g);
+                if (fam == FAM_HELMHOLTZ) near_dynamic_quad_f32<G>(lin, a.k, x0, do_s, polar_d, acc, g);
+                near_static_quad_ff<G>(lin, x0, do_s, polar_d, acc, g);
+            }
+            if (telles) near_telles_sum_f32<G>(e, fam, a.k, x0, r6, acc, g);
+        }
+        if (g.lane == 0) put(i, j, acc);
+    }
+    // self terms, 16 lanes each
+    const Lanes<16> h;
+    for (int64_t item = thread / 16; item < n_self; item += threads / 16) {
+        const int j = a.j0 + (int)item;
+        double x0[3];
+        for (int d = 0; d < 3; ++d) x0[d] = a.test.center[3 * (int64_t)j + d];
+        Elem64 e;
+        load_elem(a.trial, j, e);
+        Acc acc;
+        if (e.nc != 3) self_quad(e, fam, a.k, x0, do_s, do_d, acc, h);
+        else if (do_s) self_tria_lanes<false>(e, fam, cd{a.k, 0.0}, x0, acc, h);
+        if (h.lane == 0) put(j, j, acc);
+    }
+}
+
+template <int G>
+static cudaError_t launch_singular_quad(const RegularArgs &a, const NearList &near, int64_t items, int sms, int *err,
+                                        cudaStream_t s)
+{
+    const cudaError_t e = cudaFuncSetAttribute(k_singular_quad<G>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               regular_carveout_percent());
+    if (e != cudaSuccess) return e;
+    const int64_t near_n = near.col_ptr ? near.nnz : 0, self_n = items - near_n;
+    const int64_t want = (std::max(near_n * G, self_n * 16) + SING_THREADS - 1) / SING_THREADS;
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, 4 * (int64_t)sms));
+    k_singular_quad<G><<<blocks, SING_THREADS, 0, s>>>(a, near, err);
+    return cudaGetLastError();
+}
+
 // held to 128 registers so that three blocks of the concurrent regular kernel
 // keep every SM beside this kernel's one (it would take 164 by itself, with
 // the FP32 dynamic part beside the FP64 schemes, which left room for two)
@@ -702,6 +781,15 @@ cudaError_t launch_assemble_singular(const RegularArgs &a, const NearList &near,
         const int g = items * 4 <= room ? 4 : (items * 2 <= room ? 2 : 1);
         return a.k_im != 0.0 ? launch_singular_tria_g<float2, true>(a, near, items, g, sms, dev, s)
                              : launch_singular_tria_g<float2, false>(a, near, items, g, sms, dev, s);
+    }
+    if (a.precision == 0 && a.dtype == 0 && a.nk <= 1 && !a.force_batch && a.trial.has_quad && a.k_im == 0.0) {
+        // few pairs are bound by one pair's chain, many by the repeated set-up
+        // (cylinders of 288 / 1480 / 2496 / 5544 / 9792 quads, eight items a quad, a
+        // call: k_singular 650 / 666 / 697 / 890 / 1200 us, 2 lanes 317 / 353 / 418 /
+        // 743 / 1286, 4 lanes 218 / 336 / 516 / 990 / 1705)
+        const int64_t room = 4 * (int64_t)sms * SING_THREADS;
+        if (items * 6 <= room) return launch_singular_quad<4>(a, near, items, sms, err, s);
+        if (items * 4 <= room * 3) return launch_singular_quad<2>(a, near, items, sms, err, s);
     }
     // this kernel needs no shared memory, but the regular kernel's blocks
     // beside it do: the same carveout preference as theirs, so that an SM

@@ -717,8 +717,9 @@ __device__ __forceinline__ void kern32(int fam, float k, const float rv[3], cons
 // were a third of the singular kernel's time on quads (with the static part in
 // float-float and fewer divisions in the inverse mapping, closed cylinder of
 // 9 792 quads, SLP and DLP: 1997 -> 1200 us; entries' error unchanged).
+template <int G = 1>
 static __device__ __noinline__ void near_polar_sum_f32(const Elem64 &e, int fam, double k, const double x0[3], double xi0,
-                                          double eta0, bool do_s, bool do_d, Acc &a)
+                                          double eta0, bool do_s, bool do_d, Acc &a, const Lanes<G> &g = Lanes<G>())
 {
     QuadAround32 q;
     quad_around32(e, x0, xi0, eta0, q);
@@ -726,7 +727,7 @@ static __device__ __noinline__ void near_polar_sum_f32(const Elem64 &e, int fam,
     const ff xm = ff_from(-1.0 - xi0), xp = ff_from(1.0 - xi0), em = ff_from(-1.0 - eta0), ep = ff_from(1.0 - eta0);
     float sr = 0, si = 0, dsr = 0, dsi = 0;
 #pragma unroll 1
-    for (int n = 0; n < 4; ++n) {
+    for (int n = g.lane; n < 4; n += G) {
         // along the side (corners n and n + 1 counter-clockwise) and across it
         const bool back = n >= 2, vertical = n & 1;
         const ff lo = vertical ? em : xm, hi = vertical ? ep : xp;
@@ -780,16 +781,17 @@ static __device__ __noinline__ void near_polar_sum_f32(const Elem64 &e, int fam,
             dsi += wth * pdi;
         }
     }
-    a.sr += sr;
-    a.si += si;
-    a.dr += dsr;
-    a.di += dsi;
+    a.sr += g.sum(sr);
+    a.si += g.sum(si);
+    a.dr += g.sum(dsr);
+    a.di += g.sum(dsi);
 }
 
 // near_telles_sum with the FP32 sums (quads): the Telles coefficients in FP64,
 // the points expanded around the inverse-mapped point
+template <int G = 1>
 static __device__ __noinline__ void near_telles_sum_f32(const Elem64 &e, int fam, double k, const double x0[3], const double im[3],
-                                           Acc &a)
+                                           Acc &a, const Lanes<G> &g = Lanes<G>())
 {
     double dist = im[2];
     double rb;
@@ -822,7 +824,7 @@ static __device__ __noinline__ void near_telles_sum_f32(const Elem64 &e, int fam
     }
     const float kf = (float)k;
     float sdr = 0, sdi = 0;
-    for (int ia = 0; ia < 16; ++ia) {
+    for (int ia = g.lane; ia < 16; ia += G) {
         double x, w;
         gauss_pt(16, ia, x, w);
         const float u = (float)(fma(fma(fma(ca[0], x, cb[0]), x, cc[0]), x, cdd[0] - im[0]));
@@ -844,14 +846,15 @@ static __device__ __noinline__ void near_telles_sum_f32(const Elem64 &e, int fam
         sdr += w0 * pr;
         sdi += w0 * pim;
     }
-    a.dr += sdr;
-    a.di += sdi;
+    a.dr += g.sum(sdr);
+    a.di += g.sum(sdi);
 }
 
 // the dynamic part K_k - K_0 of near_plane over a flat (linearised) quad in
 // FP32: 8 x 8 Gauss as near_dynamic, points expanded around the centre
+template <int G = 1>
 static __device__ __noinline__ void near_dynamic_quad_f32(const Elem64 &e, double k, const double x0[3], bool do_s, bool do_d,
-                                             Acc &a)
+                                             Acc &a, const Lanes<G> &g = Lanes<G>())
 {
     QuadAround32 q;
     quad_around32(e, x0, 0.0, 0.0, q);
@@ -861,7 +864,7 @@ static __device__ __noinline__ void near_dynamic_quad_f32(const Elem64 &e, doubl
     constexpr float INV4PI = (float)INV_FOUR_PI;
     const float kf = (float)k;
     float sr = 0, si = 0, dr = 0, di = 0;
-    for (int p = 0; p < 64; ++p) {
+    for (int p = g.lane; p < 64; p += G) {
         const int qa = (p >> 3) & 3, qb = p & 3;
         const float u = p & 32 ? -GAUSS8_FF.xh[qa] : GAUSS8_FF.xh[qa], v = p & 4 ? -GAUSS8_FF.xh[qb] : GAUSS8_FF.xh[qb];
         const float uv = u * v;
@@ -892,44 +895,51 @@ static __device__ __noinline__ void near_dynamic_quad_f32(const Elem64 &e, doubl
             di -= uu * (kr * cs - sn);
         }
     }
-    a.sr += sr;
-    a.si += si;
-    a.dr += dr;
-    a.di += di;
+    a.sr += g.sum(sr);
+    a.si += g.sum(si);
+    a.dr += g.sum(dr);
+    a.di += g.sum(di);
 }
 
 
-template <class K>
-__device__ inline void self_quad(const Elem64 &e, int fam, K k, const double x0[3], bool do_s, bool do_d, Acc &a)
+template <class K, int G = 1>
+__device__ inline void self_quad(const Elem64 &e, int fam, K k, const double x0[3], bool do_s, bool do_d, Acc &acc,
+                                 const Lanes<G> &g = Lanes<G>())
 {
+    Acc a;
     for (int d = 0; d < 4; ++d) {
         double P2[2], P3[2];
         domain_corner(4, d, P2[0], P2[1]);
         domain_corner(4, (d + 1) % 4, P3[0], P3[1]);
-        for (int ia = 0; ia < 4; ++ia)
-            for (int ib = 0; ib < 4; ++ib) {
-                double u, wu, v, wv;
-                gauss_pt(4, ia, u, wu);
-                gauss_pt(4, ib, v, wv);
-                // corners P0 = P1 = (0,0) (the collocation point), P2, P3
-                double N[4], dN[4][2];
-                shape(4, u, v, N);
-                dshape(4, u, v, dN);
-                double xi = N[2] * P2[0] + N[3] * P3[0];
-                double eta = N[2] * P2[1] + N[3] * P3[1];
-                double j00 = dN[2][0] * P2[0] + dN[3][0] * P3[0];
-                double j01 = dN[2][0] * P2[1] + dN[3][0] * P3[1];
-                double j10 = dN[2][1] * P2[0] + dN[3][1] * P3[0];
-                double j11 = dN[2][1] * P2[1] + dN[3][1] * P3[1];
-                double wd = wu * wv * (j00 * j11 - j01 * j10);
-                cd ks{0, 0}, kd{0, 0};
-                kern_on_elem(e, fam, k, x0, xi, eta, do_s, do_d, ks, kd);
-                a.sr += ks.re * wd;
-                a.si += ks.im * wd;
-                a.dr += kd.re * wd;
-                a.di += kd.im * wd;
-            }
+        // point by point, or a lane's points (G a power of two up to 16)
+        for (int p = g.lane; p < 16; p += G) {
+            const int ia = p >> 2, ib = p & 3;
+            double u, wu, v, wv;
+            gauss_pt(4, ia, u, wu);
+            gauss_pt(4, ib, v, wv);
+            // corners P0 = P1 = (0,0) (the collocation point), P2, P3
+            double N[4], dN[4][2];
+            shape(4, u, v, N);
+            dshape(4, u, v, dN);
+            double xi = N[2] * P2[0] + N[3] * P3[0];
+            double eta = N[2] * P2[1] + N[3] * P3[1];
+            double j00 = dN[2][0] * P2[0] + dN[3][0] * P3[0];
+            double j01 = dN[2][0] * P2[1] + dN[3][0] * P3[1];
+            double j10 = dN[2][1] * P2[0] + dN[3][1] * P3[0];
+            double j11 = dN[2][1] * P2[1] + dN[3][1] * P3[1];
+            double wd = wu * wv * (j00 * j11 - j01 * j10);
+            cd ks{0, 0}, kd{0, 0};
+            kern_on_elem(e, fam, k, x0, xi, eta, do_s, do_d, ks, kd);
+            a.sr += ks.re * wd;
+            a.si += ks.im * wd;
+            a.dr += kd.re * wd;
+            a.di += kd.im * wd;
+        }
     }
+    acc.sr += g.sum(a.sr);
+    acc.si += g.sum(a.si);
+    acc.dr += g.sum(a.dr);
+    acc.di += g.sum(a.di);
 }
 
 }  // namespace nihu

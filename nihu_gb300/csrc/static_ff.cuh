@@ -161,7 +161,9 @@ __device__ inline bool near_static4_ff(const double *__restrict__ frame, const d
 
 // near_static on a flat quadrilateral, for results that are stored in FP32: its
 // plane frame in FP64 (DevMesh::frame's layout, four corners), the rest as above
-static __device__ __noinline__ void near_static_quad_ff(const Elem64 &e, const double x0[3], bool do_s, bool do_d, Acc &a)
+template <int G = 1>
+static __device__ __noinline__ void near_static_quad_ff(const Elem64 &e, const double x0[3], bool do_s, bool do_d, Acc &a,
+                                                        const Lanes<G> &g = Lanes<G>())
 {
     double loc[4][2], z, T[3][3], frame[17];
     plane_local_frame(e, x0, loc, z, T);
@@ -175,7 +177,7 @@ static __device__ __noinline__ void near_static_quad_ff(const Elem64 &e, const d
         frame[10 + 2 * c] = loc[c][1] - loc[0][1];
     }
     Acc4 st;
-    near_static4_ff<1, 4>(frame, e.c[0], x0, x0, OpSet{do_s, do_d, false, false}, st);
+    near_static4_ff<G, 4>(frame, e.c[0], x0, x0, OpSet{do_s, do_d, false, false}, st, g);
     if (do_s) a.sr += st.sr;
     if (do_d) a.dr += st.dr;
 }

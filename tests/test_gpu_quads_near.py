@@ -72,3 +72,20 @@ def test_points_above(gpu_ctx, oracle, shift, k):
     # above the middle, a side, a corner and elsewhere
     mesh = plate(5, 5)
     check(gpu_ctx, oracle, (mesh[0] + np.array(shift), mesh[1]), mesh, k)
+
+
+@pytest.mark.parametrize("k", [0.0, 3.0])
+@pytest.mark.parametrize("n", [3, 14, 18, 30])
+def test_lanes_by_number_of_pairs(gpu_ctx, oracle, n, k):
+    # 54 to 5400 quads: four lanes a pair, two, and (from about 7 000 quads) one;
+    # rows of two ends of the mesh
+    mesh = meshes.cube_sphere(n)
+    if n < 30:
+        return check(gpu_ctx, oracle, mesh, mesh, k)
+    family, fam = (g.HELMHOLTZ_3D, oracle.HELMHOLTZ) if k else (g.LAPLACE_3D, oracle.LAPLACE)
+    S, D = assemble(gpu_ctx, mesh, mesh, family, k)
+    for rows in ((0, 40), (len(mesh[1]) - 40, len(mesh[1]))):
+        s = oracle.assemble(mesh, mesh, fam, oracle.SLP, k, rows=rows, threads=8)
+        d = oracle.assemble(mesh, mesh, fam, oracle.DLP, k, rows=rows, threads=8)
+        assert np.abs(S[rows[0]:rows[1]] - s).max() <= 1e-5 * np.abs(s).max()
+        assert np.abs(D[rows[0]:rows[1]] - d).max() <= 1e-5 * np.abs(d).max()
