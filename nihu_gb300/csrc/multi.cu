@@ -92,16 +92,15 @@ constexpr int BT = 256;
 
 // part[((v * nrhs + r) * blocks + b)] = sum over the block's rows of conj(V_v[:, r]) . W[:, r];
 // F32: products and the thread's and warp's sums in FP32 (the block's in FP64),
-// four basis vectors to a block, which convert W once.  V2: float2 reads a copy
+// NV basis vectors to a block, which convert W once.  V2: float2 reads a copy
 // of the basis that was rounded once, with the same products: the conversions
 // of the FP64 one, four a point and vector on the narrow FP64 pipe, bounded the
 // Gram-Schmidt passes (15 680 unknowns, 64 right-hand sides, 16 steps: the
 // solve 15.5 ms, here 14.0).
-template <bool F32, class V2>
+template <bool F32, int NV, class V2>
 __global__ void __launch_bounds__(BT) k_bdot(const V2 *__restrict__ V, const double2 *__restrict__ W, int64_t n,
                                              int nrhs, int nv, double2 *part)
 {
-    constexpr int NV = F32 ? 4 : 1;
     __shared__ double sr[NV][BT / 32], si[NV][BT / 32];
     const int v0 = blockIdx.z * NV, r = blockIdx.y;
     const V2 *a = V + ((int64_t)v0 * nrhs + r) * n;
@@ -150,32 +149,50 @@ __global__ void k_bdot_reduce(const double2 *__restrict__ part, int count, int b
 }
 
 // W[:, r] += sign * sum_{v < nv} V_v[:, r] h[v * nrhs + r]; F32: the sum in FP32
-template <bool F32, class V2>
-__global__ void k_bcombo(const V2 *__restrict__ V, int64_t n, int nrhs, int nv, const double2 *__restrict__ h,
+template <bool F32>
+__global__ void k_bcombo(const double2 *__restrict__ V, int64_t n, int nrhs, int nv, const double2 *__restrict__ h,
                          double sign, double2 *W)
 {
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int r = blockIdx.y;
+    if (i >= n) return;
     using T = std::conditional_t<F32, float, double>;
+    T sr = 0, si = 0;
+    for (int v = 0; v < nv; ++v) {
+        const double2 a = V[((int64_t)v * nrhs + r) * n + i], c = h[v * nrhs + r];
+        const T ar = (T)a.x, ai = (T)a.y, cr = (T)c.x, ci = (T)c.y;
+        sr += ar * cr - ai * ci;
+        si += ar * ci + ai * cr;
+    }
+    double2 acc = W[(int64_t)r * n + i];
+    acc.x += sign * (double)sr;
+    acc.y += sign * (double)si;
+    W[(int64_t)r * n + i] = acc;
+}
+
+// the same from the FP32 copy of the basis, the coefficients rounded once a block
+__global__ void __launch_bounds__(256) k_bcombo32(const float2 *__restrict__ V, int64_t n, int nrhs, int nv,
+                                                  const double2 *__restrict__ h, double sign, double2 *W)
+{
     constexpr int TILE = 64;  // coefficients staged at a time
-    __shared__ T hr[TILE], hi[TILE];
+    __shared__ float2 hs[TILE];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y;
-    T sr = 0, si = 0;
+    float sr = 0, si = 0;
     for (int v0 = 0; v0 < nv; v0 += TILE) {
         const int nt = min(TILE, nv - v0);
         __syncthreads();
         if (threadIdx.x < nt) {
             const double2 c = h[(v0 + threadIdx.x) * nrhs + r];
-            hr[threadIdx.x] = (T)c.x;
-            hi[threadIdx.x] = (T)c.y;
+            hs[threadIdx.x] = make_float2((float)c.x, (float)c.y);
         }
         __syncthreads();
         if (i < n)
 #pragma unroll 4
             for (int v = 0; v < nt; ++v) {
-                const V2 a = V[((int64_t)(v0 + v) * nrhs + r) * n + i];
-                const T ar = (T)a.x, ai = (T)a.y, cr = hr[v], ci = hi[v];
-                sr += ar * cr - ai * ci;
-                si += ar * ci + ai * cr;
+                const float2 a = V[((int64_t)(v0 + v) * nrhs + r) * n + i], c = hs[v];
+                sr += a.x * c.x - a.y * c.y;
+                si += a.x * c.y + a.y * c.x;
             }
     }
     if (i >= n) return;
@@ -231,7 +248,7 @@ cudaError_t launch_bdot(const double2 *V, int nv, const double2 *W, int64_t n, i
                         cudaStream_t s)
 {
     const int blocks = bdot_blocks(n);
-    k_bdot<false><<<dim3(blocks, nrhs, nv), BT, 0, s>>>(V, W, n, nrhs, nv, part);
+    k_bdot<false, 1><<<dim3(blocks, nrhs, nv), BT, 0, s>>>(V, W, n, nrhs, nv, part);
     return bdot_reduce(part, nv * nrhs, blocks, out, s);
 }
 
@@ -239,9 +256,16 @@ cudaError_t launch_bdot32(const double2 *V, const float2 *V32, int nv, const dou
                           double2 *part, double2 *out, cudaStream_t s)
 {
     const int blocks = bdot_blocks(n);
-    const dim3 g(blocks, nrhs, (nv + 3) / 4);
-    if (V32) k_bdot<true><<<g, BT, 0, s>>>(V32, W, n, nrhs, nv, part);
-    else k_bdot<true><<<g, BT, 0, s>>>(V, W, n, nrhs, nv, part);
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // four vectors a block where that still makes two blocks per SM (10 580 unknowns,
+    // seven right-hand sides: a solve 10.28 ms with four, 10.08 with one)
+    const dim3 g4(blocks, nrhs, (nv + 3) / 4), g1(blocks, nrhs, nv);
+    const bool four = (int64_t)blocks * nrhs * g4.z >= 2 * (int64_t)sms;
+    if (V32 && four) k_bdot<true, 4><<<g4, BT, 0, s>>>(V32, W, n, nrhs, nv, part);
+    else if (V32) k_bdot<true, 1><<<g1, BT, 0, s>>>(V32, W, n, nrhs, nv, part);
+    else k_bdot<true, 1><<<g1, BT, 0, s>>>(V, W, n, nrhs, nv, part);
     return bdot_reduce(part, nv * nrhs, blocks, out, s);
 }
 
@@ -256,7 +280,7 @@ cudaError_t launch_bcombo32(const double2 *V, const float2 *V32, int64_t n, int 
                             double sign, double2 *W, cudaStream_t s)
 {
     const dim3 g((unsigned)((n + 255) / 256), nrhs);
-    if (V32) k_bcombo<true><<<g, 256, 0, s>>>(V32, n, nrhs, nv, h, sign, W);
+    if (V32) k_bcombo32<<<g, 256, 0, s>>>(V32, n, nrhs, nv, h, sign, W);
     else k_bcombo<true><<<g, 256, 0, s>>>(V, n, nrhs, nv, h, sign, W);
     return cudaGetLastError();
 }

@@ -46,3 +46,9 @@ def test_with_a_memory_budget(gpu_ctx):
     X, _ = solve(ctx, 700, 3, 0.5)
     Y, _ = solve(gpu_ctx, 700, 3, 0.5)
     assert np.abs(X - Y).max() <= 1e-6 * np.abs(Y).max()
+
+
+@pytest.mark.parametrize("n", [257, 600, 2049])
+def test_with_the_copy(gpu_ctx, n):
+    # n nrhs >= 32768 values keep the FP32 copy
+    solve(gpu_ctx, n, -(-32768 // n), 0.5)
