@@ -55,7 +55,8 @@ __global__ void __launch_bounds__(GS_THREADS) k_gmres_step(GmresStep a)
     }
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *h = reinterpret_cast<double2 *>(smem_raw);  // [m + 2]
-    double2 *part = h + (m + 2);                          // [GS_WARPS][32], then [2 m + 1]
+    double2 *h2 = h + (m + 2);                            // [m + 1]
+    double2 *part = h2 + (m + 1);                         // [GS_WARPS][32], then [2 m + 1]
     double2 *w = part + (size_t)GS_WARPS * 32 + 2 * m + 1;  // the slice
     const int64_t i0 = n * rank / G, i1 = n * (rank + 1) / G;
     const int rows = (int)(i1 - i0);
@@ -160,11 +161,10 @@ __global__ void __launch_bounds__(GS_THREADS) k_gmres_step(GmresStep a)
         return;
     }
 
-    // CGS2: h += V^H w, w -= V h, twice
-    double2 *hk = h;
-    double2 acc = make_double2(0.0, 0.0);  // thread v's sum of both projections
+    // CGS2: h = V^H w, w -= V h, twice (the second time h2)
     for (int pass = 0; pass < 2; ++pass) {
-        reduce(k + 1, hk, [&](int v) {
+        double2 *hp = pass ? h2 : h;
+        reduce(k + 1, hp, [&](int v) {
             const double2 *Vv = V + (int64_t)v * n + i0;
             double sr = 0.0, si = 0.0;
             for (int i = lane; i < rows; i += 32) {
@@ -174,16 +174,12 @@ __global__ void __launch_bounds__(GS_THREADS) k_gmres_step(GmresStep a)
             }
             return make_double2(warp_sum(sr), warp_sum(si));
         });
-        if (tid <= k) {
-            acc.x += hk[tid].x;
-            acc.y += hk[tid].y;
-        }
         for (int i = tid; i < rows; i += GS_THREADS) {
             double2 x = w[i];
             const double2 *Vi = V + i0 + i;
 #pragma unroll 4
             for (int v = 0; v <= k; ++v) {
-                const double2 q = cmul2(__ldcg(Vi + (int64_t)v * n), hk[v]);
+                const double2 q = cmul2(__ldcg(Vi + (int64_t)v * n), hp[v]);
                 x.x -= q.x;
                 x.y -= q.y;
             }
@@ -197,9 +193,12 @@ __global__ void __launch_bounds__(GS_THREADS) k_gmres_step(GmresStep a)
         double2 *Vn = V + (int64_t)(k + 1) * n + i0;
         for (int i = tid; i < rows; i += GS_THREADS) Vn[i] = make_double2(w[i].x * s, w[i].y * s);
     }
-    if (tid <= k) h[tid] = acc;
+    if (rank != 0) return;
+    // the column of H is the sum of both projections; a cycle may have more
+    // steps than the block threads
+    for (int v = tid; v <= k; v += GS_THREADS) h[v] = make_double2(h[v].x + h2[v].x, h[v].y + h2[v].y);
     __syncthreads();
-    if (rank == 0 && tid == 0) {
+    if (tid == 0) {
         // the previous rotations, then a new one zeroing the subdiagonal
         double2 *Hk = H + (size_t)k * (m + 1);
         h[k + 1] = make_double2(hn, 0.0);
@@ -282,7 +281,7 @@ cudaError_t gmres_step_plan(int64_t n, int restart, int device, GmresPlan *plan)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gmres_step, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e != cudaSuccess) return e;
     plan->ctas = (int)std::max<int64_t>(1, std::min<int64_t>((n + GS_ROWS - 1) / GS_ROWS, sms));
-    plan->smem = sizeof(double2) * ((size_t)restart + 2 + GS_WARPS * 32 + 2 * (size_t)restart + 1 +
+    plan->smem = sizeof(double2) * (2 * (size_t)restart + 3 + GS_WARPS * 32 + 2 * (size_t)restart + 1 +
                                     (size_t)((n + plan->ctas - 1) / plan->ctas));
     if (plan->smem > (size_t)optin) return cudaErrorInvalidValue;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_step, GS_THREADS, plan->smem);

@@ -1,0 +1,45 @@
+"""A GMRES cycle of more steps than the step kernel has threads (256), through
+the composite solve, whose restart has no bound of its own below 2048.
+
+The mesh is 600 large triangles thrown into the unit cube: every one is near
+most others, the matrix DLP - I/2 has no clustered spectrum (condition number
+1.1e4) and needs about 410 steps at 1e-8.
+
+Tolerance: the stopping rule bounds the residual by 1e-8 of the right-hand
+side, up to the loss of orthogonality of the FP64 basis (CGS2: a few eps), and
+the matrices the solve assembles are the ones compared with: 2e-8.  The solution
+is then within the condition number times that, 2.2e-4.
+"""
+import numpy as np
+import pytest
+
+import nihu_gb300 as g
+from nihu_gb300 import meshes
+
+pytestmark = pytest.mark.gpu
+
+
+def soup(n, seed=0):
+    rng = np.random.default_rng(seed)
+    centre = rng.random((n, 1, 3))
+    nodes = (centre + rng.random((n, 3, 3)) - 0.5).reshape(-1, 3)
+    return meshes._pack(nodes, np.arange(3 * n).reshape(n, 3), meshes.TRIA_1)
+
+
+@pytest.mark.parametrize("restart", [500, 600])
+def test_more_than_256_steps(gpu_ctx, restart):
+    mesh, k = soup(600), 2.0
+    n = len(mesh[1])
+    S, D = (np.zeros((n, n), complex, order="F") for _ in range(2))
+    dm = g.api.DeviceMesh(gpu_ctx, *mesh)
+    gpu_ctx.check(g.lib().nihu_gb_assemble(gpu_ctx.handle, dm.handle, dm.handle, g.HELMHOLTZ_3D, g.SLP | g.DLP, k, 1.0, 0.0,
+                                           g.REGULAR_FP64, g.C128, S.ctypes.data, D.ctypes.data, n, 0, g.HOST))
+    rng = np.random.default_rng(1)
+    q = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    A, b = D - 0.5 * np.eye(n), S @ q
+    p, it, res = g.solve_cbie(g.create_mesh(*mesh), k, q, dtype=g.C128, precision="fp64", restart=restart,
+                              max_iters=restart, tol=1e-8, ctx=gpu_ctx)
+    assert 256 < it <= 500 and res < 1e-8
+    assert np.linalg.norm(A @ p - b) <= 2e-8 * np.linalg.norm(b)
+    ref = np.linalg.solve(A, b)
+    assert np.linalg.norm(p - ref) <= 2.2e-4 * np.linalg.norm(ref)
