@@ -85,6 +85,9 @@ __global__ void __launch_bounds__(T) k_lu32_panel(float2 *__restrict__ F, int n,
     __shared__ int s_dorig[2];
     __shared__ Lu32Moves s_mv;
     cg::cluster_group cl = cg::this_cluster();
+    // every CTA of the cluster has started before its memory is written (waited for
+    // behind the loads)
+    cg::cluster_group::arrival_token started = cl.barrier_arrive();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m = n - j0, row0 = rank * T * R + tid;
@@ -101,6 +104,7 @@ __global__ void __launch_bounds__(T) k_lu32_panel(float2 *__restrict__ F, int n,
         last[q] = -1;
     }
     if (rank == 0 && tid < LU32_NB) s_mv.dst[tid] = -1;
+    cl.barrier_wait(std::move(started));
     // one body for all columns (unrolled, every instruction would be fetched for
     // one use): the current column is position 0, a step moves all
     // positions down by one, so that after NB steps they are in place again
@@ -390,6 +394,8 @@ __global__ void __cluster_dims__(LU32_CTAS, 1, 1) __launch_bounds__(LU32_T)
     extern __shared__ float2 part[];  // [8][own rows]
     __shared__ float2 s_y[4][LU32_BLK], s_red[8][LU32_BLK], s_raw[LU32_BLK];
     cg::cluster_group cl = cg::this_cluster();
+    // every CTA has started before its memory is written (waited for behind the gather)
+    cg::cluster_group::arrival_token started = cl.barrier_arrive();
     const int rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = (warp & 1) * 32 + lane, g = warp >> 1;
@@ -405,6 +411,7 @@ __global__ void __cluster_dims__(LU32_CTAS, 1, 1) __launch_bounds__(LU32_T)
         }
         mine[q * LU32_BLK] = v;
     }
+    cl.barrier_wait(std::move(started));
     // eight columns of the tile (row block rb, column block cb)
     auto load_tile = [&](int rb, int cb, float2 t[8]) {
         const int i = rb * LU32_BLK + row;
