@@ -507,9 +507,8 @@ template <int FAM>
 static cudaError_t launch_bm2(const BmArgs &a, cudaStream_t s)
 {
     if (!bm_system(a)) return cudaErrorInvalidValue;
-    int dev = 0, sms = 148;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     static bool carveout_set[64] = {};
     if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
         const cudaError_t e = cudaFuncSetAttribute(k_regular_bm2<FAM>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -517,10 +516,14 @@ static cudaError_t launch_bm2(const BmArgs &a, cudaStream_t s)
         if (e != cudaSuccess) return e;
         carveout_set[dev] = true;
     }
-    const int cpb = two_row_cols(a.test.n, a.j1 - a.j0, sms);
-    const dim3 grid((a.test.n + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS, (a.j1 - a.j0 + cpb - 1) / cpb);
-    k_regular_bm2<FAM><<<grid, TWO_ROW_THREADS, 0, s>>>(a, cpb);
-    return cudaGetLastError();
+    return two_row_launches(a.test.n, a.j0, a.j1, [&](int j0, int j1, dim3 grid, int cols) {
+        BmArgs b = a;
+        b.j0 = j0;
+        b.j1 = j1;
+        b.out_a = reinterpret_cast<float2 *>(a.out_a) + (int64_t)(j0 - a.j0) * a.ld;
+        b.out_b = reinterpret_cast<float2 *>(a.out_b) + (int64_t)(j0 - a.j0) * a.ld;
+        k_regular_bm2<FAM><<<grid, TWO_ROW_THREADS, 0, s>>>(b, cols);
+    });
 }
 
 template <typename R, typename Out, int FAM>

@@ -757,16 +757,17 @@ __global__ void __launch_bounds__(TWO_ROW_THREADS, 20 / TWO_ROW_WARPS) k_galerki
 template <int FAM>
 static cudaError_t launch_galerkin_regular2(const GalArgs &a, cudaStream_t s)
 {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int cpb = two_row_cols(a.test.n, a.j1 - a.j0, sms);
-    const dim3 grid((a.test.n + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS, (a.j1 - a.j0 + cpb - 1) / cpb);
     const auto kernel = a.ops == OP_SLP   ? k_galerkin_regular2<FAM, OP_SLP>
                         : a.ops == OP_DLP ? k_galerkin_regular2<FAM, OP_DLP>
                                           : k_galerkin_regular2<FAM, OP_SLP | OP_DLP>;
-    kernel<<<grid, TWO_ROW_THREADS, 0, s>>>(a, cpb);
-    return cudaGetLastError();
+    return two_row_launches(a.test.n, a.j0, a.j1, [&](int j0, int j1, dim3 grid, int cols) {
+        GalArgs b = a;
+        b.j0 = j0;
+        b.j1 = j1;
+        b.out_s = reinterpret_cast<float2 *>(a.out_s) + (int64_t)(j0 - a.j0) * a.ld;
+        b.out_d = reinterpret_cast<float2 *>(a.out_d) + (int64_t)(j0 - a.j0) * a.ld;
+        kernel<<<grid, TWO_ROW_THREADS, 0, s>>>(b, cols);
+    });
 }
 
 // ------------------------------------------------- near pairs, FP32 triangles

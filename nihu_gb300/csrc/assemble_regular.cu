@@ -727,9 +727,8 @@ __global__ void __launch_bounds__(TWO_ROW_THREADS, 32 / TWO_ROW_WARPS) k_regular
 template <int FAM, int OPS, bool CK, bool PLAIN>
 static cudaError_t launch_regular2(const RegularArgs &a, cudaStream_t s)
 {
-    int dev = 0, sms = 148;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     static bool carveout_set[64] = {};
     if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
         const cudaError_t e = cudaFuncSetAttribute(k_regular2<FAM, OPS, CK, PLAIN>,
@@ -738,10 +737,14 @@ static cudaError_t launch_regular2(const RegularArgs &a, cudaStream_t s)
         if (e != cudaSuccess) return e;
         carveout_set[dev] = true;
     }
-    const int cpb = two_row_cols(a.test.n, a.j1 - a.j0, sms);
-    const dim3 grid((a.test.n + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS, (a.j1 - a.j0 + cpb - 1) / cpb);
-    k_regular2<FAM, OPS, CK, PLAIN><<<grid, TWO_ROW_THREADS, 0, s>>>(a, cpb);
-    return cudaGetLastError();
+    return two_row_launches(a.test.n, a.j0, a.j1, [&](int j0, int j1, dim3 grid, int cols) {
+        RegularArgs b = a;
+        b.j0 = j0;
+        b.j1 = j1;
+        b.out_s = reinterpret_cast<float2 *>(a.out_s) + (int64_t)(j0 - a.j0) * a.ld;
+        b.out_d = reinterpret_cast<float2 *>(a.out_d) + (int64_t)(j0 - a.j0) * a.ld;
+        k_regular2<FAM, OPS, CK, PLAIN><<<grid, TWO_ROW_THREADS, 0, s>>>(b, cols);
+    });
 }
 
 template <int FAM, bool CK, bool PLAIN>

@@ -97,6 +97,26 @@ inline int two_row_cols(int n_rows, int n_cols, int sms)
     return (int)(c < 1 ? 1 : (c > TWO_ROW_COLS ? TWO_ROW_COLS : c));
 }
 
+// the launches that cover columns [j0, j1), launch(first column, end, grid, columns
+// per block) each: one, or beyond a million columns (a few field points of a
+// very large mesh) as many as grid.y, 65 535 column blocks, asks for
+template <class F>
+inline cudaError_t two_row_launches(int n_rows, int j0, int j1, F &&launch)
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int cols = two_row_cols(n_rows, j1 - j0, sms);
+    const unsigned rows = (unsigned)((n_rows + TWO_ROW_ROWS - 1) / TWO_ROW_ROWS);
+    for (int64_t j = j0; j < j1; j += 65535 * (int64_t)cols) {
+        const int end = (int)(j1 - j < 65535 * (int64_t)cols ? j1 : j + 65535 * (int64_t)cols);
+        launch((int)j, end, dim3(rows, (unsigned)((end - j + cols - 1) / cols)), cols);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 template <bool FULL, class K>
 __device__ __forceinline__ void two_row_columns(const K &op, TwoRowShared &sh, const DevMesh &test, int ib, int ncols)
 {
