@@ -1,6 +1,7 @@
 // C ABI of the GB300 collocation BEM library (declared in include/nihu_gb300.h).
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -38,6 +39,8 @@ struct nihu_gb_ctx {
     int64_t launches = 0;
     int *d_flag = nullptr;       // device error flag / small scratch (4 ints)
     void *h_small = nullptr;     // pinned host scratch (64 KB)
+    void *h_big = nullptr;       // pinned host scratch of h_big_bytes (host_scratch)
+    size_t h_big_bytes = 0;
     uint64_t next_uid = 1;
     // nearly singular pair lists keyed by (test uid, trial uid)
     std::map<std::pair<uint64_t, uint64_t>, NearList> near;
@@ -55,7 +58,7 @@ struct nihu_gb_ctx {
     cudaGraphExec_t lu_exec = nullptr;
     int lu_n = 0;
     int64_t lu_launches = 0;
-    void *lu_F = nullptr, *lu_aux = nullptr;
+    void *lu_F = nullptr, *lu_perm = nullptr, *lu_work = nullptr;
 };
 
 struct nihu_gb_mesh {
@@ -129,6 +132,25 @@ nihu_gb_status scratch(nihu_gb_ctx *ctx, const char *name, size_t bytes, void **
     nihu_gb_status st = dmalloc(ctx, bytes, out);
     if (st != NIHU_GB_OK) return st;
     ctx->scratch[name] = {*out, bytes};
+    return NIHU_GB_OK;
+}
+
+// pinned host scratch of at least `bytes`, which kernels may address; the
+// previous one is freed (call it with no kernel in flight that uses that)
+nihu_gb_status host_scratch(nihu_gb_ctx *ctx, size_t bytes, void **out)
+{
+    if (ctx->h_big_bytes < bytes) {
+        if (ctx->h_big) cudaFreeHost(ctx->h_big);
+        ctx->h_big = nullptr;
+        ctx->h_big_bytes = 0;
+        const cudaError_t e = cudaMallocHost(&ctx->h_big, bytes);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return cuda_fail(ctx, e, "pinned host memory");
+        }
+        ctx->h_big_bytes = bytes;
+    }
+    *out = ctx->h_big;
     return NIHU_GB_OK;
 }
 
@@ -310,6 +332,14 @@ cudaError_t timed_gemv(nihu_gb_ctx *ctx, int dtype, const void *A, int64_t m, in
     return launch_gemv(dtype, A, m, n, lda, x, y, are, aim, bre, bim, partial, splits, ctx->stream);
 }
 
+// column splits of a matvec; under a memory budget of 256 columns at least, so that
+// its partial sums stay below a hundredth of the matrix
+int matvec_splits(const nihu_gb_ctx *ctx, int64_t m, int64_t n, int dtype)
+{
+    const int splits = gemv_splits(m, n, dtype);
+    return ctx->budget ? (int)std::min<int64_t>(splits, std::max<int64_t>(1, n / 256)) : splits;
+}
+
 bool valid_dtype(int d) { return d == NIHU_GB_C64 || d == NIHU_GB_C128; }
 bool valid_where(int w) { return w == NIHU_GB_HOST || w == NIHU_GB_DEVICE; }
 
@@ -477,6 +507,7 @@ void nihu_gb_ctx_destroy(nihu_gb_ctx *ctx)
     for (auto &kv : ctx->scratch) dfree(ctx, kv.second.first);
     dfree(ctx, ctx->d_flag);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
+    if (ctx->h_big) cudaFreeHost(ctx->h_big);
     if (ctx->cublas) cublasDestroy(ctx->cublas);
     if (ctx->lu_exec) cudaGraphExecDestroy(ctx->lu_exec);
     collect_phases(ctx);
@@ -1270,7 +1301,7 @@ nihu_gb_status nihu_gb_matvec(nihu_gb_ctx *ctx, int dtype_a, const void *A, int6
         dy = (double2 *)py;
         lda = m;
     }
-    int splits = gemv_splits(m, n, dtype_a);
+    int splits = matvec_splits(ctx, m, n, dtype_a);
     void *part;
     if ((st = scratch(ctx, "mv_part", 16 * (size_t)splits * m, &part))) return st;
     CK(timed_gemv(ctx, dtype_a, dA, m, n, lda, dx, dy, alpha_re, alpha_im, beta_re, beta_im, (double2 *)part, splits));
@@ -1293,15 +1324,37 @@ nihu_gb_status gmres_device(nihu_gb_ctx *ctx, int dtype_a, const void *A, int64_
     // the bound of restart times vector blocks that this solver has always had
     if ((m + 1) * std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, 64)) > 4096)
         return fail(ctx, NIHU_GB_ERR_INVALID_ARGUMENT, "GMRES restart too large");
-    const int splits = gemv_splits(n, n, dtype_a);
+    const int splits = matvec_splits(ctx, n, n, dtype_a);
     GmresPlan plan;
-    CK(gmres_step_plan(n, m, ctx->device, &plan));
-    void *pV, *ppart, *psmall, *pstate, *psums;
+    CK(gmres_step_plan(n, m, ctx->device, INT_MAX, &plan));
+    void *pV, *ppart, *pwork, *psmall;
+    size_t small = 16 * gmres_small_entries(m), work = 64 + 32 * (size_t)(m + 1) * plan.ctas + small;
+    bool small_on_host = false;
+    if (ctx->budget) {
+        // what two vectors and the projections of every 1024 rows take: fewer thread
+        // blocks, and H with the rotations in host memory where half the blocks are not
+        // left beside them
+        const size_t dots = (size_t)std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, 64));
+        const size_t room = 32 * (size_t)n + 16 * (dots + 1) * (m + 1), least = 64 + 32 * (size_t)(m + 1);
+        if (work > room) {
+            auto blocks = [&](size_t used) {
+                return room < used + least ? 1 : (int)std::min<size_t>(plan.ctas, (room - used - 64) / (32 * (size_t)(m + 1)));
+            };
+            small_on_host = room < small + least || 2 * blocks(small) < plan.ctas;
+            if (small_on_host) small = 0;
+            CK(gmres_step_plan(n, m, ctx->device, blocks(small), &plan));
+            work = 64 + 32 * (size_t)(m + 1) * plan.ctas + small;
+        }
+    }
     if ((st = scratch(ctx, "gm_V", 16 * (size_t)n * (m + 1), &pV))) return st;
     if ((st = scratch(ctx, "mv_part", 16 * (size_t)splits * n, &ppart))) return st;
-    if ((st = scratch(ctx, "gm_small", 16 * gmres_small_entries(m), &psmall))) return st;
-    if ((st = scratch(ctx, "gm_state", 64, &pstate))) return st;
-    if ((st = scratch(ctx, "gm_sums", 16 * 2 * (size_t)(m + 1) * plan.ctas, &psums))) return st;
+    if ((st = scratch(ctx, "gm_work", work, &pwork))) return st;
+    void *pstate = pwork, *psums = (char *)pwork + 64;
+    if (small_on_host) {
+        if ((st = host_scratch(ctx, 16 * gmres_small_entries(m), &psmall))) return st;
+    } else {
+        psmall = (char *)pwork + work - small;
+    }
     GmresHost *hs = (GmresHost *)ctx->h_small;  // pinned, mapped
     hs->seq = 0;
     hs->flag = GMRES_GO;
@@ -1430,8 +1483,8 @@ namespace {
 // correction is within 64 FP64 roundings of x (|d| <= 64 eps |x|, the
 // accuracy of an FP64 factorisation).  *refined = false (and nothing solved)
 // when the order is beyond the FP32 kernels' shared memory and registers or the
-// corrections stop shrinking (cond(A) near 1 / eps32), or a memory budget has no
-// room for the inverses: the caller then factorises in FP64.  A is left unchanged.
+// corrections stop shrinking (cond(A) near 1 / eps32), or there is no memory for
+// the factors: the caller then factorises in FP64.  A is left unchanged.
 nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int64_t lda, const double2 *b, double2 *x,
                               bool *refined)
 {
@@ -1440,32 +1493,29 @@ nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
     if (!lu32_fits((int)n, (size_t)smem_optin)) return NIHU_GB_OK;
     nihu_gb_status st;
-    void *pf, *paux, *pd, *pr, *psums, *ppart;
-    const int splits = gemv_splits(n, n, NIHU_GB_C128);
-    if ((st = scratch(ctx, "lu32_F", 8 * (size_t)n * n, &pf))) return st;
-    {
-        // the diagonal blocks' inverses are 1 KB a row: where a memory budget has no room
-        // for them the caller's FP64 factorisation, which needs none, still runs
-        const std::string msg = ctx->err;
-        if (scratch(ctx, "lu32_aux", lu32_aux_bytes((int)n), &paux)) {
-            ctx->err = msg;
-            return NIHU_GB_OK;
-        }
+    void *pf, *pperm, *pd, *pr, *psums, *ppart;
+    const int splits = matvec_splits(ctx, n, n, NIHU_GB_C128);
+    if ((st = scratch(ctx, "lu_piv", sizeof(int) * n, &pperm))) return st;
+    const std::string msg = ctx->err;
+    // the factorisation's scratch is d, which the solves write
+    if (scratch(ctx, "lu32_F", 8 * (size_t)n * n, &pf) ||
+        scratch(ctx, "lu32_d", std::max<size_t>(16 * (size_t)n, LU32_WORK_BYTES), &pd) ||
+        scratch(ctx, "lu32_r", 16 * (size_t)n, &pr) || scratch(ctx, "lu32_sums", 2 * sizeof(double), &psums) ||
+        scratch(ctx, "lu32_part", 16 * (size_t)splits * n, &ppart)) {
+        ctx->err = msg;
+        return NIHU_GB_OK;
     }
-    if ((st = scratch(ctx, "lu32_d", 16 * (size_t)n, &pd))) return st;
-    if ((st = scratch(ctx, "lu32_r", 16 * (size_t)n, &pr))) return st;
-    if ((st = scratch(ctx, "lu32_sums", 2 * sizeof(double), &psums))) return st;
-    if ((st = scratch(ctx, "lu32_part", 16 * (size_t)splits * n, &ppart))) return st;
     double2 *d = (double2 *)pd, *r = (double2 *)pr;
     CK(lu32_prepare((int)n, (size_t)smem_optin));
-    if (!(ctx->lu_exec && ctx->lu_n == n && ctx->lu_F == pf && ctx->lu_aux == paux)) {
+    if (!(ctx->lu_exec && ctx->lu_n == n && ctx->lu_F == pf && ctx->lu_perm == pperm && ctx->lu_work == pd)) {
         // record the panel sequence once per order and buffers
         if (ctx->lu_exec) cudaGraphExecDestroy(ctx->lu_exec);
         ctx->lu_exec = nullptr;
         cudaGraph_t graph = nullptr;
         int64_t counted = 0;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = launch_lu32_factor((float2 *)pf, (int)n, paux, ctx->d_flag + 1, &counted, ctx->stream);
+        cudaError_t e = launch_lu32_factor((float2 *)pf, (int)n, (int *)pperm, pd, ctx->d_flag + 1, &counted,
+                                           ctx->stream);
         cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
         if (e == cudaSuccess) e = e2;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&ctx->lu_exec, graph, 0);
@@ -1476,13 +1526,14 @@ nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int
         }
         ctx->lu_n = (int)n;
         ctx->lu_F = pf;
-        ctx->lu_aux = paux;
+        ctx->lu_perm = pperm;
+        ctx->lu_work = pd;
         ctx->lu_launches = counted;
     }
     CK(cudaMemsetAsync(ctx->d_flag + 1, 0, sizeof(int), ctx->stream));
     {
         Phase ph(ctx, "lu_factor");
-        CK(launch_to_c64(A, lda, (int)n, (float2 *)pf, paux, ctx->stream));
+        CK(launch_to_c64(A, lda, (int)n, (float2 *)pf, (int *)pperm, ctx->stream));
         CK(cudaGraphLaunch(ctx->lu_exec, ctx->stream));
         ctx->launches += 1 + ctx->lu_launches;
     }
@@ -1496,7 +1547,7 @@ nihu_gb_status lu_solve_mixed(nihu_gb_ctx *ctx, const double2 *A, int64_t n, int
     double sums[2] = {0.0, 0.0}, prev = 0.0;
     const double eps = 2.220446049250313e-16;
     for (int it = 0; it < 12; ++it) {
-        CK(launch_lu32_solve((const float2 *)pf, (int)n, paux, r, d, ctx->stream));
+        CK(launch_lu32_solve((const float2 *)pf, (int)n, (const int *)pperm, r, d, ctx->stream));
         CK(launch_lu32_update_x(x, d, (int)n, (double *)psums, ctx->stream));
         CK(cudaMemcpyAsync(r, b, 16 * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
         CK(launch_gemv(NIHU_GB_C128, A, n, n, lda, x, r, -1.0, 0.0, 1.0, 0.0, (double2 *)ppart, splits, ctx->stream));
@@ -1579,7 +1630,7 @@ nihu_gb_status solve_tail(nihu_gb_ctx *ctx, int64_t n, int dtype, void *G, void 
                           void *p, int solver, int restart, int max_iters, double tol, int *iters, double *rel_residual)
 {
     nihu_gb_status st;
-    int splits = gemv_splits(n, n, dtype);
+    int splits = matvec_splits(ctx, n, n, dtype);
     void *part;
     if ((st = scratch(ctx, "mv_part", 16 * (size_t)splits * n, &part))) return st;
     CK(timed_gemv(ctx, dtype, G, n, n, n, (const double2 *)dq, (double2 *)drhs, 1.0, 0.0, 0.0, 0.0, (double2 *)part, splits));

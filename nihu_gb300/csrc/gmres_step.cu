@@ -273,14 +273,14 @@ __global__ void __launch_bounds__(256) k_gmres_update(GmresStep a, double2 *x)
 
 }  // namespace
 
-cudaError_t gmres_step_plan(int64_t n, int restart, int device, GmresPlan *plan)
+cudaError_t gmres_step_plan(int64_t n, int restart, int device, int max_ctas, GmresPlan *plan)
 {
     int optin = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gmres_step, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e != cudaSuccess) return e;
-    plan->ctas = (int)std::max<int64_t>(1, std::min<int64_t>((n + GS_ROWS - 1) / GS_ROWS, sms));
+    plan->ctas = (int)std::max<int64_t>(1, std::min<int64_t>((n + GS_ROWS - 1) / GS_ROWS, std::min(sms, max_ctas)));
     plan->smem = sizeof(double2) * (2 * (size_t)restart + 3 + GS_WARPS * 32 + 2 * (size_t)restart + 1 +
                                     (size_t)((n + plan->ctas - 1) / plan->ctas));
     if (plan->smem > (size_t)optin) return cudaErrorInvalidValue;

@@ -59,7 +59,8 @@ struct GmresPlan {
     size_t smem = 0;
 };
 inline size_t gmres_small_entries(int m) { return (size_t)(m + 1) * m + 2 * m + (m + 1); }
-cudaError_t gmres_step_plan(int64_t n, int restart, int device, GmresPlan *plan);
+// max_ctas: no more thread blocks than that (their partial sums are 32 (restart + 1) B each)
+cudaError_t gmres_step_plan(int64_t n, int restart, int device, int max_ctas, GmresPlan *plan);
 cudaError_t launch_gmres_step(const GmresStep &a, const GmresPlan &plan, cudaStream_t s);
 // x += V H^{-1} g over the steps done
 cudaError_t launch_gmres_update(const GmresStep &a, double2 *x, cudaStream_t s);
@@ -68,19 +69,19 @@ cudaError_t launch_lu_factor(double2 *A, int64_t n, int64_t lda, int *piv, int *
                              cudaStream_t s);
 // lu32.cu: mixed-precision LU (FP32 factors of the FP64 matrix, refined by the
 // caller): whether order n fits the kernels (smem_max: the device's per-block
-// opt-in limit), and the bytes of its auxiliary buffer (the row order, the
-// diagonal blocks' inverses)
+// opt-in limit)
 bool lu32_fits(int n, size_t smem_max);
-size_t lu32_aux_bytes(int n);
 // kernel attributes for order n (outside any stream capture)
 cudaError_t lu32_prepare(int n, size_t smem_max);
-// F (n x n complex64, leading dimension n) = A rounded to complex64, and aux for its factorisation
-cudaError_t launch_to_c64(const double2 *A, int64_t lda, int n, float2 *F, void *aux, cudaStream_t s);
-// F in place = its FP32 LU factors with partial pivoting (info = 1 + first
-// zero pivot column); stream-capturable
-cudaError_t launch_lu32_factor(float2 *F, int n, void *aux, int *info, int64_t *launches, cudaStream_t s);
+// F (n x n complex64, leading dimension n) = A rounded to complex64, perm [n] = identity
+cudaError_t launch_to_c64(const double2 *A, int64_t lda, int n, float2 *F, int *perm, cudaStream_t s);
+// F in place = its FP32 LU factors with partial pivoting (perm: the row order; info =
+// 1 + first zero pivot column), the diagonal blocks of 64 inverted; work: scratch of
+// LU32_WORK_BYTES; stream-capturable
+constexpr size_t LU32_WORK_BYTES = 192;
+cudaError_t launch_lu32_factor(float2 *F, int n, int *perm, void *work, int *info, int64_t *launches, cudaStream_t s);
 // d = (P^T L U)^{-1} r with the FP32 factors
-cudaError_t launch_lu32_solve(const float2 *F, int n, void *aux, const double2 *r, double2 *d, cudaStream_t s);
+cudaError_t launch_lu32_solve(const float2 *F, int n, const int *perm, const double2 *r, double2 *d, cudaStream_t s);
 // x += d; sums[0] = |d|^2, sums[1] = |x|^2
 cudaError_t launch_lu32_update_x(double2 *x, const double2 *d, int n, double *sums, cudaStream_t s);
 cudaError_t launch_lu_solve(const double2 *A, int64_t n, int64_t lda, const int *piv, const double2 *b, double2 *x,

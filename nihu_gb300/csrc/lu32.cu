@@ -7,8 +7,8 @@
 //   k_lu32_panel   the panel with its rows in registers (one cluster)
 //   k_lu32_trail   its row exchanges on all other columns, the panel's rows of
 //                  U (unit-lower triangular solve), the trailing matrix's update
-// and k_lu32_diag, the inverses of the factors' 64 x 64 diagonal blocks, with
-// which k_lu32_solve's block steps are products.
+// and k_lu32_diag, which puts the inverses of the factors' 64 x 64 diagonal blocks in
+// their place, so that k_lu32_solve's block steps are products.
 //
 // Order 1280: the factorisation 4.36 -> 2.31 ms, one solve 650 -> 72 us.
 #include <cooperative_groups.h>
@@ -33,6 +33,7 @@ constexpr int LU32_LEFT = 8;    // columns left of a panel to a warp
 struct Lu32Moves {
     int src[LU32_NB], dst[LU32_NB], from[LU32_NB];
 };
+static_assert(sizeof(Lu32Moves) <= LU32_WORK_BYTES, "the factorisation's scratch");
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b)
 {
@@ -336,20 +337,23 @@ __global__ void __launch_bounds__(W * 2 * LU32_NB, W == 8 ? 2 : 1) k_lu32_trail(
     }
 }
 
-// inv + (2 b + upper) 64^2, column-major: the inverse of diagonal block b of L
-// (blockIdx.y 0) or U (1), eight lanes a column; the last block is filled up with
-// the identity
+// The factors' 64 x 64 diagonal blocks replaced by the inverses of their L
+// (blockIdx.y 0, strictly below the diagonal, where the unit one is not stored) and
+// U (1, the rest), eight lanes a column; the last block is filled up with the
+// identity.  Each thread block reads only the triangle that it writes.
 constexpr size_t LU32_DIAG_SMEM = 2 * sizeof(float2) * LU32_BLK * (LU32_BLK + 1);
-__global__ void __launch_bounds__(8 * LU32_BLK) k_lu32_diag(const float2 *__restrict__ F, int n, float2 *__restrict__ inv)
+__global__ void __launch_bounds__(8 * LU32_BLK) k_lu32_diag(float2 *__restrict__ F, int n)
 {
     extern __shared__ float2 sm[];
     float2(*D)[LU32_BLK + 1] = reinterpret_cast<float2(*)[LU32_BLK + 1]>(sm);  // D[row][column]
     float2(*X)[LU32_BLK + 1] = reinterpret_cast<float2(*)[LU32_BLK + 1]>(sm + LU32_BLK * (LU32_BLK + 1));  // X[column][row]
     const int b0 = blockIdx.x * LU32_BLK, j = threadIdx.x >> 3, h = threadIdx.x & 7;
     const bool upper = blockIdx.y;
+    float2 *G = F + (int64_t)b0 * n + b0;
     for (int t = threadIdx.x; t < LU32_BLK * LU32_BLK; t += 8 * LU32_BLK) {
         const int r = t % LU32_BLK, c = t / LU32_BLK;
-        D[r][c] = b0 + c < n && b0 + r < n ? F[(int64_t)(b0 + c) * n + b0 + r] : make_float2(c == r ? 1.0f : 0.0f, 0.0f);
+        const bool own = b0 + c < n && b0 + r < n && (upper ? r <= c : r > c);
+        D[r][c] = own ? G[(int64_t)c * n + r] : make_float2(c == r ? 1.0f : 0.0f, 0.0f);
         X[c][r] = make_float2(0.0f, 0.0f);
     }
     __syncthreads();
@@ -371,9 +375,11 @@ __global__ void __launch_bounds__(8 * LU32_BLK) k_lu32_diag(const float2 *__rest
         if (h == 0) X[j][r] = v;
         __syncwarp();
     }
-    float2 *out = inv + (2 * (int64_t)blockIdx.x + upper) * LU32_BLK * LU32_BLK;
     __syncthreads();
-    for (int t = threadIdx.x; t < LU32_BLK * LU32_BLK; t += 8 * LU32_BLK) out[t] = X[t / LU32_BLK][t % LU32_BLK];
+    for (int t = threadIdx.x; t < LU32_BLK * LU32_BLK; t += 8 * LU32_BLK) {
+        const int r = t % LU32_BLK, c = t / LU32_BLK;
+        if (b0 + c < n && b0 + r < n && (upper ? r <= c : r > c)) G[(int64_t)c * n + r] = X[c][r];
+    }
 }
 
 // d = U^{-1} L^{-1} P r on one cluster.  The rows' blocks of 64 go round the
@@ -388,8 +394,8 @@ __global__ void __launch_bounds__(8 * LU32_BLK) k_lu32_diag(const float2 *__rest
 // other CTAs per block; one CTA, whose thread 0 also ran through the pivots,
 // read the factors at 0.1 TB/s (order 1280: 650 us, here 72; without tiles loaded ahead 115).
 __global__ void __cluster_dims__(LU32_CTAS, 1, 1) __launch_bounds__(LU32_T)
-    k_lu32_solve(const float2 *__restrict__ F, int n, const int *__restrict__ perm, const float2 *__restrict__ inv,
-                 const double2 *__restrict__ r, double2 *__restrict__ d)
+    k_lu32_solve(const float2 *__restrict__ F, int n, const int *__restrict__ perm, const double2 *__restrict__ r,
+                 double2 *__restrict__ d)
 {
     extern __shared__ float2 part[];  // [8][own rows]
     __shared__ float2 s_y[4][LU32_BLK], s_red[8][LU32_BLK], s_raw[LU32_BLK];
@@ -420,10 +426,14 @@ __global__ void __cluster_dims__(LU32_CTAS, 1, 1) __launch_bounds__(LU32_T)
         for (int c = 0; c < 8; ++c)
             t[c] = i < n && j + c < n ? __ldg(F + (int64_t)(j + c) * n + i) : make_float2(0.0f, 0.0f);
     };
+    // the same of the diagonal block's inverse, of U's or of the unit-lower L's
     auto load_inv = [&](int b, int upper, float2 t[8]) {
-        const float2 *p = inv + (2 * (int64_t)b + upper) * LU32_BLK * LU32_BLK + g * 8 * LU32_BLK + row;
+        load_tile(b, b, t);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) t[c] = __ldg(p + c * LU32_BLK);
+        for (int c = 0; c < 8; ++c) {
+            const int j = g * 8 + c;
+            if (upper ? row > j : row <= j) t[c] = make_float2(!upper && row == j ? 1.0f : 0.0f, 0.0f);
+        }
     };
     auto take_off = [&](float2 &v, const float2 t[8], const float2 *y) {
 #pragma unroll
@@ -554,16 +564,6 @@ static size_t lu32_solve_smem(int n)
     return 8 * sizeof(float2) * LU32_BLK * (size_t)((lu32_blocks(n) + LU32_CTAS - 1) / LU32_CTAS);
 }
 
-size_t lu32_aux_bytes(int n)
-{
-    return sizeof(float2) * 2 * LU32_BLK * LU32_BLK * (size_t)lu32_blocks(n) + sizeof(int) * (size_t)n + sizeof(Lu32Moves);
-}
-
-// the auxiliary buffer's parts
-static float2 *lu32_inv(void *aux) { return (float2 *)aux; }
-static int *lu32_perm(void *aux, int n) { return (int *)(lu32_inv(aux) + 2 * (size_t)LU32_BLK * LU32_BLK * lu32_blocks(n)); }
-static Lu32Moves *lu32_moves(void *aux, int n) { return (Lu32Moves *)(lu32_perm(aux, n) + n); }
-
 bool lu32_fits(int n, size_t smem_max)
 {
     if (n < 1 || n > LU32_T * 8 * LU32_CTAS) return false;  // the panel's registers (4 columns, 8 rows a thread)
@@ -584,9 +584,9 @@ cudaError_t lu32_prepare(int n, size_t smem_max)
     return e;
 }
 
-cudaError_t launch_to_c64(const double2 *A, int64_t lda, int n, float2 *F, void *aux, cudaStream_t s)
+cudaError_t launch_to_c64(const double2 *A, int64_t lda, int n, float2 *F, int *perm, cudaStream_t s)
 {
-    k_to_c64<<<dim3((n + 255) / 256, n), 256, 0, s>>>(A, lda, n, F, lu32_perm(aux, n));
+    k_to_c64<<<dim3((n + 255) / 256, n), 256, 0, s>>>(A, lda, n, F, perm);
     return cudaGetLastError();
 }
 
@@ -610,16 +610,16 @@ static cudaError_t launch_panel(float2 *F, int n, int j0, int *nb, Lu32Moves *mo
 }
 
 template <int W>
-static void launch_trail(float2 *F, int n, int j0, int nb, void *aux, cudaStream_t s)
+static void launch_trail(float2 *F, int n, int j0, int nb, const Lu32Moves *moves, int *perm, cudaStream_t s)
 {
     const int strips = (n - j0 - nb + W - 1) / W;
     const int left = j0 / (LU32_LEFT * W) + 1;  // blocks for the columns left of the panel and perm
-    k_lu32_trail<W><<<strips + left, W * 2 * LU32_NB, 0, s>>>(F, n, j0, nb, strips, lu32_moves(aux, n), lu32_perm(aux, n));
+    k_lu32_trail<W><<<strips + left, W * 2 * LU32_NB, 0, s>>>(F, n, j0, nb, strips, moves, perm);
 }
 
-cudaError_t launch_lu32_factor(float2 *F, int n, void *aux, int *info, int64_t *launches, cudaStream_t s)
+cudaError_t launch_lu32_factor(float2 *F, int n, int *perm, void *work, int *info, int64_t *launches, cudaStream_t s)
 {
-    Lu32Moves *moves = lu32_moves(aux, n);
+    Lu32Moves *moves = (Lu32Moves *)work;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -635,18 +635,18 @@ cudaError_t launch_lu32_factor(float2 *F, int n, void *aux, int *info, int64_t *
         else if (m <= 512 * 4 * LU32_CTAS) e = launch_panel<8, 4, 512>(F, n, j0, &nb, moves, info, s);
         else e = launch_panel<4, 8, 512>(F, n, j0, &nb, moves, info, s);
         if (e != cudaSuccess) return e;
-        if (m - nb <= 16 * sms) launch_trail<8>(F, n, j0, nb, aux, s);
-        else launch_trail<16>(F, n, j0, nb, aux, s);
+        if (m - nb <= 16 * sms) launch_trail<8>(F, n, j0, nb, moves, perm, s);
+        else launch_trail<16>(F, n, j0, nb, moves, perm, s);
         *launches += 2;
     }
-    k_lu32_diag<<<dim3(lu32_blocks(n), 2), 8 * LU32_BLK, LU32_DIAG_SMEM, s>>>(F, n, lu32_inv(aux));
+    k_lu32_diag<<<dim3(lu32_blocks(n), 2), 8 * LU32_BLK, LU32_DIAG_SMEM, s>>>(F, n);
     *launches += 1;
     return cudaGetLastError();
 }
 
-cudaError_t launch_lu32_solve(const float2 *F, int n, void *aux, const double2 *r, double2 *d, cudaStream_t s)
+cudaError_t launch_lu32_solve(const float2 *F, int n, const int *perm, const double2 *r, double2 *d, cudaStream_t s)
 {
-    k_lu32_solve<<<LU32_CTAS, LU32_T, lu32_solve_smem(n), s>>>(F, n, lu32_perm(aux, n), lu32_inv(aux), r, d);
+    k_lu32_solve<<<LU32_CTAS, LU32_T, lu32_solve_smem(n), s>>>(F, n, perm, r, d);
     return cudaGetLastError();
 }
 
