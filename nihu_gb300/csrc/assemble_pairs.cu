@@ -29,6 +29,7 @@ namespace nihu {
 
 constexpr int PAIR_THREADS = 256;
 constexpr int PAIR_SING_THREADS = 128;
+constexpr int PAIR_SING_BLOCKS = 3;  // per SM: at most 168 registers a thread
 
 __device__ __forceinline__ bool pair_valid(const PairArgs &a, int i, int j)
 {
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_pairs_regular(PairArgs a)
 
 // CK: a complex (lossy) wave number, the FP64 complex schemes in both modes
 template <typename Out, bool CK>
-__global__ void __launch_bounds__(PAIR_SING_THREADS) k_pairs_singular(PairArgs a)
+__global__ void __launch_bounds__(PAIR_SING_THREADS, PAIR_SING_BLOCKS) k_pairs_singular(PairArgs a)
 {
     const unsigned long long n_near = a.n_sing[0], count = n_near + a.n_sing[1];
     const bool S = (a.ops & OP_SLP) != 0, D = (a.ops & OP_DLP) != 0;
@@ -330,10 +331,11 @@ cudaError_t launch_assemble_pairs(const PairArgs &a, cudaStream_t s)
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // the singular list's length stays on the device: the kernel reads it
     const int64_t swant = (a.n + PAIR_SING_THREADS - 1) / PAIR_SING_THREADS;
-    // three 4-warp blocks per SM, what the registers hold (the float-float sums
-    // are bound by FP32 issue): 5.1 M pairs, 310 k of them nearly singular, in
-    // 0.78 ms (two blocks 0.86 ms)
-    const int sblocks = (int)std::max<int64_t>(1, std::min<int64_t>(swant, 3 * (int64_t)sms));
+    // three 4-warp blocks per SM, for which the registers are bounded (40 bytes
+    // spilled; the latency of one thread's float-float chain is what bounds the
+    // kernel): 5.1 M pairs, 310 k of them nearly singular, in 0.78 ms (two blocks,
+    // which 247 unbounded registers leave, 0.91 ms)
+    const int sblocks = (int)std::max<int64_t>(1, std::min<int64_t>(swant, PAIR_SING_BLOCKS * (int64_t)sms));
     const bool ck = a.family == FAM_HELMHOLTZ && a.k_im != 0.0;
     if (ck) {
         if (a.dtype == 0) k_pairs_singular<float2, true><<<sblocks, PAIR_SING_THREADS, 0, s>>>(a);
