@@ -334,9 +334,9 @@ cudaError_t timed_gemv(nihu_gb_ctx *ctx, int dtype, const void *A, int64_t m, in
 
 // column splits of a matvec; under a memory budget of 256 columns at least, so that
 // its partial sums stay below a hundredth of the matrix
-int matvec_splits(const nihu_gb_ctx *ctx, int64_t m, int64_t n, int dtype)
+int matvec_splits(const nihu_gb_ctx *ctx, int64_t m, int64_t n, int dtype, int sum_warps = 1)
 {
-    const int splits = gemv_splits(m, n, dtype);
+    const int splits = gemv_splits(m, n, dtype, sum_warps);
     return ctx->budget ? (int)std::min<int64_t>(splits, std::max<int64_t>(1, n / 256)) : splits;
 }
 
@@ -1324,7 +1324,7 @@ nihu_gb_status gmres_device(nihu_gb_ctx *ctx, int dtype_a, const void *A, int64_
     // the bound of restart times vector blocks that this solver has always had
     if ((m + 1) * std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, 64)) > 4096)
         return fail(ctx, NIHU_GB_ERR_INVALID_ARGUMENT, "GMRES restart too large");
-    const int splits = matvec_splits(ctx, n, n, dtype_a);
+    const int splits = matvec_splits(ctx, n, n, dtype_a, GMRES_SUM_WARPS);
     GmresPlan plan;
     CK(gmres_step_plan(n, m, ctx->device, INT_MAX, &plan));
     void *pV, *ppart, *pwork, *psmall;

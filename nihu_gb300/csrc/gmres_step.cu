@@ -29,6 +29,7 @@ namespace {
 
 constexpr int GS_THREADS = 256;
 constexpr int GS_WARPS = GS_THREADS / 32;
+static_assert(GS_WARPS == GMRES_SUM_WARPS, "the partial products are summed by every warp");
 constexpr int GS_ROWS = 32;  // fewest rows per CTA
 
 __device__ __forceinline__ double2 cmul2(double2 a, double2 b)

@@ -166,7 +166,6 @@ __global__ void k_gemv_reduce(const double2 *__restrict__ partial, int splits, i
     y += (int64_t)blockIdx.y * m;
     if (i >= m) return;
     double sr = 0.0, si = 0.0;
-#pragma unroll 8
     for (int s = 0; s < splits; ++s) {
         double2 v = partial[(int64_t)s * m + i];
         sr += v.x;
@@ -177,7 +176,7 @@ __global__ void k_gemv_reduce(const double2 *__restrict__ partial, int splits, i
     y[i] = make_double2(are * sr - aim * si + bre * yo.x - bim * yo.y, are * si + aim * sr + bre * yo.y + bim * yo.x);
 }
 
-int gemv_splits(int64_t m, int64_t n, int dtype)
+int gemv_splits(int64_t m, int64_t n, int dtype, int sum_warps)
 {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -186,12 +185,24 @@ int gemv_splits(int64_t m, int64_t n, int dtype)
     int64_t row_blocks = (m + rows_per_block - 1) / rows_per_block;
     int64_t want = (int64_t)sms * 4;
     int64_t splits = (want + row_blocks - 1) / row_blocks;
-    // at least 32 columns per split: the partial sums (16 B a row) then stay below
-    // a sixteenth of the matrix, and a small or middling one fills the GPU (5120
-    // unknowns: 200 blocks and 46 us a product with 256 columns at least, 610
-    // blocks and 35 us now)
-    splits = min(splits, max((int64_t)1, n / 32));
-    return (int)max((int64_t)1, min(splits, (int64_t)1024));
+    // of at least 256 columns, or of at least 32 where that is faster.  complex64: a
+    // block takes 184 ns a column, all together no less than HBM does (6.7 TB/s);
+    // complex128: the FP64 pipe takes 270 ns a column and block of an SM; and the sum
+    // of the partial products takes a warp 200 ns a split.  Measured, 256 / 32 columns:
+    // complex64, 320 unknowns 33 / 20 us, 5120 61 / 57, 8000 96 / 100, 1000 x 20000
+    // 75 / 88, 20000 x 1000 74 / 43; complex128, 4000 unknowns 156 / 132, 5120
+    // 218 / 234, 1000 x 20000 227 / 175
+    auto clamp = [&](int64_t columns) {
+        return max((int64_t)1, min(min(splits, max((int64_t)1, n / columns)), (int64_t)1024));
+    };
+    auto ns = [&](int64_t s) {
+        const int64_t columns = (n + s - 1) / s;
+        const int64_t product = dtype == 0 ? max(184 * columns, (int64_t)((double)m * (double)n * 8.0 / 6700.0))
+                                           : 270 * columns * ((row_blocks * s + sms - 1) / sms);
+        return product + 200 * s / sum_warps;
+    };
+    const int64_t coarse = clamp(256), fine = clamp(32);
+    return (int)(ns(fine) < ns(coarse) ? fine : coarse);
 }
 
 static void gemv_partial(int dtype, const void *A, int64_t m, int64_t n, int64_t lda, int64_t a_stride, int batch,

@@ -6,8 +6,10 @@
 
 namespace nihu {
 
-// number of column splits of a matvec (partial buffer holds splits * m complex128)
-int gemv_splits(int64_t m, int64_t n, int dtype);
+// number of column splits of a matvec (partial buffer holds splits * m complex128);
+// sum_warps: warps among which the sum over the splits of a row is divided
+int gemv_splits(int64_t m, int64_t n, int dtype, int sum_warps = 1);
+constexpr int GMRES_SUM_WARPS = 8;  // of the GMRES step
 cudaError_t launch_gemv(int dtype, const void *A, int64_t m, int64_t n, int64_t lda, const double2 *x, double2 *y,
                         double are, double aim, double bre, double bim, double2 *partial, int splits, cudaStream_t s);
 
