@@ -31,6 +31,11 @@ constexpr int GS_THREADS = 256;
 constexpr int GS_WARPS = GS_THREADS / 32;
 static_assert(GS_WARPS == GMRES_SUM_WARPS, "the partial products are summed by every warp");
 constexpr int GS_ROWS = 32;  // fewest rows per CTA
+// basis vectors from which on each thread takes one (its product with w, its sum
+// over the CTAs): a warp's sum over its lanes, 20 FP64 additions a vector, is then
+// most of the step (2000 unknowns, GMRES(256), 256 steps: 69.7 -> 44.0 ms; eight
+// launches a step, before the cooperative one, 60.2)
+constexpr int GS_LONG = 64;
 
 __device__ __forceinline__ double2 cmul2(double2 a, double2 b)
 {
@@ -162,9 +167,68 @@ __global__ void __launch_bounds__(GS_THREADS) k_gmres_step(GmresStep a)
         return;
     }
 
+    // out[v] = V_v^H w, v <= k: a vector a thread
+    auto project_long = [&](double2 *out) {
+        double2 *all = a.sums + (size_t)buf * (m + 1) * G;
+        for (int v = tid; v <= k; v += GS_THREADS) {
+            const double2 *Vv = V + (int64_t)v * n + i0;
+            double sr = 0.0, si = 0.0;
+#pragma unroll 4
+            for (int i = 0; i < rows; ++i) {
+                const double2 q = cmulc(Vv[i], w[i]);
+                sr += q.x;
+                si += q.y;
+            }
+            __stcg(all + (size_t)rank * (m + 1) + v, make_double2(sr, si));
+        }
+        grid.sync();
+        for (int v = tid; v <= k; v += GS_THREADS) {
+            double sr = 0.0, si = 0.0;
+#pragma unroll 8
+            for (int c = 0; c < G; ++c) {
+                const double2 t = __ldcg(all + (size_t)c * (m + 1) + v);
+                sr += t.x;
+                si += t.y;
+            }
+            out[v] = make_double2(sr, si);
+        }
+        buf ^= 1;
+        __syncthreads();
+    };
+
     // CGS2: h = V^H w, w -= V h, twice (the second time h2)
+    const bool many = k + 1 >= GS_LONG;
     for (int pass = 0; pass < 2; ++pass) {
         double2 *hp = pass ? h2 : h;
+        if (many) {
+            project_long(hp);
+            // 32 rows at a time, every eighth vector per warp, the warps subtracted in order
+            for (int r0 = 0; r0 < rows; r0 += 32) {
+                const int i = r0 + lane;
+                double sr = 0.0, si = 0.0;
+                if (i < rows) {
+                    const double2 *Vi = V + i0 + i;
+#pragma unroll 4
+                    for (int v = warp; v <= k; v += GS_WARPS) {
+                        const double2 q = cmul2(__ldcg(Vi + (int64_t)v * n), hp[v]);
+                        sr += q.x;
+                        si += q.y;
+                    }
+                }
+                part[warp * 32 + lane] = make_double2(sr, si);
+                __syncthreads();
+                if (warp == 0 && i < rows) {
+                    double2 x = w[i];
+                    for (int q = 0; q < GS_WARPS; ++q) {
+                        x.x -= part[q * 32 + lane].x;
+                        x.y -= part[q * 32 + lane].y;
+                    }
+                    w[i] = x;
+                }
+                __syncthreads();
+            }
+            continue;
+        }
         reduce(k + 1, hp, [&](int v) {
             const double2 *Vv = V + (int64_t)v * n + i0;
             double sr = 0.0, si = 0.0;

@@ -43,3 +43,28 @@ def test_more_than_256_steps(gpu_ctx, restart):
     assert np.linalg.norm(A @ p - b) <= 2e-8 * np.linalg.norm(b)
     ref = np.linalg.solve(A, b)
     assert np.linalg.norm(p - ref) <= 2.2e-4 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [63, 64, 65, 97, 255, 256])
+def test_every_step_of_a_cycle(gpu_ctx, n):
+    # a cyclic shift in a random unitary basis, from its first basis vector: the
+    # residual stays what it is for n - 1 steps
+    rng = np.random.default_rng(n)
+    U = np.linalg.qr(rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))[0]
+    A, b = np.asfortranarray(np.roll(U, 1, axis=1) @ U.conj().T), U[:, 0].copy()
+    x, it, res = g.gmres(A, b, restart=n, max_iters=n, tol=1e-10, ctx=gpu_ctx)
+    assert it == n and np.linalg.norm(A @ x - b) <= 1e-10
+
+
+@pytest.mark.parametrize("n", [321, 4900])
+def test_cycles_beyond_a_vector_per_thread(gpu_ctx, n):
+    # eigenvalues in a disc of radius 0.9 about 1: about a factor of 0.9 a step
+    rng = np.random.default_rng(n)
+    A = np.empty((n, n), complex, order="F")
+    A.real, A.imag = rng.standard_normal((n, n)), rng.standard_normal((n, n))
+    A *= 0.9 / np.sqrt(2 * n)
+    A[np.arange(n), np.arange(n)] += 1
+    b = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    x, it, res = g.gmres(A, b, restart=200, max_iters=200, tol=1e-6, ctx=gpu_ctx)
+    assert 65 <= it <= 200 and res < 1e-6
+    assert np.linalg.norm(A @ x - b) <= 2e-6 * np.linalg.norm(b)
