@@ -357,8 +357,10 @@ __global__ void __launch_bounds__(8 * LU32_BLK) k_lu32_diag(float2 *__restrict__
         X[c][r] = make_float2(0.0f, 0.0f);
     }
     __syncthreads();
-    for (int s = 0; s < LU32_BLK; ++s) {
-        const int r = upper ? LU32_BLK - 1 - s : s;
+    // a row a step, 0.8 us each: the matrix's alone
+    const int rows = min(LU32_BLK, n - b0);
+    for (int s = 0; s < rows; ++s) {
+        const int r = upper ? rows - 1 - s : s;
         float2 v = make_float2(h == 0 && r == j ? 1.0f : 0.0f, 0.0f);
 #pragma unroll
         for (int q = 0; q < LU32_BLK; q += 8) csubf(v, D[r][q + h], X[j][q + h]);  // zero from row r on
@@ -522,6 +524,45 @@ __global__ void __cluster_dims__(LU32_CTAS, 1, 1) __launch_bounds__(LU32_T)
     }
 }
 
+// the same for one diagonal block (n <= 64): no cluster to launch and to wait for
+// (order 1, the whole solve: 167 -> 150 us)
+__global__ void __launch_bounds__(LU32_T) k_lu32_solve_block(const float2 *__restrict__ F, int n, const int *__restrict__ perm,
+                                                             const double2 *__restrict__ r, double2 *__restrict__ d)
+{
+    __shared__ float2 s_y[LU32_BLK], s_red[8][LU32_BLK];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row = (warp & 1) * 32 + lane, g = warp >> 1;
+    if (tid < LU32_BLK) {
+        const double2 x = tid < n ? r[perm[tid]] : make_double2(0.0, 0.0);
+        s_y[tid] = make_float2((float)x.x, (float)x.y);
+    }
+    for (int upper = 0; upper < 2; ++upper) {
+        float2 t[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int j = g * 8 + c;
+            const bool own = row < n && j < n && (upper ? row <= j : row > j);
+            t[c] = own ? __ldg(F + (int64_t)j * n + row) : make_float2(!upper && row == j ? 1.0f : 0.0f, 0.0f);
+        }
+        __syncthreads();
+        float2 v = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) csubf(v, t[c], s_y[g * 8 + c]);
+        s_red[g][row] = v;
+        __syncthreads();
+        if (g == 0) {
+            v = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int h = 0; h < 8; ++h) {
+                v.x -= s_red[h][row].x;
+                v.y -= s_red[h][row].y;
+            }
+            s_y[row] = v;
+            if (upper && row < n) d[row] = make_double2((double)v.x, (double)v.y);
+        }
+    }
+}
+
 // x += d; sums[0] = |d|^2, sums[1] = |x|^2 (one block, fixed order)
 __global__ void __launch_bounds__(1024) k_lu32_update_x(double2 *x, const double2 *__restrict__ d, int n, double *sums)
 {
@@ -605,7 +646,7 @@ static cudaError_t launch_panel(float2 *F, int n, int j0, int *nb, Lu32Moves *mo
     cfg.blockDim = dim3(T);
     cfg.stream = s;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ctas > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k_lu32_panel<NB, R, T>, F, n, j0, *nb, moves, info);
 }
 
@@ -646,7 +687,8 @@ cudaError_t launch_lu32_factor(float2 *F, int n, int *perm, void *work, int *inf
 
 cudaError_t launch_lu32_solve(const float2 *F, int n, const int *perm, const double2 *r, double2 *d, cudaStream_t s)
 {
-    k_lu32_solve<<<LU32_CTAS, LU32_T, lu32_solve_smem(n), s>>>(F, n, perm, r, d);
+    if (n <= LU32_BLK) k_lu32_solve_block<<<1, LU32_T, 0, s>>>(F, n, perm, r, d);
+    else k_lu32_solve<<<LU32_CTAS, LU32_T, lu32_solve_smem(n), s>>>(F, n, perm, r, d);
     return cudaGetLastError();
 }
 
