@@ -772,8 +772,8 @@ static cudaError_t launch_galerkin_regular2(const GalArgs &a, cudaStream_t s)
 
 // ------------------------------------------------- near pairs, FP32 triangles
 
-// sin and cos in FP32: the Taylor series to x^11 and x^12 for |x| <= pi/2
-// (truncation below 4e-8), when the caller's bound allows (warp-uniform), else
+// sin and cos in FP32: the Taylor series to x^13 and x^12 for |x| <= pi/2
+// (truncation below 7e-10 and 7e-9), when the caller's bound allows (warp-uniform), else
 // the library's
 __device__ __forceinline__ void sincos_short(float x, bool bounded, float &s, float &c)
 {
@@ -782,7 +782,7 @@ __device__ __forceinline__ void sincos_short(float x, bool bounded, float &s, fl
         return;
     }
     const float u = x * x;
-    float p = -1.0f / 39916800.0f, q = 1.0f / 479001600.0f;
+    float p = fmaf(1.0f / 6227020800.0f, u, -1.0f / 39916800.0f), q = 1.0f / 479001600.0f;
     p = fmaf(p, u, 1.0f / 362880.0f);
     q = fmaf(q, u, -1.0f / 3628800.0f);
     p = fmaf(p, u, -1.0f / 5040.0f);
