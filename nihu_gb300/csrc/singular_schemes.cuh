@@ -381,7 +381,8 @@ __device__ inline void near_dynamic_f32(const Elem64 &e, double k, const double 
 // are stored in FP32 (ffloat.cuh): E - 1 and (1 + z) E - 1 with E = e^{-z},
 // z = ikr, whose difference from 1 keeps 1e-12 of 1.  The points are formed
 // from the corner relative to x0 and the sides; r.n is the same at all of
-// them.  |k| r <= 64 is the caller's promise.  Bound by FP32 issue: about 560
+// them.  Lengths are scaled by a power of two near the element's size, so that no
+// power of r leaves FP32 range.  |k| r <= 64 is the caller's promise.  Bound by FP32 issue: about 560
 // instructions a point in place of 190 FP64 ones (16 SM cycles each); 4493
 // triangles, k = 4 - 0.3i, the singular kernel: 1175 -> 254 us.
 template <int G>
@@ -392,16 +393,18 @@ __device__ inline void near_dynamic_ck_ff(const Elem64 &e, cd k, const double x0
     for (int d = 0; d < 3; ++d) { e1[d] = e.c[1][d] - e.c[0][d]; e2[d] = e.c[2][d] - e.c[0][d]; }
     cross3(e1, e2, nt);
     const double J = norm3(nt);
+    const int ex2 = ((__float_as_int(sqrtf((float)J)) >> 23) & 255) - 127;
+    const float sc = __int_as_float((127 - ex2) << 23), isc = __int_as_float((127 + ex2) << 23);  // 2^-+ex2
     ff b[3], f1[3], f2[3];
     double rn = 0.0;
     for (int d = 0; d < 3; ++d) {
         const double c = e.c[0][d] - x0[d];
         rn += c * nt[d];
-        b[d] = ff_from(c);
-        f1[d] = ff_from(e1[d]);
-        f2[d] = ff_from(e2[d]);
+        b[d] = ff_scale(ff_from(c), sc);
+        f1[d] = ff_scale(ff_from(e1[d]), sc);
+        f2[d] = ff_scale(ff_from(e2[d]), sc);
     }
-    const ff kr = ff_from(k.re), ki = ff_from(k.im), one{1.0f, 0.0f};
+    const ff kr = ff_scale(ff_from(k.re), isc), ki = ff_scale(ff_from(k.im), isc), one{1.0f, 0.0f};
     ff sr{0.0f, 0.0f}, si = sr, dr = sr, di = sr;
 #pragma unroll 1
     for (int p = g.lane; p < 42; p += G) {
@@ -435,7 +438,7 @@ __device__ inline void near_dynamic_ck_ff(const Elem64 &e, cd k, const double x0
             di = ff_add(di, ff_mul(u, zi));
         }
     }
-    const double ws = J * INV_FOUR_PI, wd = rn * INV_FOUR_PI;  // rn / J is r.n, times the weight's J
+    const double ds = sc, ws = J * INV_FOUR_PI * ds, wd = rn * INV_FOUR_PI * (ds * ds * ds);  // rn / J is r.n, times the weight's J
     if (do_s) {
         a.sr += ws * g.sum(ff_double(sr));
         a.si += ws * g.sum(ff_double(si));
