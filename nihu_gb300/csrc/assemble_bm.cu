@@ -490,11 +490,6 @@ __global__ void __launch_bounds__(TWO_ROW_THREADS, 28 / TWO_ROW_WARPS) k_regular
     else two_row_columns<false>(op, sh, a.test, ib, ncols);
 }
 
-// three or four blocks of k_regular_bm2 (18 KB of shared memory each): the
-// 100 KB configuration, which the singular kernel beside it asks for as well,
-// so that an SM it starts on is configured for both
-static int bm2_carveout_percent() { return 44; }
-
 // all four operators are the Burton-Miller system: unit coefficients of SLP
 // and DLP, one coefficient c of DLPt and HSP, overwritten outputs
 static bool bm_system(const BmArgs &a)
@@ -512,7 +507,7 @@ static cudaError_t launch_bm2(const BmArgs &a, cudaStream_t s)
     static bool carveout_set[64] = {};
     if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
         const cudaError_t e = cudaFuncSetAttribute(k_regular_bm2<FAM>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                                   bm2_carveout_percent());
+                                                   TWO_ROW_CARVEOUT);
         if (e != cudaSuccess) return e;
         carveout_set[dev] = true;
     }
@@ -651,7 +646,7 @@ cudaError_t launch_assemble_singular_bm(const BmArgs &a, const NearList &near, c
     static bool carveout_set[64] = {};
     if (dev >= 0 && dev < 64 && !carveout_set[dev]) {
         cudaError_t e = cudaFuncSetAttribute(k_singular_bm<float2, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                             bm2_carveout_percent());
+                                             TWO_ROW_CARVEOUT);
         if (e != cudaSuccess) return e;
         carveout_set[dev] = true;
     }

@@ -492,10 +492,10 @@ __global__ void __launch_bounds__(GAL_THREADS) k_galerkin_regular(GalArgs a)
 // which they may share a node), tested against the largest of the warp's rows;
 // lists 0 and 1 compare node ids within it.
 //
-// Bound by FP32 issue: the one-row kernel ran every lane of a warp through the
-// largest product of its 32 pairs.  5120 triangles, k = 5, both operators:
-// with the near pairs' kernel 1269 us before, 888 us now; alone 635 us (45% of
-// the issue slots; 96 registers, spill-free only up to 20 warps per SM, which
+// Bound by latency at 20 warps an SM (96 registers; 45% of the issue slots).  The
+// one-row kernel ran every lane of a warp through the largest product of its 32
+// pairs.  5120 triangles, k = 5, both operators: with the near pairs' kernel 1269
+// us before, 892 us now; alone 635 us (spill-free only up to 20 warps per SM, which
 // measured 30 us less than 28).
 struct Gal2Val {
     f2 sr, si, dr, di;

@@ -467,12 +467,7 @@ __global__ void __launch_bounds__(REG_THREADS) k_regular(RegularArgs a)
     }
 }
 
-int regular_carveout_percent()
-{
-    // four blocks of k_regular2 (18 KB of shared memory each, plus the 1 KB the
-    // runtime reserves per block): the 100 KB configuration
-    return 44;
-}
+int regular_carveout_percent() { return TWO_ROW_CARVEOUT; }
 
 // ------------------------------------------------- two rows per thread
 // The FP32 kernel of a single wave number into complex64 matrices, through the
@@ -706,7 +701,8 @@ struct Reg2Op {
     }
 };
 
-// 64 registers: three blocks fit beside the concurrent singular kernel's one
+// 64 registers, eight blocks an SM, six beside one block of the concurrent singular
+// kernel
 template <int FAM, int OPS, bool CK, bool PLAIN>
 __global__ void __launch_bounds__(TWO_ROW_THREADS, 32 / TWO_ROW_WARPS) k_regular2(const __grid_constant__ RegularArgs a, int cols_per_block)
 {

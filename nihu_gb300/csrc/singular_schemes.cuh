@@ -382,9 +382,11 @@ __device__ inline void near_dynamic_f32(const Elem64 &e, double k, const double 
 // z = ikr, whose difference from 1 keeps 1e-12 of 1.  The points are formed
 // from the corner relative to x0 and the sides; r.n is the same at all of
 // them.  Lengths are scaled by a power of two near the element's size, so that no
-// power of r leaves FP32 range.  |k| r <= 64 is the caller's promise.  Bound by FP32 issue: about 560
+// power of r leaves FP32 range.  |k| r <= 64 is the caller's promise.  About 560
 // instructions a point in place of 190 FP64 ones (16 SM cycles each); 4493
-// triangles, k = 4 - 0.3i, the singular kernel: 1175 -> 254 us.
+// triangles, k = 4 - 0.3i, the singular kernel: 1175 -> 254 us.  Bound by the
+// latency of a thread's chain: eight warps an SM issue in 40% of the cycles, and
+// the FP64 pipe, the set-up's, is active in 33%.
 template <int G>
 __device__ inline void near_dynamic_ck_ff(const Elem64 &e, cd k, const double x0[3], bool do_s, bool do_d, Acc &a,
                                           const Lanes<G> &g)

@@ -36,8 +36,11 @@ struct OpSet {
 // against rounding when x0 lies on a side's line.  Lengths are scaled by a
 // power of two near the element's size, so that no product leaves FP32 range.
 //
-// Bound by FP32 issue: about 18 000 FP32 instructions per pair in place of
-// 8 500 FP64 ones (GB300: 128 against 2 per SM and cycle).  On the sphere of
+// About 18 000 FP32 instructions per pair in place of 8 500 FP64 ones (GB300:
+// 128 against 2 per SM and cycle).  Bound by the latency of one thread's chain: the
+// kernels that call it issue in 46% of the cycles with twelve warps an SM (pair
+// lists; their FP64 set-up and self terms keep that pipe active in 65%) and in
+// 34% with eight (the Burton-Miller system).  On the sphere of
 // 20480 triangles the singular kernel of the Burton-Miller system, beside the
 // regular one, went from 4.04 to 0.84 ms and the near field list of 5.1 M
 // pairs from 3.53 to 0.78 ms; the complex64 entries' error against 64 bits

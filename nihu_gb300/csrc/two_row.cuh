@@ -87,6 +87,14 @@ struct TwoRowShared {
     }
 };
 
+// what a block takes of an SM's shared memory, 1 KB of it the runtime's own
+constexpr size_t TWO_ROW_SMEM = sizeof(TwoRowShared) + 1024;
+// the shared-memory carveout, in per cent of 228 KB, that the kernels with two rows
+// a thread and the singular ones beside them ask for alike: the 100 KB
+// configuration, which holds the eight blocks an SM that launch bounds allow
+constexpr int TWO_ROW_CARVEOUT = 44;
+static_assert(8 * TWO_ROW_SMEM <= 100 * 1024, "eight blocks in the 100 KB configuration");
+
 // columns per block: all TWO_ROW_COLS, or on a small mesh as few as keep
 // about four blocks per SM (320 elements: one column, 320 blocks; the regular
 // kernel 110 -> 13 us)
