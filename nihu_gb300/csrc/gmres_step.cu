@@ -46,6 +46,8 @@ __device__ __forceinline__ double2 cmulc(double2 a, double2 b)  // conj(a) b
     return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
 }
 
+// LONG: a step of GS_LONG basis vectors or more
+template <bool LONG>
 __global__ void __launch_bounds__(GS_THREADS) k_gmres_step(GmresStep a)
 {
     cg::grid_group grid = cg::this_grid();
@@ -197,10 +199,9 @@ __global__ void __launch_bounds__(GS_THREADS) k_gmres_step(GmresStep a)
     };
 
     // CGS2: h = V^H w, w -= V h, twice (the second time h2)
-    const bool many = k + 1 >= GS_LONG;
     for (int pass = 0; pass < 2; ++pass) {
         double2 *hp = pass ? h2 : h;
-        if (many) {
+        if constexpr (LONG) {
             project_long(hp);
             // 32 rows at a time, every eighth vector per warp, the warps subtracted in order
             for (int r0 = 0; r0 < rows; r0 += 32) {
@@ -343,13 +344,17 @@ cudaError_t gmres_step_plan(int64_t n, int restart, int device, int max_ctas, Gm
     int optin = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gmres_step, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gmres_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    if (e == cudaSuccess && restart >= GS_LONG)
+        e = cudaFuncSetAttribute(k_gmres_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e != cudaSuccess) return e;
     plan->ctas = (int)std::max<int64_t>(1, std::min<int64_t>((n + GS_ROWS - 1) / GS_ROWS, std::min(sms, max_ctas)));
     plan->smem = sizeof(double2) * (2 * (size_t)restart + 3 + GS_WARPS * 32 + 2 * (size_t)restart + 1 +
                                     (size_t)((n + plan->ctas - 1) / plan->ctas));
     if (plan->smem > (size_t)optin) return cudaErrorInvalidValue;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_step, GS_THREADS, plan->smem);
+    e = restart >= GS_LONG
+            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_step<true>, GS_THREADS, plan->smem)
+            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_step<false>, GS_THREADS, plan->smem);
     if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
     return e;
 }
@@ -366,7 +371,8 @@ cudaError_t launch_gmres_step(const GmresStep &a, const GmresPlan &plan, cudaStr
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_gmres_step, a);
+    return !a.b && a.k + 1 >= GS_LONG ? cudaLaunchKernelEx(&cfg, k_gmres_step<true>, a)
+                                      : cudaLaunchKernelEx(&cfg, k_gmres_step<false>, a);
 }
 
 cudaError_t launch_gmres_update(const GmresStep &a, double2 *x, cudaStream_t s)
