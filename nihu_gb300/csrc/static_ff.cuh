@@ -30,7 +30,11 @@ struct OpSet {
 //   HSP   s^2/z (A cos psi + B sin psi) t^{-3/2},  A = s (n.f) - n_2 z, B = s (n.l)
 //   DLPt  -(A cos psi + B sin psi) / sqrt(t) + (n.f cos psi + n.l sin psi)
 //         log((s + sqrt t) / cos psi) - n_2 sgn(z)
-// (f the foot direction, l the side's).  The rule is symmetric about the
+// (f the foot direction, l the side's).  DLPt's last term and the 1 of DLP's
+// 1 - |z|/r are constant: they take the angle that the sides make up, 2 pi or 0,
+// exactly, so that a surface that is nearly flat keeps its small DLP and DLPt
+// entries (a plate folded by 1e-7: error 3.5e-5 of the largest entry when they were
+// summed, 1e-7 now).  The rule is symmetric about the
 // side's middle angle, so one sin / cos of h x serves the two points +-x.
 // cos psi never falls below s / max(rho_1, rho_2), which the clamp keeps
 // against rounding when x0 lies on a side's line.  Lengths are scaled by a
@@ -62,10 +66,9 @@ __device__ inline bool near_static4_ff(const double *__restrict__ frame, const d
     if (ops.h && !in_plane && 1e3f * (float)fabs(z) < (float)(fabs(n0) + fabs(n1)) * len0) return false;
     const int ex2 = ((__float_as_int(len0) >> 23) & 255) - 127;
     const float sc = __int_as_float((127 - ex2) << 23), isc = __int_as_float((127 + ex2) << 23);  // 2^-+ex2
-    const ff zf = ff_scale(ff_from(fabs(z)), sc), z2 = ff_mul(zf, zf), n2f = ff_from(n2);
-    const ff n2sg = z > 0.0 ? n2f : (z < 0.0 ? ff_neg(n2f) : ff{0.0f, 0.0f});
+    const ff zf = ff_scale(ff_from(fabs(z)), sc), z2 = ff_mul(zf, zf);
     const bool six = ops.s || ops.d || ops.t;
-    double s_sum = 0.0, d_sum = 0.0, t_sum = 0.0, h_sum = 0.0;
+    double s_sum = 0.0, d_sum = 0.0, t_sum = 0.0, h_sum = 0.0, angle = 0.0;
 #pragma unroll 1
     for (int sd = g.lane; sd < SIDES; sd += G) {
         const int e1 = sd, e2 = sd == SIDES - 1 ? 0 : sd + 1;
@@ -110,17 +113,18 @@ __device__ inline bool near_static4_ff(const double *__restrict__ frame, const d
                     const ff ic = ff_recip(c);
                     const ff zc = ff_mul(zf, c);
                     if (ops.s) sl = ff_add(sl, ff_mul(w, ff_mul(ff_sub(rt, zc), ic)));
-                    if (ops.d) sdl = ff_add(sdl, ff_mul(w, ff_sub(ff{1.0f, 0.0f}, ff_mul(zc, rs))));
+                    if (ops.d) sdl = ff_add(sdl, ff_mul(w, ff_mul(zc, rs)));
                     if (ops.t) {
                         const ff g = ff_add(ff_mul(naf, c), ff_mul(nbf, sn));
                         const ff v = ff_mul(ff_add(ff_mul(A, c), ff_mul(B, sn)), rs);
                         const ff lg = ff_log(ff_mul(ff_add(s, rt), ic), ex2);
-                        st = ff_add(st, ff_mul(w, ff_sub(ff_sub(ff_mul(g, lg), v), n2sg)));
+                        st = ff_add(st, ff_mul(w, ff_sub(ff_mul(g, lg), v)));
                     }
                 });
             }
+            angle += wj;
             s_sum += wj * ff_double(sl);
-            d_sum += wj * ff_double(sdl);
+            d_sum -= wj * ff_double(sdl);
             t_sum += wj * ff_double(st);
         }
         if (ops.h) {
@@ -152,9 +156,16 @@ __device__ inline bool near_static4_ff(const double *__restrict__ frame, const d
         s_sum = g.sum(s_sum);
         d_sum = g.sum(d_sum);
         t_sum = g.sum(t_sum);
+        angle = g.sum(angle);
         h_sum = g.sum(h_sum);
     }
+    // the constants of DLP and DLPt times the angle that the sides make up: a
+    // multiple of 2 pi but for rounding, unless the foot is a corner
+    const double turns = rint(angle * (1.0 / PI));
+    const double full = fabs(angle - turns * PI) < 1e-9 ? turns * (2.0 * PI) : 2.0 * angle;
     const double sg = (0.0 < z) - (z < 0.0);
+    d_sum += full;
+    t_sum -= n2 * sg * full;
     a.sr += s_sum * (INV_FOUR_PI * isc);
     a.dr += sg * d_sum * INV_FOUR_PI;
     a.tr += t_sum * INV_FOUR_PI;
