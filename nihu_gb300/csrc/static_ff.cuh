@@ -164,8 +164,8 @@ __device__ inline bool near_static4_ff(const double *__restrict__ frame, const d
     const double turns = rint(angle * (1.0 / PI));
     const double full = fabs(angle - turns * PI) < 1e-9 ? turns * (2.0 * PI) : 2.0 * angle;
     const double sg = (0.0 < z) - (z < 0.0);
-    d_sum += full;
-    t_sum -= n2 * sg * full;
+    if (ops.d) d_sum += full;
+    if (ops.t) t_sum -= n2 * sg * full;
     a.sr += s_sum * (INV_FOUR_PI * isc);
     a.dr += sg * d_sum * INV_FOUR_PI;
     a.tr += t_sum * INV_FOUR_PI;

@@ -65,3 +65,18 @@ def test_pair_list(gpu_ctx, angle):
         got = g.assemble_pairs(mesh, mesh, r, c, ops, 2.0, dtype=g.C64, ctx=gpu_ctx)[out].astype(complex)
         ref = g.assemble_pairs(mesh, mesh, r, c, ops, 2.0, dtype=g.C128, precision="fp64", ctx=gpu_ctx)[out]
         assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("ops", [g.SLP, g.DLP, g.DLPT, g.HSP, g.SLP | g.DLP, g.DLPT | g.HSP, g.DLP | g.DLPT, g.SLP | g.HSP])
+def test_operators_of_a_sharp_fold(gpu_ctx, ops):
+    # collocation points close above the insides of elements, and only some of the
+    # operators asked for: the others contribute nothing
+    nodes, el = folded(np.deg2rad(175))
+    mesh = g.create_mesh(nodes, el)
+    n = len(el)
+    r, c = (x.ravel() for x in np.meshgrid(np.arange(n), np.arange(n), indexing="ij"))
+    got = g.assemble_pairs(mesh, mesh, r, c, ops, 2.0, dtype=g.C64, ctx=gpu_ctx)
+    ref = g.assemble_pairs(mesh, mesh, r, c, ops, 2.0, dtype=g.C128, precision="fp64", ctx=gpu_ctx)
+    for x, y in zip(got, ref):
+        if y is not None:
+            assert np.abs(x.astype(complex) - y).max() <= 1e-5 * np.abs(y).max()
