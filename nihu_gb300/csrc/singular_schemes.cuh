@@ -478,8 +478,8 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
         ex(e, res[0], res[1], y);
         edx(e, res[0], res[1], dxi, deta);
         cross3(dxi, deta, n);
-        const double isq = rsqrt(norm3(n));  // one reciprocal a step for what is divided by it
-        for (int d = 0; d < 3; ++d) n[d] *= isq;
+        double sq = sqrt(norm3(n));
+        for (int d = 0; d < 3; ++d) n[d] /= sq;
         double f[3];
         for (int d = 0; d < 3; ++d) f[d] = y[d] + n[d] * res[2] - x0[d];
         double err = norm3(f);
@@ -492,12 +492,12 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
             for (int d = 0; d < 3; ++d) r6[d] = res[d];
             return got5;
         }
-        // d n / d xi = (x_xixi x x_eta + x_xi x x_xieta) / sqrt|n|, x_xixi = x_etaeta = 0
+        // d n / d xi = (x_xixi x x_eta + x_xi x x_xieta) / sq, x_xixi = x_etaeta = 0
         double t2[3], dnxi[3], dneta[3];
         cross3(dxi, dxe, t2);
-        for (int d = 0; d < 3; ++d) dnxi[d] = t2[d] * isq;
+        for (int d = 0; d < 3; ++d) dnxi[d] = t2[d] / sq;
         cross3(dxe, deta, t2);
-        for (int d = 0; d < 3; ++d) dneta[d] = t2[d] * isq;
+        for (int d = 0; d < 3; ++d) dneta[d] = t2[d] / sq;
         double M[3][4];
         for (int d = 0; d < 3; ++d) {
             M[d][0] = dxi[d] + dnxi[d] * res[2];
@@ -505,16 +505,14 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
             M[d][2] = n[d];
             M[d][3] = f[d];
         }
-        double ip[3];  // 1 / pivot
         for (int c = 0; c < 3; ++c) {
             int p = c;
             for (int r = c + 1; r < 3; ++r)
                 if (fabs(M[r][c]) > fabs(M[p][c])) p = r;
             if (p != c)
                 for (int q = 0; q < 4; ++q) { double t = M[c][q]; M[c][q] = M[p][q]; M[p][q] = t; }
-            ip[c] = 1.0 / M[c][c];
             for (int r = c + 1; r < 3; ++r) {
-                double fct = M[r][c] * ip[c];
+                double fct = M[r][c] / M[c][c];
                 for (int q = c; q < 4; ++q) M[r][q] -= fct * M[c][q];
             }
         }
@@ -522,7 +520,7 @@ __device__ inline bool inverse_mapping(const Elem64 &e, const double x0[3], bool
         for (int r = 2; r >= 0; --r) {
             double v = M[r][3];
             for (int q = r + 1; q < 3; ++q) v -= M[r][q] * s[q];
-            s[r] = v * ip[r];
+            s[r] = v / M[r][r];
         }
         for (int d = 0; d < 3; ++d) res[d] -= s[d];
     }
