@@ -694,10 +694,11 @@ struct Gal2Op {
 #pragma unroll
                 for (int u = 0; u < 3; ++u) {
                     const float4 x = __ldg(px + 2 * u);
-                    const float ux = d.x - x.x, uy = d.y - x.y, uz = d.z - x.z, w = x.w * INV4PI;
-                    gal2_point1<FAM, PS, DO_D>(ux + y0.x, uy + y0.y, uz + y0.z, y0.w * w, p.y, p.z, p.w, k, o);
-                    gal2_point1<FAM, PS, DO_D>(ux + y1.x, uy + y1.y, uz + y1.z, y1.w * w, p.y, p.z, p.w, k, o);
-                    gal2_point1<FAM, PS, DO_D>(ux + y2.x, uy + y2.y, uz + y2.z, y2.w * w, p.y, p.z, p.w, k, o);
+                    const float w = x.w * INV4PI;
+                    // the points' difference first: one rounding at the size of r
+                    gal2_point1<FAM, PS, DO_D>(d.x + (y0.x - x.x), d.y + (y0.y - x.y), d.z + (y0.z - x.z), y0.w * w, p.y, p.z, p.w, k, o);
+                    gal2_point1<FAM, PS, DO_D>(d.x + (y1.x - x.x), d.y + (y1.y - x.y), d.z + (y1.z - x.z), y1.w * w, p.y, p.z, p.w, k, o);
+                    gal2_point1<FAM, PS, DO_D>(d.x + (y2.x - x.x), d.y + (y2.y - x.y), d.z + (y2.z - x.z), y2.w * w, p.y, p.z, p.w, k, o);
                 }
             } else {
                 const int inc = a.test.nc[i], jnc = a.trial.nc[j], cmax = inc == 4 || jnc == 4 ? 1 : 0;
@@ -706,10 +707,10 @@ struct Gal2Op {
                 const int npi = level_npts(inc, cmax, 1), npj = level_npts(jnc, cmax, 1);
                 for (int u = 0; u < npi; ++u) {
                     const float4 x = __ldg(px + 2 * u);
-                    const float ux = d.x - x.x, uy = d.y - x.y, uz = d.z - x.z, w = x.w * INV4PI;
+                    const float w = x.w * INV4PI;
                     for (int v = 0; v < npj; ++v) {
                         const float4 y = __ldg(py + 2 * v), n = __ldg(py + 2 * v + 1);
-                        gal2_point1<FAM, PS, DO_D>(ux + y.x, uy + y.y, uz + y.z, y.w * w, n.x, n.y, n.z, k, o);
+                        gal2_point1<FAM, PS, DO_D>(d.x + (y.x - x.x), d.y + (y.y - x.y), d.z + (y.z - x.z), y.w * w, n.x, n.y, n.z, k, o);
                     }
                 }
             }
