@@ -306,14 +306,16 @@ __device__ __forceinline__ void bm2_point(f2 r2, f2 w4, f2 rnx, f2 nrny, f2 nnn,
     o.bi = g * f2_fma(x, f2_fma(nci, p, ncr * q), sn);
 }
 
-// the same of one pair, rny = r.ny, nn = nx.ny (the listed ones)
-template <int FAM, bool S_, bool D_, bool T_, bool H_>
-__device__ __forceinline__ void bm2_point1(float rx, float ry, float rz, float w4, float rnx, float rny, float nn, float k,
+// the same of one pair, rny = r.ny, nn = nx.ny (the listed ones); W4: w is w J / (4 pi), else w J
+// (reg2_point1 in assemble_regular.cu)
+template <int FAM, bool S_, bool D_, bool T_, bool H_, bool W4>
+__device__ __forceinline__ void bm2_point1(float rx, float ry, float rz, float w, float rnx, float rny, float nn, float k,
                                            float cr, float ci, float ws, float4 &ab)
 {
+    constexpr float INV4PI = 0.0795774715459476679f;
     const float r2 = rx * rx + ry * ry + rz * rz;
     const float rinv = rsqrtf(r2);
-    const float g = w4 * rinv, i2 = rinv * rinv, g2 = g * i2;
+    const float g = W4 ? w * rinv : w * rinv * INV4PI, i2 = rinv * rinv, g2 = g * i2;
     float s = 0.0f, c = 1.0f, kr = 0.0f;
     if constexpr (FAM == FAM_HELMHOLTZ) {
         kr = k * (r2 * rinv);
@@ -439,7 +441,6 @@ struct Bm2Op {
     template <int LIST>
     __device__ __forceinline__ void pair(int i, int c) const
     {
-        constexpr float INV4PI = 0.0795774715459476679f;
         const TwoRowCol &t = sh.col[c];
         const float3 d = t.diff(a.test, i);
         const float4 p = t.p0(), n = a.test.p0[i];
@@ -447,10 +448,10 @@ struct Bm2Op {
         const bool far_s = LIST == 0 || (d.x * d.x + d.y * d.y + d.z * d.z) * t.hi().w >= 82.81f;
         float4 ab = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (LIST == 0)
-            bm2_point1<FAM, true, true, true, false>(d.x, d.y, d.z, p.x, -(d.x * n.y + d.y * n.z + d.z * n.w),
+            bm2_point1<FAM, true, true, true, false, true>(d.x, d.y, d.z, p.x, -(d.x * n.y + d.y * n.z + d.z * n.w),
                                                      d.x * p.y + d.y * p.z + d.z * p.w, nn, k, cr, ci, 1.0f, ab);
         else if (far_s)
-            bm2_point1<FAM, true, false, false, false>(d.x, d.y, d.z, p.x, 0.0f, 0.0f, nn, k, cr, ci, 1.0f, ab);
+            bm2_point1<FAM, true, false, false, false, true>(d.x, d.y, d.z, p.x, 0.0f, 0.0f, nn, k, cr, ci, 1.0f, ab);
         const int par = a.test.clo[i].w != 0.0f ? 1 : 0;
         const float4 *pts = a.trial.pts32 + 2 * (((int64_t)(jb + c) * 2 + par) * SLOTS + level_slot0(1));
         const int np = level_npts(3, par, 1);
@@ -459,9 +460,9 @@ struct Bm2Op {
             const float px = d.x + v.x, py = d.y + v.y, pz = d.z + v.z;
             const float rnx = -(px * n.y + py * n.z + pz * n.w), rny = px * p.y + py * p.z + pz * p.w;
             if (LIST == 0)
-                bm2_point1<FAM, false, false, false, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci, 0.0f, ab);
+                bm2_point1<FAM, false, false, false, true, false>(px, py, pz, v.w, rnx, rny, nn, k, cr, ci, 0.0f, ab);
             else
-                bm2_point1<FAM, true, true, true, true>(px, py, pz, v.w * INV4PI, rnx, rny, nn, k, cr, ci,
+                bm2_point1<FAM, true, true, true, true, false>(px, py, pz, v.w, rnx, rny, nn, k, cr, ci,
                                                         far_s ? 0.0f : 1.0f, ab);
         }
         put_one(i, c, ab);

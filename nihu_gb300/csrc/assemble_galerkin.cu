@@ -500,13 +500,14 @@ __global__ void __launch_bounds__(GAL_THREADS) k_galerkin_regular(GalArgs a)
 struct Gal2Val {
     f2 sr, si, dr, di;
 };
-// one point of two pairs; w4: the product of both weights and Jacobians over 4 pi
+// one point of two pairs; w4: the trial point's weight and Jacobian over 4 pi, wx: the
+// test point's (a rounding of their product would be the same for all pairs of two shapes)
 template <int FAM, bool S_, bool D_>
-__device__ __forceinline__ void gal2_point(f2 rx, f2 ry, f2 rz, f2 w4, f2 nx, f2 ny, f2 nz, float k, Gal2Val &v)
+__device__ __forceinline__ void gal2_point(f2 rx, f2 ry, f2 rz, f2 w4, f2 wx, f2 nx, f2 ny, f2 nz, float k, Gal2Val &v)
 {
     const f2 r2 = f2_fma(rz, rz, f2_fma(rx, rx, ry * ry));
     const f2 rinv = f2_rsqrt(r2);
-    const f2 g = w4 * rinv;
+    const f2 g = w4 * rinv * wx;
     f2 f{};  // g (r.n) / r^2: minus the DLP's factor
     if constexpr (D_) f = (g * (rinv * rinv)) * f2_fma(rz, nz, f2_fma(ry, ny, rx * nx));
     if constexpr (FAM == FAM_HELMHOLTZ) {
@@ -533,14 +534,17 @@ struct Gal2Sums {
     float sr = 0.0f, si = 0.0f, dr = 0.0f, di = 0.0f;
 };
 
-// one point of one pair
-template <int FAM, bool S_, bool D_>
-__device__ __forceinline__ void gal2_point1(float rx, float ry, float rz, float w4, float nx, float ny, float nz, float k,
+// one point of one pair, w the trial point's weight, wx the test point's; W4: w is over
+// 4 pi already (else points of equal weights round that one by one, which their sum
+// averages)
+template <int FAM, bool S_, bool D_, bool W4>
+__device__ __forceinline__ void gal2_point1(float rx, float ry, float rz, float w, float wx, float nx, float ny, float nz, float k,
                                             Gal2Sums &o)
 {
+    constexpr float INV4PI = 0.0795774715459476679f;
     const float r2 = rx * rx + ry * ry + rz * rz;
     const float rinv = rsqrtf(r2);
-    const float g = w4 * rinv;
+    const float g = (W4 ? w * rinv : w * rinv * INV4PI) * wx;
     float sn = 0.0f, cs = 1.0f, kr = 0.0f;
     if constexpr (FAM == FAM_HELMHOLTZ) {
         kr = k * (r2 * rinv);
@@ -672,20 +676,19 @@ struct Gal2Op {
     {
         const TwoRowCol &t = sh.col[c];
         v = zero();
-        gal2_point<FAM, DO_S, DO_D>(dx, dy, dz, t.w4 * e.area, t.nx, t.ny, t.nz, k, v);
+        gal2_point<FAM, DO_S, DO_D>(dx, dy, dz, t.w4, e.area, t.nx, t.ny, t.nz, k, v);
     }
     template <int LIST>
     __device__ __forceinline__ void pair(int i, int c) const
     {
         if constexpr (LIST == 1 || (DO_S && DO_D)) {
-            constexpr float INV4PI = 0.0795774715459476679f;
             constexpr bool PS = LIST == 1 && DO_S;  // the SLP at the level-1 points
             const TwoRowCol &t = sh.col[c];
             const int j = jb + c;
             const float3 d = t.diff(a.test, i);
             const float4 p = t.p0();
             Gal2Sums o;
-            if (LIST == 0) gal2_point1<FAM, true, false>(d.x, d.y, d.z, p.x * a.test.p0[i].x, p.y, p.z, p.w, k, o);
+            if (LIST == 0) gal2_point1<FAM, true, false, true>(d.x, d.y, d.z, p.x, a.test.p0[i].x, p.y, p.z, p.w, k, o);
             if (!a.test.has_quad && !a.trial.has_quad) {
                 // 3 x 3 points, one normal
                 const float4 *px = a.test.pts32 + 2 * ((int64_t)i * 2 * SLOTS + level_slot0(1));
@@ -694,11 +697,10 @@ struct Gal2Op {
 #pragma unroll
                 for (int u = 0; u < 3; ++u) {
                     const float4 x = __ldg(px + 2 * u);
-                    const float w = x.w * INV4PI;
                     // the points' difference first: one rounding at the size of r
-                    gal2_point1<FAM, PS, DO_D>(d.x + (y0.x - x.x), d.y + (y0.y - x.y), d.z + (y0.z - x.z), y0.w * w, p.y, p.z, p.w, k, o);
-                    gal2_point1<FAM, PS, DO_D>(d.x + (y1.x - x.x), d.y + (y1.y - x.y), d.z + (y1.z - x.z), y1.w * w, p.y, p.z, p.w, k, o);
-                    gal2_point1<FAM, PS, DO_D>(d.x + (y2.x - x.x), d.y + (y2.y - x.y), d.z + (y2.z - x.z), y2.w * w, p.y, p.z, p.w, k, o);
+                    gal2_point1<FAM, PS, DO_D, false>(d.x + (y0.x - x.x), d.y + (y0.y - x.y), d.z + (y0.z - x.z), y0.w, x.w, p.y, p.z, p.w, k, o);
+                    gal2_point1<FAM, PS, DO_D, false>(d.x + (y1.x - x.x), d.y + (y1.y - x.y), d.z + (y1.z - x.z), y1.w, x.w, p.y, p.z, p.w, k, o);
+                    gal2_point1<FAM, PS, DO_D, false>(d.x + (y2.x - x.x), d.y + (y2.y - x.y), d.z + (y2.z - x.z), y2.w, x.w, p.y, p.z, p.w, k, o);
                 }
             } else {
                 const int inc = a.test.nc[i], jnc = a.trial.nc[j], cmax = inc == 4 || jnc == 4 ? 1 : 0;
@@ -707,10 +709,9 @@ struct Gal2Op {
                 const int npi = level_npts(inc, cmax, 1), npj = level_npts(jnc, cmax, 1);
                 for (int u = 0; u < npi; ++u) {
                     const float4 x = __ldg(px + 2 * u);
-                    const float w = x.w * INV4PI;
                     for (int v = 0; v < npj; ++v) {
                         const float4 y = __ldg(py + 2 * v), n = __ldg(py + 2 * v + 1);
-                        gal2_point1<FAM, PS, DO_D>(d.x + (y.x - x.x), d.y + (y.y - x.y), d.z + (y.z - x.z), y.w * w, n.x, n.y, n.z, k, o);
+                        gal2_point1<FAM, PS, DO_D, false>(d.x + (y.x - x.x), d.y + (y.y - x.y), d.z + (y.z - x.z), y.w, x.w, n.x, n.y, n.z, k, o);
                     }
                 }
             }

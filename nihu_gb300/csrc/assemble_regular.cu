@@ -533,13 +533,16 @@ __device__ __forceinline__ void reg2_point(f2 r2, f2 w4, f2 rn, float k, float k
 }
 
 // the same of one pair (the listed ones: packed in twos they need more
-// registers than the loop leaves, and spill)
-template <int FAM, bool CK, bool S_, bool D_>
-__device__ __forceinline__ void reg2_point1(float rx, float ry, float rz, float w4, float rn, float k, float ki, float4 &o)
+// registers than the loop leaves, and spill).  W4: w is w J / (4 pi), else w J: points
+// of equal weights then round their products with 1 / (4 pi) one by one, which
+// their sum averages
+template <int FAM, bool CK, bool S_, bool D_, bool W4>
+__device__ __forceinline__ void reg2_point1(float rx, float ry, float rz, float w, float rn, float k, float ki, float4 &o)
 {
+    constexpr float INV4PI = 0.0795774715459476679f;
     const float r2 = rx * rx + ry * ry + rz * rz;
     const float rinv = rsqrtf(r2);
-    const float g = w4 * rinv;
+    const float g = W4 ? w * rinv : w * rinv * INV4PI;
     if constexpr (FAM == FAM_HELMHOLTZ) {
         const float r = r2 * rinv, kr = k * r;
         float sn, cs, a1 = 1.0f;
@@ -666,14 +669,13 @@ struct Reg2Op {
     template <int LIST>
     __device__ __forceinline__ void pair(int i, int c) const
     {
-        constexpr float INV4PI = 0.0795774715459476679f;
         if constexpr (LIST == 1 || (DO_S && DO_D)) {
             constexpr bool PS = LIST == 1 && DO_S;  // the SLP at the level-1 points
             const TwoRowCol &t = sh.col[c];
             const float3 d = t.diff(a.test, i);
             const float4 p = t.p0();
             float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (LIST == 0) reg2_point1<FAM, CK, true, false>(d.x, d.y, d.z, p.x, 0.0f, k, ki, o);
+            if (LIST == 0) reg2_point1<FAM, CK, true, false, true>(d.x, d.y, d.z, p.x, 0.0f, k, ki, o);
             const int par = a.test.clo[i].w != 0.0f ? 1 : 0;
             const bool quad = a.trial.has_quad && a.trial.nc[jb + c] == 4;
             const float4 *pts = a.trial.pts32 + 2 * (((int64_t)(jb + c) * 2 + par) * SLOTS + level_slot0(1));
@@ -689,7 +691,7 @@ struct Reg2Op {
                     if (quad) n = __ldg(pts + 2 * q + 1);
                     rn = px * n.x + py * n.y + pz * n.z;
                 }
-                reg2_point1<FAM, CK, PS, DO_D>(px, py, pz, v.w * INV4PI, rn, k, ki, o);
+                reg2_point1<FAM, CK, PS, DO_D, false>(px, py, pz, v.w, rn, k, ki, o);
             }
             put_one(i, c, o);
         }

@@ -317,10 +317,12 @@ __device__ inline void near_dynamic4_f32(const Elem64 &e, double k, const double
         const float r2 = rv0 * rv0 + rv1 * rv1 + rv2 * rv2;
         const float rinv = rsqrtf(r2);
         const float kr = kf * (r2 * rinv);
-        // one sincos of the half angle: cos(kr) - 1 without cancellation
-        float hs, hc;
-        sincosf(0.5f * kr, &hs, &hc);
-        const float cm1 = -2.0f * hs * hs, sn = 2.0f * hs * hc, cs = 1.0f + cm1;
+        float sn, cs;
+        sincosf(kr, &sn, &cs);
+        // cos(kr) - 1 without cancellation (all three from one half angle's sine and
+        // cosine: near entries' errors up to a quarter larger)
+        const float hs = sinf(0.5f * kr);
+        const float cm1 = -2.0f * hs * hs;
         const float t = w * wj * rinv;
         const float rdnx = -(rv0 * xn[0] + rv1 * xn[1] + rv2 * xn[2]) * rinv;
         const float rdny = (rv0 * en[0] + rv1 * en[1] + rv2 * en[2]) * rinv;
