@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(GAL_THREADS) k_galerkin_regular(GalArgs a)
 // Bound by latency at 20 warps an SM (96 registers; 45% of the issue slots).  The
 // one-row kernel ran every lane of a warp through the largest product of its 32
 // pairs.  5120 triangles, k = 5, both operators: with the near pairs' kernel 1269
-// us before, 892 us now; alone 635 us (spill-free only up to 20 warps per SM, which
+// us before, 903 us now; alone 635 us (spill-free only up to 20 warps per SM, which
 // measured 30 us less than 28).
 struct Gal2Val {
     f2 sr, si, dr, di;

@@ -333,7 +333,7 @@ cudaError_t launch_assemble_pairs(const PairArgs &a, cudaStream_t s)
     const int64_t swant = (a.n + PAIR_SING_THREADS - 1) / PAIR_SING_THREADS;
     // three 4-warp blocks per SM, for which the registers are bounded (40 bytes
     // spilled; the latency of one thread's float-float chain is what bounds the
-    // kernel): 5.1 M pairs, 310 k of them nearly singular, in 0.78 ms (two blocks,
+    // kernel): 5.1 M pairs, 310 k of them nearly singular, in 0.80 ms (two blocks,
     // which 247 unbounded registers leave, 0.91 ms)
     const int sblocks = (int)std::max<int64_t>(1, std::min<int64_t>(swant, PAIR_SING_BLOCKS * (int64_t)sms));
     const bool ck = a.family == FAM_HELMHOLTZ && a.k_im != 0.0;

@@ -784,12 +784,12 @@ cudaError_t launch_assemble_singular(const RegularArgs &a, const NearList &near,
     }
     if (a.precision == 0 && a.dtype == 0 && a.nk <= 1 && !a.force_batch && a.trial.has_quad && a.k_im == 0.0) {
         // few pairs are bound by one pair's chain, many by the repeated set-up
-        // (cylinders of 288 / 1480 / 2496 / 5544 / 9792 quads, eight items a quad, a
-        // call: k_singular 650 / 666 / 697 / 890 / 1200 us, 2 lanes 317 / 353 / 418 /
-        // 743 / 1286, 4 lanes 218 / 336 / 516 / 990 / 1705)
+        // (cylinders of 288 / 832 / 1480 / 2496 / 3712 / 5544 quads, eight items a quad, a
+        // call: k_singular 444 / 441 / 649 / 748 / 533 / 667 us, 2 lanes 333 / 318 / 370 /
+        // 446 / 545 / 829, 4 lanes 242 / 272 / 367 / 562 / 737 / 1107)
         const int64_t room = 4 * (int64_t)sms * SING_THREADS;
         if (items * 6 <= room) return launch_singular_quad<4>(a, near, items, sms, err, s);
-        if (items * 4 <= room * 3) return launch_singular_quad<2>(a, near, items, sms, err, s);
+        if (items * 3 <= room) return launch_singular_quad<2>(a, near, items, sms, err, s);
     }
     // this kernel needs no shared memory, but the regular kernel's blocks
     // beside it do: the same carveout preference as theirs, so that an SM

@@ -718,8 +718,8 @@ __device__ __forceinline__ void kern32(int fam, float k, const float rv[3], cons
 // sines in float-float, one pair of them for two points of the symmetric rule:
 // FP64 angles, sines and quotients per point, and the FP64 rule's conversions,
 // were a third of the singular kernel's time on quads (with the static part in
-// float-float and fewer divisions in the inverse mapping, closed cylinder of
-// 9 792 quads, SLP and DLP: 1997 -> 1200 us; entries' error unchanged).
+// float-float, closed cylinder of 9 792 quads, SLP and DLP: 1997 -> 1250 us;
+// entries' error unchanged).
 template <int G = 1>
 static __device__ __noinline__ void near_polar_sum_f32(const Elem64 &e, int fam, double k, const double x0[3], double xi0,
                                           double eta0, bool do_s, bool do_d, Acc &a, const Lanes<G> &g = Lanes<G>())

@@ -47,7 +47,7 @@ struct OpSet {
 // 34% with eight (the Burton-Miller system).  On the sphere of
 // 20480 triangles the singular kernel of the Burton-Miller system, beside the
 // regular one, went from 4.04 to 0.84 ms and the near field list of 5.1 M
-// pairs from 3.53 to 0.78 ms; the complex64 entries' error against 64 bits
+// pairs from 3.53 to 0.80 ms; the complex64 entries' error against 64 bits
 // stays 2.6e-8 and 2.4e-8.  Returns false (nothing added) where the HSP's 1/z
 // cancels between the sides by more than three digits: |z| small against the
 // in-plane part of nx times the side, a folded pair whose collocation point
